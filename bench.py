@@ -518,16 +518,12 @@ def run_secondary(args):
     line = {"metric": metric, "value": value, "unit": unit, "n_gpus": 1, "steps": args.steps, "warmup": args.warmup,
             "ms_per_step": ms / args.steps, "higher_is_better": True, "dtype": "f32", "data": "synthetic", "config": cfg}
     if args.workload == "hausdorff":
-        # the tensor-core screen: sample-triangle pairs screened (one K = 16
-        # bf16 MMA column each, 2 x 16 flops) and exact distances left
+        # the cluster search: sample-triangle pairs of the clusters visited,
+        # of all pairs, and the exact distances among them
         st = g.hd_stats()
-        secs = ms / args.steps / 1000.0
-        tflops = 2 * 16 * st["screened"] / secs / 1e12
-        bf16_peak = json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["bf16_tflops"] \
-            if os.path.exists(os.path.join(ROOT, "MEASURED_PEAKS.json")) else 1900.0
-        line["screen"] = {"screened_pairs": st["screened"], "exact_distances": st["exact"],
-                          "exact_fraction": st["exact"] / max(st["screened"], 1), "timeout": st["timeout"],
-                          "tensor_tflops": tflops, "bf16_peak_tflops": bf16_peak, "tensor_frac": tflops / bf16_peak}
+        line["screen"] = {"screened_pairs": st["screened"], "screened_fraction": st["screened"] / units,
+                          "exact_distances": st["exact"], "exact_fraction": st["exact"] / max(st["screened"], 1),
+                          "timeout": st["timeout"]}
         # the same batch through the exhaustive search alone
         g2 = tree_mod.GpuTree(width=3, width2=3, depth=1, nConcaveEdges=0, hullMaxVerts=4096,
                               hullBudgetBytes=6 << 30, scratchWords=256 << 20, hdScreenMinTris=-1)

@@ -20,11 +20,10 @@ enum { CTR_V = 0, CTR_T = 1, CTR_E = 2, CTR_S = 3, CTR_OVERFLOW = 4, CTR_HULLFAI
 // algorithmic bytes of plan, emit and hull as 64-bit counters (a candidate
 // reads its parent once, writes its children once and each child's points
 // are read once by its hull), then Hausdorff results
-// and the Hausdorff screen's statistics: exact point-triangle distances
-// (64-bit), screened pairs (64-bit) and a flag for a tensor-core wait that
-// timed out
+// and the Hausdorff search's statistics: exact point-triangle distances
+// (64-bit), sample-triangle pairs of the clusters it visited (64-bit)
 enum { CTR_VALID_LO = 8, CTR_VALID_HI = 9, CTR_BYTES_PLAN = 10, CTR_BYTES_EMIT = 12, CTR_BYTES_HULL = 14, CTR_HD = 16,
-       CTR_HD_EXACT = 16 + 1024, CTR_HD_SCREENED = 16 + 1026, CTR_HD_ERR = 16 + 1028, CTR_WORDS = 16 + 1032 };
+       CTR_HD_EXACT = 16 + 1024, CTR_HD_SCREENED = 16 + 1026, CTR_WORDS = 16 + 1028 };
 __device__ __forceinline__ void add_bytes(uint32_t* ctr, int slot, unsigned long long b) {
   atomicAdd(reinterpret_cast<unsigned long long*>(ctr + slot), b);
 }
@@ -97,16 +96,19 @@ struct Level {
 struct HdArgs {
   uint32_t nPairs;
   uint32_t nMeshes;          // 2 * nPairs
-  const uint32_t* capOff;    // per mesh: sample offset (float4 units)
   const uint32_t* capN;      // per mesh: sample capacity
-  float4* samples;
   uint32_t* ns;              // per mesh: sample count
   uint32_t partBase;
-  uint32_t maxSide;          // largest per-side capacity
-  uint32_t screenMin;        // targets with at least this many triangles are screened
-  const uint32_t* triOff;    // per mesh: first triangle of its screen data
-  uint4* triB;               // per triangle: tensor-core operand row (16 bf16)
-  float4* triG;              // per triangle: corners; w = radius, |c|_1, |c|^2
+  uint32_t screenMin;        // targets with at least this many triangles are searched by clusters
+  const uint32_t* triOff;    // per mesh: first entry of its triangles below (a multiple of 32)
+  uint32_t* cnt;             // per triangle: its area, then its samples
+  uint32_t* soff;            // per triangle: its cell, then (sorted) its first sample
+  uint32_t* perm;            // sorted triangles' indices
+  float4* triC;              // sorted triangles: centroid, radius
+  float4* triG;              // sorted triangles: three corners
+  float4* box;               // per cluster of 32 sorted triangles: low and high corner
+  uint32_t* tilePre;         // prefix of the meshes' 32-sample tiles (nMeshes + 1)
+  uint32_t* work;            // next tile
 };
 
 // Physical words of one hull slab whose reference size (which fixes the face

@@ -33,7 +33,7 @@ void launch_seed_bound(const Level& P, const Dev& D, cudaStream_t s);
 void launch_evaluate(uint32_t stateBase, uint32_t headerOff, uint32_t mode, uint32_t nSeeds, uint32_t jobBase,
                      uint32_t edgePlaneBase, uint32_t edgeStride, const Dev& D, cudaStream_t s);
 void launch_hull(const Level& P, const Dev& D, int width, cudaStream_t s);
-void launch_hd(const HdArgs& A, const Dev& D, cudaStream_t s);
+void launch_hd(const HdArgs& A, const Dev& D, int nSM, cudaStream_t s);
 int hull_blocks_per_sm(int width);
 }  // namespace cuacd
 
@@ -62,6 +62,8 @@ static const uint32_t VIS_MAX = CUACD_VIS_MAX;
 // 256-thread block (narrower blocks for mid-sized parts measured slower: the
 // passes over all points and candidates need the width)
 static const uint32_t SMALL_NV = 1024;
+// Hausdorff targets with at least this many triangles are searched by clusters
+static const uint32_t HD_SCREEN_MIN = 64;
 // parents with more points than this get a block per plan / emit job
 static const uint32_t BIG_JOB_NV = 2048;
 
@@ -686,11 +688,8 @@ struct Tree {
     uint32_t stride = doExport ? 3 * 2 * std::min<uint32_t>((uint32_t)cfg.hullMaxVerts, maxNv) : 0;
     if ((uint64_t)tTop + (uint64_t)n * stride > cfg.triCap) return fail(CUACD_E_CAPACITY, "hull export exceeds triangle pool");
     // sample scratch of the fused Hausdorff (tree.ts:686-698)
-    std::vector<uint32_t> capOff, capN;
-    uint64_t totalCap = 0;
-    uint32_t maxSide = 0;
+    std::vector<uint32_t> capN;
     if (withHd) {
-      capOff.resize(2 * n);
       capN.resize(2 * n);
       uint64_t off = 0;
       for (int k = 0; k < n; k++) {
@@ -699,12 +698,10 @@ struct Tree {
         uint64_t cap = 2 * (2 * res + std::max<uint64_t>(m[k].nt, 2ull * m[k].nv) + 16);
         if (3 * (off + cap) > cfg.scratchWords) return fail(CUACD_E_SCRATCH, "hausdorff sample scratch exceeds capacity");
         uint32_t ca = (uint32_t)(cap / 2), cb = (uint32_t)(cap - cap / 2);
-        capOff[k] = (uint32_t)off; capN[k] = ca;
-        capOff[n + k] = (uint32_t)(off + ca); capN[n + k] = cb;
+        capN[k] = ca;
+        capN[n + k] = cb;
         off += cap;
-        maxSide = std::max(maxSide, std::max(ca, cb));
       }
-      totalCap = off;
     }
     CK(cudaMemcpyAsync(D.parts, parts.data(), (size_t)n * sizeof(PartDesc), cudaMemcpyHostToDevice, stream));
     if (withHd) CK(cudaMemsetAsync(D.parts + n, 0, (size_t)n * sizeof(PartDesc), stream));
@@ -724,7 +721,7 @@ struct Tree {
         triCap[k] = m[k].nt;
         triCap[n + k] = stride / 3;
       }
-      if ((rc = runHd((uint32_t)n, 0, capOff, capN, totalCap, maxSide, triCap))) return rc;
+      if ((rc = runHd((uint32_t)n, 0, capN, triCap))) return rc;
     }
     CK(cudaEventRecord(ev1, stream));
     CK(cudaGetLastError());
@@ -809,58 +806,61 @@ struct Tree {
     }
     return area;
   }
-  // triCap: per mesh, an upper bound on its triangles (the screen's data)
-  int runHd(uint32_t nPairs, uint32_t partBase, const std::vector<uint32_t>& capOff, const std::vector<uint32_t>& capN,
-            uint64_t totalCap, uint32_t maxSide, const std::vector<uint32_t>& triCap) {
-    const size_t metaBytes = (size_t)(4 * 2 * nPairs) * 4;
-    std::vector<uint32_t> hm(8 * nPairs, 0u);
-    std::memcpy(hm.data(), capOff.data(), 4ull * 2 * nPairs);
-    std::memcpy(hm.data() + 2 * nPairs, capN.data(), 4ull * 2 * nPairs);
+  // triCap: per mesh, an upper bound on its triangles
+  int runHd(uint32_t nPairs, uint32_t partBase, const std::vector<uint32_t>& capN, const std::vector<uint32_t>& triCap) {
+    const uint32_t nm = 2 * nPairs;
+    // sample capacities, triangle offsets (host) | sample counts, tile prefix, work counter (device)
+    std::vector<uint32_t> hm(2 * (size_t)nm);
+    std::memcpy(hm.data(), capN.data(), 4ull * nm);
     uint64_t nTri = 0;
-    for (uint32_t m = 0; m < 2 * nPairs; m++) {
-      hm[6 * nPairs + m] = (uint32_t)nTri;
-      nTri += triCap[m];
+    for (uint32_t m = 0; m < nm; m++) {
+      hm[nm + m] = (uint32_t)nTri;
+      nTri += ((uint64_t)triCap[m] + 31) & ~31ull;  // clusters of 32 start at multiples of 32
     }
     if (nTri > 0xffffffffull) return fail(CUACD_E_CAPACITY, "hausdorff batch: too many triangles");
-    const size_t sampOff = (metaBytes + 255) & ~(size_t)255;
-    const size_t triBOff = (sampOff + (size_t)totalCap * 16 + 255) & ~(size_t)255;
-    const size_t triGOff = triBOff + (size_t)nTri * 32;
-    int rc = bHd.ensure(triGOff + (size_t)nTri * 48 + 16);
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    const size_t cOff = up((4 * (size_t)nm + 2) * 4), gOff = cOff + (size_t)nTri * 16, boxOff = gOff + (size_t)nTri * 48;
+    const size_t cntOff = boxOff + (size_t)nTri, soffOff = cntOff + (size_t)nTri * 4, permOff = soffOff + (size_t)nTri * 4;
+    int rc = bHd.ensure(permOff + (size_t)nTri * 4 + 16);
     if (rc) return rc;
+    uint8_t* d = (uint8_t*)bHd.p;
     uint32_t* meta = (uint32_t*)bHd.p;
     if ((rc = hMeta.ensure(hm.size() * 4))) return rc;
     std::memcpy(hMeta.p, hm.data(), hm.size() * 4);
     CK(cudaMemcpyAsync(meta, hMeta.p, hm.size() * 4, cudaMemcpyHostToDevice, stream));
-    CK(cudaMemsetAsync(D.ctr + CTR_HD_EXACT, 0, 8 * 4, stream));
+    CK(cudaMemsetAsync(D.ctr + CTR_HD_EXACT, 0, 4 * 4, stream));
     HdArgs A;
     A.nPairs = nPairs;
-    A.nMeshes = 2 * nPairs;
-    A.capOff = meta;
-    A.capN = meta + 2 * nPairs;
-    A.ns = meta + 4 * nPairs;
-    A.triOff = meta + 6 * nPairs;
-    A.samples = (float4*)((uint8_t*)bHd.p + sampOff);
-    A.triB = (uint4*)((uint8_t*)bHd.p + triBOff);
-    A.triG = (float4*)((uint8_t*)bHd.p + triGOff);
+    A.nMeshes = nm;
+    A.capN = meta;
+    A.triOff = meta + nm;
+    A.ns = meta + 2 * nm;
+    A.tilePre = meta + 3 * nm;
+    A.work = meta + 4 * nm + 1;
+    A.triC = (float4*)(d + cOff);
+    A.triG = (float4*)(d + gOff);
+    A.box = (float4*)(d + boxOff);
+    A.cnt = (uint32_t*)(d + cntOff);
+    A.soff = (uint32_t*)(d + soffOff);
+    A.perm = (uint32_t*)(d + permOff);
     A.partBase = partBase;
-    A.maxSide = maxSide;
-    A.screenMin = cfg.hdScreenMinTris == 0 ? 256u : (cfg.hdScreenMinTris < 0 ? 0xffffffffu : (uint32_t)cfg.hdScreenMinTris);
-    launch_hd(A, D, stream);
+    A.screenMin = cfg.hdScreenMinTris == 0 ? HD_SCREEN_MIN : (cfg.hdScreenMinTris < 0 ? 0xffffffffu : (uint32_t)cfg.hdScreenMinTris);
+    launch_hd(A, D, nSM, stream);
     hdStatsPending = true;
     return 0;
   }
-  // statistics of the last Hausdorff batch's screen: exact distances,
-  // screened sample-triangle pairs, timeout flag
+  // statistics of the last Hausdorff batch's cluster search: exact distances,
+  // sample-triangle pairs of the clusters visited, and 0 (the search waits on nothing)
   bool hdStatsPending = false;
   uint64_t hdStats[3] = {0, 0, 0};
   int readHdStats() {
     if (!hdStatsPending) return 0;
-    uint32_t w[6];
+    uint32_t w[4];
     CK(cudaStreamSynchronize(stream));
     CK(cudaMemcpy(w, D.ctr + CTR_HD_EXACT, sizeof w, cudaMemcpyDeviceToHost));
     hdStats[0] = (uint64_t)w[0] | ((uint64_t)w[1] << 32);
     hdStats[1] = (uint64_t)w[2] | ((uint64_t)w[3] << 32);
-    hdStats[2] = w[4];
+    hdStats[2] = 0;
     hdStatsPending = false;
     return 0;
   }
@@ -884,24 +884,22 @@ struct Tree {
       uint64_t res = std::max<uint64_t>(1000, (uint64_t)std::floor(2000.0 * mesh_area(m)));
       return 2 * res + m.nt + 16;
     };
-    std::vector<uint32_t> capOff(2 * n), capN(2 * n);
+    std::vector<uint32_t> capN(2 * n);
     uint64_t off = 0;
-    uint32_t maxSide = 0;
     for (int k = 0; k < n; k++) {
       uint64_t cap = 2 * std::max(bound(a[k]), bound(b[k]));
       if (3 * (off + cap) > cfg.scratchWords) return fail(CUACD_E_SCRATCH, "hausdorff sample scratch exceeds capacity");
       uint32_t ca = (uint32_t)(cap / 2), cb = (uint32_t)(cap - cap / 2);
-      capOff[k] = (uint32_t)off; capN[k] = ca;
-      capOff[n + k] = (uint32_t)(off + ca); capN[n + k] = cb;
+      capN[k] = ca;
+      capN[n + k] = cb;
       off += cap;
-      maxSide = std::max(maxSide, std::max(ca, cb));
     }
     CK(cudaMemcpyAsync(D.parts, parts.data(), 2ull * n * sizeof(PartDesc), cudaMemcpyHostToDevice, stream));
     CK(cudaMemsetAsync(D.ctr + CTR_HD, 0, 4ull * n, stream));
     CK(cudaEventRecord(ev0, stream));
     std::vector<uint32_t> triCap(2 * n);
     for (int k = 0; k < 2 * n; k++) triCap[k] = all[k].nt;
-    if ((rc = runHd((uint32_t)n, 0, capOff, capN, off, maxSide, triCap))) return rc;
+    if ((rc = runHd((uint32_t)n, 0, capN, triCap))) return rc;
     CK(cudaEventRecord(ev1, stream));
     CK(cudaGetLastError());
     if ((rc = hRead.ensure(4ull * n))) return rc;

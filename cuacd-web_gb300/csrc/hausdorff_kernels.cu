@@ -6,15 +6,23 @@
 // step-th (or every even) triangle that gets none; barycentrics from a Wang
 // hash of t * 65537 + k.
 //
-// GB300 design: each mesh is sampled exactly once by one group (the
-// reference re-samples both meshes in every 256-sample slice); the total
-// area is summed in double so the per-triangle counts do not depend on a
-// reduction order. The distance pass gives each thread one sample and
-// streams the other mesh's triangles through shared memory in tiles; the
-// squared distance maximum goes to one word per pair by an atomic max on
-// its (non-negative) float bits.
-#include <cuda_bf16.h>
-
+// The result of a pair is the largest, over the samples of both sides, of
+// the smallest squared distance tri_sq(sample, triangle of the other side).
+// Neither the order of the triangles nor that of the samples matters, and a
+// sample or triangle that provably cannot decide it need not be looked at:
+//   k_hd_prep   a block per mesh: areas, sample counts, the triangles in
+//               Morton order of their centroids in clusters of 32 with
+//               bounding boxes, and the samples' prefix in that order;
+//   k_hd_tiles  the work list: 32 consecutive samples of a mesh each;
+//   k_hd_near   a warp per 32 samples: the clusters whose box may hold a
+//               nearest triangle, nearest box first, a centroid test per
+//               triangle, tri_sq for the survivors; a sample whose distance
+//               cannot exceed the pair's largest one so far is dropped.
+// What bounds it: dependent loads and divergence in k_hd_near. Against a
+// tensor-core bound of every sample-triangle pair, whose epilogue was bound by
+// instruction issue: 24 cut halves of 1.5-30k triangles with their hulls
+// 11.4 -> 0.86 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.66 ms, 192
+// pairs of 160-6,000 triangles 5.8 + 0.71 -> 0.50 ms.
 #include "cuacd_dev.cuh"
 
 namespace cuacd {
@@ -30,63 +38,6 @@ __device__ __forceinline__ uint32_t wang(uint32_t s) {
 __device__ __forceinline__ float tri_area(f3 a, f3 b, f3 c) {
   f3 n = cross(b - a, c - a);
   return 0.5f * sqrtf(dot(n, n));
-}
-
-template <int G>
-__global__ void __launch_bounds__(256) k_hd_sample(const HdArgs A, const Dev D) {
-  __shared__ GrpSmem gsm[Grp<G>::PER_BLOCK];
-  const int gi = Grp<G>::gid(), lid = Grp<G>::lid();
-  GrpSmem& sm = gsm[gi];
-  const uint32_t m = blockIdx.x * Grp<G>::PER_BLOCK + gi;
-  if (m >= A.nMeshes) return;
-  const PartDesc pd = D.parts[A.partBase + m];
-  const uint32_t nt = pd.nt, cap = A.capN[m];
-  float4* out = A.samples + A.capOff[m];
-  if (nt == 0) {
-    if (lid == 0) A.ns[m] = 0;
-    return;
-  }
-  double a = 0.0;
-  for (uint32_t t = lid; t < nt; t += G) {
-    const uint32_t* tr = D.T + pd.tOff + 3 * (size_t)t;
-    a += (double)tri_area(ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[0]), ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[1]),
-                          ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[2]));
-  }
-  const float total = (float)grp_sum_d<G>(a, sm);
-  float res = floorf(2000.0f * total);
-  if (res < 1000.0f) res = 1000.0f;
-  const uint32_t step = (float)nt > res ? nt / (uint32_t)res : 0;
-  uint32_t run = 0;
-  for (uint32_t c = 0; c * G < nt; c++) {
-    const uint32_t t = c * G + lid;
-    uint32_t N = 0;
-    f3 pa = mk3(0.f, 0.f, 0.f), pb = pa, pc = pa;
-    if (t < nt) {
-      const uint32_t* tr = D.T + pd.tOff + 3 * (size_t)t;
-      pa = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[0]);
-      pb = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[1]);
-      pc = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[2]);
-      const float ta = tri_area(pa, pb, pc);
-      const uint32_t areaCount = total > 1e-20f ? (uint32_t)floorf((res / total) * ta) : 0u;
-      if ((float)nt > res) N = areaCount > 0 ? areaCount : ((t % max(step, 1u)) == 0 ? 1u : 0u);
-      else N = areaCount > 0 ? areaCount : ((t % 2u) == 0 ? 1u : 0u);
-    }
-    uint32_t tot;
-    const uint32_t pre = grp_scan_u<G>(N, &tot, sm);
-    for (uint32_t k = 0; k < N; k++) {
-      const uint32_t idx = run + pre + k;
-      if (idx >= cap) break;
-      const uint32_t ha = wang(t * 65537u + k);
-      const uint32_t hb = wang(ha + 0x9e3779b9u);
-      const float ra = (float)(ha & 0xFFFFFFu) / (float)0xFFFFFFu;
-      const float rb = (float)(hb & 0xFFFFFFu) / (float)0xFFFFFFu;
-      const float sqa = sqrtf(ra);
-      const f3 s = ((1.0f - sqa) * pa + (sqa * (1.0f - rb)) * pb) + (sqa * rb) * pc;
-      out[idx] = make_float4(s.x, s.y, s.z, 0.0f);
-    }
-    run += tot;
-  }
-  if (lid == 0) A.ns[m] = min(run, cap);
 }
 
 // squared distance from p to triangle (a, b, c) (hausdorff_shader.ts:32-52)
@@ -118,339 +69,514 @@ __device__ __forceinline__ float tri_sq(f3 p, f3 a, f3 b, f3 c) {
   return fminf(seg_sq(p, a, b), fminf(seg_sq(p, b, c), seg_sq(p, c, a)));
 }
 
-#define HD_TILE 128
+// ---------------------------------------------------------------------------
+// prep
 
-// grid: x = sample tile, y = pair, z = direction (0: A samples vs B, 1: B vs A)
-__global__ void __launch_bounds__(HD_TILE) k_hd_dist(const HdArgs A, const Dev D) {
-  __shared__ float tv[HD_TILE][9];
-  __shared__ float red[HD_TILE / 32];
-  const uint32_t pair = blockIdx.y, dir = blockIdx.z;
-  const uint32_t src = dir == 0 ? pair : A.nPairs + pair;
-  const uint32_t dst = dir == 0 ? A.nPairs + pair : pair;
-  const PartDesc ps = D.parts[A.partBase + src], pt = D.parts[A.partBase + dst];
-  if (ps.nt == 0 || pt.nt == 0 || pt.nt >= A.screenMin) return;
-  const uint32_t ns = A.ns[src];
-  const uint32_t s0 = blockIdx.x * HD_TILE;
-  if (s0 >= ns) return;
-  const uint32_t si = s0 + threadIdx.x;
-  f3 p = mk3(0.f, 0.f, 0.f);
-  if (si < ns) {
-    float4 q = A.samples[A.capOff[src] + si];
-    p = mk3(q.x, q.y, q.z);
+// threads of a prep block, and the triangles whose areas it computes between
+// two barriers: warp 0 adds them while the other warps compute the next ones
+#define HD_PREP 512u
+#define HD_CHUNK ((HD_PREP - 32u) * 4u)
+// Morton cells, 16 along the mesh's largest extent: a 60k-triangle surface
+// occupies about 1,500 of them, so a cluster of 32 spans about one cell
+#define HD_CELLS 4096u
+static_assert(HD_CHUNK % 32 == 0 && 2 * HD_CHUNK <= HD_CELLS, "two area chunks share the cell counters' words");
+
+__device__ __forceinline__ uint32_t spread4(uint32_t v) {
+  return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4) | ((v & 8u) << 6);
+}
+// floats as signed integers in the same order
+__device__ __forceinline__ int f_ord(float x) {
+  const int b = __float_as_int(x);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float f_unord(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
+
+__device__ __forceinline__ f3 centroid(f3 a, f3 b, f3 c) {
+  return mk3((a.x + b.x + c.x) / 3.0f, (a.y + b.y + c.y) / 3.0f, (a.z + b.z + c.z) / 3.0f);
+}
+__device__ __forceinline__ void tri_load(const Dev& D, const PartDesc& pd, uint32_t t, f3& a, f3& b, f3& c) {
+  const uint32_t* tr = D.T + pd.tOff + 3 * (size_t)t;
+  const uint32_t i = tr[0], j = tr[1], k = tr[2];
+  a = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)i);
+  b = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)j);
+  c = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)k);
+}
+// inclusive scan over the block's HD_PREP threads; *total = the sum. The
+// trailing barrier of the caller's loop separates two calls' use of ws.
+__device__ __forceinline__ uint32_t prep_scan(uint32_t v, uint32_t* ws, uint32_t* total) {
+  const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const uint32_t inc = warp_incl_u(v, lane);
+  if (lane == 31) ws[w] = inc;
+  __syncthreads();
+  const uint32_t x = lane < HD_PREP / 32 ? ws[lane] : 0u;
+  const uint32_t xi = warp_incl_u(x, lane);
+  *total = __shfl_sync(FULLMASK, xi, 31);
+  const uint32_t before = __shfl_sync(FULLMASK, xi - x, w);
+  __syncthreads();
+  return before + inc;
+}
+
+// One block per mesh. The total area is the double sum the sampling rule's
+// counts were always made from: lane l of one warp adds the areas of
+// triangles l, l + 32, ... in order and the lanes are folded in a tree, so
+// the counts do not depend on the block's shape. That warp only adds, from
+// shared memory; the gathers and square roots of the next chunk overlap it.
+// 24 cut halves and their hulls, the largest about 40k triangles, take 0.40
+// ms; one warp per mesh took 1.87 ms for the samples and a block of 256
+// threads another 0.15 ms for the triangles' data.
+__global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D) {
+  __shared__ uint32_t cells[HD_CELLS];
+  __shared__ uint32_t ws[32];
+  __shared__ float box[6][HD_PREP / 32];
+  __shared__ float sTotal;
+  const uint32_t m = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const PartDesc pd = D.parts[A.partBase + m];
+  const uint32_t nt = pd.nt, cap = A.capN[m];
+  if (nt == 0) {
+    if (tid == 0) A.ns[m] = 0;
+    return;
   }
-  float best = 1e30f;
-  for (uint32_t t0 = 0; t0 < pt.nt; t0 += HD_TILE) {
-    const uint32_t t = t0 + threadIdx.x;
-    __syncthreads();
-    if (t < pt.nt) {
-      const uint32_t* tr = D.T + pt.tOff + 3 * (size_t)t;
+  uint32_t* cnt = A.cnt + A.triOff[m];
+  uint32_t* soff = A.soff + A.triOff[m];
+  uint32_t* perm = A.perm + A.triOff[m];
+  // areas, their sum and the centroids' box
+  {
+    float* area = reinterpret_cast<float*>(cells);
+    f3 lo = mk3(3.4e38f, 3.4e38f, 3.4e38f), hi = mk3(-3.4e38f, -3.4e38f, -3.4e38f);
+    double sum = 0.0;
+    uint32_t buf = 0;
+    for (uint32_t c0 = 0; c0 < nt; c0 += HD_CHUNK, buf ^= HD_CHUNK) {
+      if (warp > 0) {
 #pragma unroll
-      for (int k = 0; k < 3; k++) {
-        f3 v = ldv(D.V, (size_t)pt.vOff + 3 * (size_t)tr[k]);
-        tv[threadIdx.x][3 * k] = v.x; tv[threadIdx.x][3 * k + 1] = v.y; tv[threadIdx.x][3 * k + 2] = v.z;
+        for (uint32_t u = 0; u < 4; u++) {
+          const uint32_t t = c0 + u * (HD_PREP - 32u) + tid - 32u;
+          if (t < nt) {
+            f3 a, b, c;
+            tri_load(D, pd, t, a, b, c);
+            const float ar = tri_area(a, b, c);
+            area[buf + t - c0] = ar;
+            cnt[t] = __float_as_uint(ar);
+            const f3 g = centroid(a, b, c);
+            lo = vmin3(lo, g);
+            hi = vmax3(hi, g);
+          }
+        }
+      }
+      __syncthreads();
+      if (warp == 0) {
+        const uint32_t n = min(HD_CHUNK, nt - c0);
+        for (uint32_t k = lane; k < n; k += 32) sum += (double)area[buf + k];
       }
     }
+    if (warp == 0) {
+      const float total = (float)warp_sum_d(sum);
+      if (lane == 0) sTotal = total;
+    }
+    lo.x = warp_min_f(lo.x); lo.y = warp_min_f(lo.y); lo.z = warp_min_f(lo.z);
+    hi.x = warp_max_f(hi.x); hi.y = warp_max_f(hi.y); hi.z = warp_max_f(hi.z);
+    if (lane == 0) {
+      box[0][warp] = lo.x; box[1][warp] = lo.y; box[2][warp] = lo.z;
+      box[3][warp] = hi.x; box[4][warp] = hi.y; box[5][warp] = hi.z;
+    }
     __syncthreads();
-    const uint32_t cnt = min((uint32_t)HD_TILE, pt.nt - t0);
-    for (uint32_t k = 0; k < cnt; k++) {
-      const float* w = tv[k];
-      best = fminf(best, tri_sq(p, mk3(w[0], w[1], w[2]), mk3(w[3], w[4], w[5]), mk3(w[6], w[7], w[8])));
+  }
+  f3 lo = mk3(box[0][0], box[1][0], box[2][0]), hi = mk3(box[3][0], box[4][0], box[5][0]);
+  for (uint32_t w = 1; w < HD_PREP / 32; w++) {
+    lo = vmin3(lo, mk3(box[0][w], box[1][w], box[2][w]));
+    hi = vmax3(hi, mk3(box[3][w], box[4][w], box[5][w]));
+  }
+  const float inv = 16.0f / fmaxf(fmaxf(fmaxf(hi.x - lo.x, hi.y - lo.y), hi.z - lo.z), 1e-30f);
+  for (uint32_t k = tid; k < HD_CELLS; k += HD_PREP) cells[k] = 0;
+  __syncthreads();
+  // sample counts, cut off at the mesh's capacity in triangle order, and the
+  // triangles' cells
+  const float total = sTotal;
+  float res = floorf(2000.0f * total);
+  if (res < 1000.0f) res = 1000.0f;
+  const uint32_t step = (float)nt > res ? nt / (uint32_t)res : 0;
+  uint32_t run = 0;
+  for (uint32_t c0 = 0; c0 < nt; c0 += 4 * HD_PREP) {
+    uint32_t N[4], sum = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      const uint32_t t = c0 + 4 * tid + u;
+      N[u] = 0;
+      if (t < nt) {
+        const float ta = __uint_as_float(cnt[t]);
+        const uint32_t areaCount = total > 1e-20f ? (uint32_t)floorf((res / total) * ta) : 0u;
+        if ((float)nt > res) N[u] = areaCount > 0 ? areaCount : ((t % max(step, 1u)) == 0 ? 1u : 0u);
+        else N[u] = areaCount > 0 ? areaCount : ((t % 2u) == 0 ? 1u : 0u);
+        f3 a, b, c;
+        tri_load(D, pd, t, a, b, c);
+        const f3 g = centroid(a, b, c);
+        const uint32_t x = min((uint32_t)fmaxf((g.x - lo.x) * inv, 0.0f), 15u);
+        const uint32_t y = min((uint32_t)fmaxf((g.y - lo.y) * inv, 0.0f), 15u);
+        const uint32_t z = min((uint32_t)fmaxf((g.z - lo.z) * inv, 0.0f), 15u);
+        const uint32_t code = spread4(x) | (spread4(y) << 1) | (spread4(z) << 2);
+        soff[t] = code;
+        atomicAdd(cells + code, 1u);
+      }
+      sum += N[u];
+    }
+    uint32_t tot;
+    uint32_t at = run + prep_scan(sum, ws, &tot) - sum;
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      const uint32_t t = c0 + 4 * tid + u;
+      if (t < nt) cnt[t] = at < cap ? min(N[u], cap - at) : 0u;
+      at += N[u];
+    }
+    run += tot;
+  }
+  if (tid == 0) A.ns[m] = min(run, cap);
+  __syncthreads();
+  // counting sort by cell (the order within a cell does not matter)
+  {
+    constexpr uint32_t PER = HD_CELLS / HD_PREP;
+    uint32_t sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < PER; k++) sum += cells[PER * tid + k];
+    uint32_t tot;
+    uint32_t at = prep_scan(sum, ws, &tot) - sum;
+#pragma unroll
+    for (uint32_t k = 0; k < PER; k++) {
+      const uint32_t v = cells[PER * tid + k];
+      cells[PER * tid + k] = at;
+      at += v;
     }
   }
-  float worst = si < ns ? best : 0.0f;
-  worst = warp_max_f(worst);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = worst;
   __syncthreads();
-  if (threadIdx.x == 0) {
-    float w = red[0];
-    for (int i = 1; i < HD_TILE / 32; i++) w = fmaxf(w, red[i]);
-    atomicMax(D.ctr + CTR_HD + pair, __float_as_uint(w));
+  for (uint32_t t = tid; t < nt; t += HD_PREP) perm[atomicAdd(cells + soff[t], 1u)] = t;
+  __syncthreads();
+  // the sorted triangles, the clusters' boxes and the samples' prefix
+  const size_t base = A.triOff[m];
+  run = 0;
+  for (uint32_t c0 = 0; c0 < nt; c0 += 4 * HD_PREP) {
+    const uint32_t i0 = c0 + 128 * warp + lane;
+    uint32_t N[4], off[4], wsum = 0;
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++) {
+      const uint32_t i = i0 + 32 * u;
+      N[u] = 0;
+      f3 blo = mk3(3.4e38f, 3.4e38f, 3.4e38f), bhi = mk3(-3.4e38f, -3.4e38f, -3.4e38f);
+      if (i < nt) {
+        const uint32_t t = perm[i];
+        f3 a, b, c;
+        tri_load(D, pd, t, a, b, c);
+        N[u] = cnt[t];
+        const f3 g = centroid(a, b, c);
+        const float ra = sqrtf(dot(a - g, a - g)), rb = sqrtf(dot(b - g, b - g)), rc = sqrtf(dot(c - g, c - g));
+        // radius rounded up past its float32 error
+        float r = fmaxf(fmaxf(ra, rb), rc) * 1.00001f + 1e-30f;
+        blo = vmin3(vmin3(a, b), c);
+        bhi = vmax3(vmax3(a, b), c);
+        // a triangle that is not finite is never culled (inf - inf and
+        // NaN - NaN are NaN, which is not below 3.4e38)
+        const float sumAbs = (l1(a) + l1(b)) + l1(c);
+        if (!(sumAbs < 3.4e38f)) {
+          r = INFINITY;
+          blo = mk3(-INFINITY, -INFINITY, -INFINITY);
+          bhi = mk3(INFINITY, INFINITY, INFINITY);
+        }
+        float4* G = A.triG + 3 * (base + i);
+        G[0] = make_float4(a.x, a.y, a.z, 0.0f);
+        G[1] = make_float4(b.x, b.y, b.z, 0.0f);
+        G[2] = make_float4(c.x, c.y, c.z, 0.0f);
+        A.triC[base + i] = make_float4(g.x, g.y, g.z, r);
+      }
+      if (i - lane < nt) {  // the warp's cluster holds a triangle
+        const float4 l = make_float4(f_unord(__reduce_min_sync(FULLMASK, f_ord(blo.x))),
+                                     f_unord(__reduce_min_sync(FULLMASK, f_ord(blo.y))),
+                                     f_unord(__reduce_min_sync(FULLMASK, f_ord(blo.z))), 0.0f);
+        const float4 h = make_float4(f_unord(__reduce_max_sync(FULLMASK, f_ord(bhi.x))),
+                                     f_unord(__reduce_max_sync(FULLMASK, f_ord(bhi.y))),
+                                     f_unord(__reduce_max_sync(FULLMASK, f_ord(bhi.z))), 0.0f);
+        if (lane == 0) {
+          float4* B = A.box + 2 * (size_t)((base + i) >> 5);
+          B[0] = l;
+          B[1] = h;
+        }
+      }
+      const uint32_t inc = warp_incl_u(N[u], lane);
+      off[u] = wsum + inc - N[u];
+      wsum += __shfl_sync(FULLMASK, inc, 31);
+    }
+    uint32_t tot;
+    // every lane holds its warp's total: scan the warps through lane 31's slot
+    const uint32_t inc = prep_scan(lane == 31 ? wsum : 0u, ws, &tot);
+    const uint32_t before = __shfl_sync(FULLMASK, inc, 31) - wsum;
+#pragma unroll
+    for (uint32_t u = 0; u < 4; u++)
+      if (i0 + 32 * u < nt) soff[i0 + 32 * u] = run + before + off[u];
+    run += tot;
+  }
+}
+
+// tiles of 32 samples per mesh: their prefix over the meshes, and the work
+// counter
+__global__ void __launch_bounds__(1024) k_hd_tiles(const HdArgs A, const Dev D) {
+  __shared__ uint32_t ws[32];
+  const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+  uint32_t run = 0;
+  for (uint32_t c0 = 0; c0 < A.nMeshes; c0 += 1024) {
+    const uint32_t m = c0 + tid;
+    uint32_t n = 0;
+    if (m < A.nMeshes) {
+      const uint32_t dst = m < A.nPairs ? m + A.nPairs : m - A.nPairs;
+      const bool both = D.parts[A.partBase + m].nt != 0 && D.parts[A.partBase + dst].nt != 0;
+      n = both ? (A.ns[m] + 31) / 32 : 0u;
+    }
+    const uint32_t inc = warp_incl_u(n, lane);
+    if (lane == 31) ws[w] = inc;
+    __syncthreads();
+    const uint32_t x = ws[lane];
+    const uint32_t xi = warp_incl_u(x, lane);
+    const uint32_t before = __shfl_sync(FULLMASK, xi - x, w);
+    if (m < A.nMeshes) A.tilePre[m] = run + before + inc - n;
+    run += __shfl_sync(FULLMASK, xi, 31);
+    __syncthreads();
+  }
+  if (tid == 0) {
+    A.tilePre[A.nMeshes] = run;
+    *A.work = 0;
   }
 }
 
 // ---------------------------------------------------------------------------
-// Tensor-core screen for target meshes of at least A.screenMin triangles.
-//
-// For sample p and triangle t with centroid c and bounding radius r,
-// dist(p, t) >= |p - c| - r and the smallest distance is at most |p - c|.
-// |p - c|^2 = |p|^2 + (|c|^2 - 2 p . c), and the bracket for 128 samples x
-// 128 triangles is one tcgen05 MMA (kind::f16, bf16 operands, fp32
-// accumulation in TMEM) with K = 16: each coordinate is split into a bf16
-// high part and a bf16 low part, and the 16 products of the row
-// [p_hi, p_hi, p_lo, p_lo, 1, 1, 0, 0] with [-2c_hi, -2c_lo, -2c_hi, -2c_lo,
-// |c|^2_hi, |c|^2_lo, 0, 0] (three lanes per point) give -2 p . c + |c|^2 to
-// about 2^-16 of its terms. Each thread owns one sample (one TMEM lane), reads
-// its row of distances and computes the exact float32 distance (tri_sq, the
-// same function as the exhaustive kernel) only for triangles whose lower
-// bound, with the screen's error bound and a 1e-3 relative margin, does not
-// exceed the running minimum or the smallest upper bound: the triangle that
-// attains the exhaustive minimum is never skipped, so the result is that
-// minimum bit for bit.
-#define HDS_M 128u          // samples per CTA = TMEM lanes
-#define HDS_N 128u          // triangles per MMA = TMEM columns (fp32)
+// nearest triangles
 
-__device__ __forceinline__ uint32_t bf16_bits(float x) { return (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(x)); }
-__device__ __forceinline__ float bf16_val(uint32_t b) { return __bfloat162float(__ushort_as_bfloat16((unsigned short)b)); }
-__device__ __forceinline__ void bf16_split(float x, uint32_t& hi, uint32_t& lo) {
-  hi = bf16_bits(x);
-  lo = bf16_bits(x - bf16_val(hi));
-}
-__device__ __forceinline__ uint32_t pack2(uint32_t lo16, uint32_t hi16) { return lo16 | (hi16 << 16); }
+#define HD_NEAR 128u
 
-// one block per mesh: the screen data of its triangles
-__global__ void __launch_bounds__(256) k_hd_prep(const HdArgs A, const Dev D) {
-  const uint32_t m = blockIdx.x;
-  if (m >= A.nMeshes) return;
-  const PartDesc pd = D.parts[A.partBase + m];
-  const uint32_t base = A.triOff[m];
-  for (uint32_t t = threadIdx.x; t < pd.nt; t += blockDim.x) {
-    const uint32_t* tr = D.T + pd.tOff + 3 * (size_t)t;
-    const f3 a = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[0]);
-    const f3 b = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[1]);
-    const f3 c = ldv(D.V, (size_t)pd.vOff + 3 * (size_t)tr[2]);
-    const f3 g = mk3((a.x + b.x + c.x) / 3.0f, (a.y + b.y + c.y) / 3.0f, (a.z + b.z + c.z) / 3.0f);
-    const float ra = sqrtf(dot(a - g, a - g)), rb = sqrtf(dot(b - g, b - g)), rc = sqrtf(dot(c - g, c - g));
-    // radius rounded up past its float32 error
-    const float r = fmaxf(fmaxf(ra, rb), rc) * 1.00001f + 1e-30f;
-    const float c1 = fabsf(g.x) + fabsf(g.y) + fabsf(g.z);
-    const float cc = dot(g, g);
-    uint32_t h[3], l[3], ch, cl;
-    bf16_split(-2.0f * g.x, h[0], l[0]);
-    bf16_split(-2.0f * g.y, h[1], l[1]);
-    bf16_split(-2.0f * g.z, h[2], l[2]);
-    bf16_split(cc, ch, cl);
-    // K order: [-2c_hi, -2c_lo, -2c_hi, -2c_lo, |c|^2 hi, |c|^2 lo, 0, 0]
-    const uint32_t k16[16] = {h[0], h[1], h[2], l[0], l[1], l[2], h[0], h[1], h[2], l[0], l[1], l[2], ch, cl, 0u, 0u};
-    uint4 r0, r1;
-    r0.x = pack2(k16[0], k16[1]); r0.y = pack2(k16[2], k16[3]); r0.z = pack2(k16[4], k16[5]); r0.w = pack2(k16[6], k16[7]);
-    r1.x = pack2(k16[8], k16[9]); r1.y = pack2(k16[10], k16[11]); r1.z = pack2(k16[12], k16[13]); r1.w = 0u;
-    A.triB[2 * (size_t)(base + t)] = r0;
-    A.triB[2 * (size_t)(base + t) + 1] = r1;
-    A.triG[3 * (size_t)(base + t)] = make_float4(a.x, a.y, a.z, r);
-    A.triG[3 * (size_t)(base + t) + 1] = make_float4(b.x, b.y, b.z, c1);
-    A.triG[3 * (size_t)(base + t) + 2] = make_float4(c.x, c.y, c.z, cc);
+// A sample's state in the culled search. best is the smallest tri_sq so far
+// and ub the smallest squared centroid distance (a centroid is a point of
+// its triangle). The search keeps a triangle unless its bound |p - c| - r, or
+// its cluster's box, is farther than reach(): the smaller of the two with
+// a 1e-3 relative margin, and an absolute one of 3e-10 |p|^2 for distances
+// that cancel far from the origin (coordinates round to 2^-24 of |p|, so
+// squared distances below (1e-3 |p|)^2 may be off by 1e-3 of themselves).
+// Those cover the float32 error of tri_sq, of the centroid and of the
+// radius, so the triangle attaining the smallest tri_sq is always looked at.
+struct HdNear {
+  f3 p;
+  float p2, best, ub;
+  __device__ __forceinline__ float reach() const { return fminf(best, ub) * 1.001f + 3e-10f * p2 + 1e-30f; }
+  // whether the sample can still raise the pair's largest distance: its
+  // smallest tri_sq is at most best, and at most ub with a wider margin
+  __device__ __forceinline__ bool counts(float gmax) const {
+    return best > gmax && !(ub * 1.01f + 3e-9f * p2 < gmax);
   }
+};
+
+__device__ __forceinline__ float warp_box_min(float v) { return f_unord(__reduce_min_sync(FULLMASK, f_ord(v))); }
+__device__ __forceinline__ float warp_box_max(float v) { return f_unord(__reduce_max_sync(FULLMASK, f_ord(v))); }
+// squared gap between two boxes (0 where they overlap)
+__device__ __forceinline__ float box_gap(f3 alo, f3 ahi, float4 blo, float4 bhi) {
+  const float dx = fmaxf(fmaxf(blo.x - ahi.x, alo.x - bhi.x), 0.0f);
+  const float dy = fmaxf(fmaxf(blo.y - ahi.y, alo.y - bhi.y), 0.0f);
+  const float dz = fmaxf(fmaxf(blo.z - ahi.z, alo.z - bhi.z), 0.0f);
+  return dx * dx + dy * dy + dz * dz;
 }
 
-// byte offset of element (row, k) of a K-major bf16 operand tile with K = 16
-// in the canonical no-swizzle layout: 8-row x 16-byte core matrices, the two
-// K halves of an 8-row group 128 bytes apart (leading byte offset), 8-row
-// groups 256 bytes apart (stride byte offset)
-__device__ __forceinline__ uint32_t tile_off(uint32_t row, uint32_t khalf) {
-  return ((row >> 3) * 2 + khalf) * 128 + (row & 7) * 16;
-}
-__device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)(128u >> 4) << 16) | ((uint64_t)(256u >> 4) << 32) |
-         (1ull << 46);
-}
-// instruction descriptor, kind::f16: fp32 accumulator, bf16 A and B, both
-// K-major, N = HDS_N, M = HDS_M
-constexpr uint32_t HDS_IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((HDS_N >> 3) << 17) | ((HDS_M >> 4) << 24);
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// at most 4 CTAs of this kernel per SM (the static shared memory below), so
-// their 4 x 128 TMEM columns never exceed the SM's 512 and allocation never
-// waits
-#define HDS_PAD_BYTES (46u * 1024u)
-
-__global__ void __launch_bounds__(HDS_M) k_hd_screen(const HdArgs A, const Dev D) {
-  __shared__ __align__(1024) uint8_t smem[HDS_PAD_BYTES];
-  uint8_t* sA = smem;                      // 128 rows x 32 bytes
-  uint8_t* sB = smem + HDS_M * 32;         // 128 rows x 32 bytes
-  float* sR = reinterpret_cast<float*>(smem + (HDS_M + HDS_N) * 32);  // per tile triangle: radius, |c|_1, |c|^2
-  float* sC1 = sR + HDS_N;
-  float* sCC = sC1 + HDS_N;
-  uint64_t* mbar = reinterpret_cast<uint64_t*>(sCC + HDS_N);
-  uint32_t* tbase = reinterpret_cast<uint32_t*>(mbar + 1);
-  float* red = reinterpret_cast<float*>(tbase + 1);
-  const uint32_t pair = blockIdx.y, dir = blockIdx.z;
-  const uint32_t src = dir == 0 ? pair : A.nPairs + pair;
-  const uint32_t dst = dir == 0 ? A.nPairs + pair : pair;
-  const PartDesc ps = D.parts[A.partBase + src], pt = D.parts[A.partBase + dst];
-  if (ps.nt == 0 || pt.nt == 0 || pt.nt < A.screenMin) return;
-  const uint32_t ns = A.ns[src];
-  const uint32_t s0 = blockIdx.x * HDS_M;
-  if (s0 >= ns) return;
-  const uint32_t tid = threadIdx.x, warp = tid >> 5;
-  if (warp == 0) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tbase)),
-                 "r"(HDS_N));
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
-  }
-  if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(mbar)));
-    asm volatile("fence.mbarrier_init.release.cluster;");
-  }
-  // this thread's sample as operand row A
-  const uint32_t si = s0 + tid;
-  f3 p = mk3(0.f, 0.f, 0.f);
-  if (si < ns) {
-    const float4 q = A.samples[A.capOff[src] + si];
-    p = mk3(q.x, q.y, q.z);
-  }
-  {
-    uint32_t h[3], l[3];
-    bf16_split(p.x, h[0], l[0]);
-    bf16_split(p.y, h[1], l[1]);
-    bf16_split(p.z, h[2], l[2]);
-    const uint32_t one = bf16_bits(1.0f);
-    // K order: [p_hi, p_hi, p_lo, p_lo, 1, 1, 0, 0]
-    const uint4 r0 = make_uint4(pack2(h[0], h[1]), pack2(h[2], h[0]), pack2(h[1], h[2]), pack2(l[0], l[1]));
-    const uint4 r1 = make_uint4(pack2(l[2], l[0]), pack2(l[1], l[2]), pack2(one, one), 0u);
-    *reinterpret_cast<uint4*>(sA + tile_off(tid, 0)) = r0;
-    *reinterpret_cast<uint4*>(sA + tile_off(tid, 1)) = r1;
-  }
-  const float p2 = dot(p, p);
-  const float p1 = fabsf(p.x) + fabsf(p.y) + fabsf(p.z);
-  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  const uint32_t tmem = *tbase;
-  const uint64_t descA = smem_desc(smem_u32(sA)), descB = smem_desc(smem_u32(sB));
-  const uint32_t base = A.triOff[dst], nt = pt.nt;
-  float best = 3.4e38f, ub = 3.4e38f;
-  uint32_t phase = 0, exact = 0;
-  bool ok = true;
-  for (uint32_t t0 = 0; t0 < nt && ok; t0 += HDS_N) {
-    // triangle rows of this tile (zero rows past the end)
+// Warps take tiles of 32 samples from the work list. Targets below
+// A.screenMin triangles are searched exhaustively; for them the sort's boxes
+// save nothing that the extra steps do not cost.
+__global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D) {
+  __shared__ float4 sCent[HD_NEAR / 32][32];
+  const uint32_t lane = threadIdx.x & 31;
+  float4* cent = sCent[threadIdx.x >> 5];
+  const uint32_t nTiles = A.tilePre[A.nMeshes];
+  unsigned long long nExact = 0, nScreen = 0;
+  for (;;) {
+    uint32_t it = 0;
+    if (lane == 0) it = atomicAdd(A.work, 1u);
+    it = __shfl_sync(FULLMASK, it, 0);
+    if (it >= nTiles) break;
+    // the tile's mesh
+    uint32_t m = 0, mEnd = A.nMeshes;
+    while (mEnd - m > 1) {
+      const uint32_t mid = (m + mEnd) >> 1;
+      if (A.tilePre[mid] <= it) m = mid;
+      else mEnd = mid;
+    }
+    const uint32_t pair = m < A.nPairs ? m : m - A.nPairs;
+    const uint32_t dst = m < A.nPairs ? m + A.nPairs : pair;
+    const uint32_t ns = A.ns[m], s0 = 32 * (it - A.tilePre[m]);
+    const uint32_t tnt = D.parts[A.partBase + dst].nt;
+    const size_t tb = A.triOff[dst];
+    bool active = s0 + lane < ns;
+    HdNear S;
     {
-      const uint32_t t = t0 + tid;
-      uint4 r0 = make_uint4(0, 0, 0, 0), r1 = r0;
-      float rr = 0.f, c1 = 0.f, cc = 0.f;
-      if (t < nt) {
-        r0 = A.triB[2 * (size_t)(base + t)];
-        r1 = A.triB[2 * (size_t)(base + t) + 1];
-        rr = A.triG[3 * (size_t)(base + t)].w;
-        c1 = A.triG[3 * (size_t)(base + t) + 1].w;
-        cc = A.triG[3 * (size_t)(base + t) + 2].w;
+      // the lane's sample (past the end, the last one again: it takes part
+      // in the tile's box only): its triangle is the last whose prefix
+      // does not exceed it
+      const uint32_t s = min(s0 + lane, ns - 1);
+      const size_t sb = A.triOff[m];
+      const uint32_t* soff = A.soff + sb;
+      uint32_t i = 0, iEnd = D.parts[A.partBase + m].nt;
+      while (iEnd - i > 1) {
+        const uint32_t mid = (i + iEnd) >> 1;
+        if (soff[mid] <= s) i = mid;
+        else iEnd = mid;
       }
-      *reinterpret_cast<uint4*>(sB + tile_off(tid, 0)) = r0;
-      *reinterpret_cast<uint4*>(sB + tile_off(tid, 1)) = r1;
-      sR[tid] = rr;
-      sC1[tid] = c1;
-      sCC[tid] = cc;
+      const uint32_t t = A.perm[sb + i], k = s - soff[i];
+      const float4 a4 = A.triG[3 * (sb + i)], b4 = A.triG[3 * (sb + i) + 1], c4 = A.triG[3 * (sb + i) + 2];
+      const f3 pa = xyz(a4), pb = xyz(b4), pc = xyz(c4);
+      const uint32_t ha = wang(t * 65537u + k);
+      const uint32_t hb = wang(ha + 0x9e3779b9u);
+      const float ra = (float)(ha & 0xFFFFFFu) / (float)0xFFFFFFu;
+      const float rb = (float)(hb & 0xFFFFFFu) / (float)0xFFFFFFu;
+      const float sqa = sqrtf(ra);
+      S.p = ((1.0f - sqa) * pa + (sqa * (1.0f - rb)) * pb) + (sqa * rb) * pc;
     }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    if (tid == 0) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      asm volatile(
-          "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-          "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-          "l"(descA), "l"(descB), "r"(HDS_IDESC), "r"(0u));
-      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-                       smem_u32(mbar))
-                   : "memory");
+    uint32_t* gmaxAt = D.ctr + CTR_HD + pair;
+    const float4* G = A.triG + 3 * tb;
+    if (tnt < A.screenMin) {
+      float best = 1e30f;
+      for (uint32_t t = 0; t < tnt; t++) {
+        const float4 a = G[3 * t], b = G[3 * t + 1], c = G[3 * t + 2];
+        best = fminf(best, tri_sq(S.p, xyz(a), xyz(b), xyz(c)));
+      }
+      const uint32_t worst = __reduce_max_sync(FULLMASK, active ? __float_as_uint(best) : 0u);
+      if (lane == 0) atomicMax(gmaxAt, worst);
+      continue;
     }
-    // the MMA's completion, with a bounded wait
-    bool done = false;
-    for (uint32_t it = 0; it < (1u << 20) && !done; it++) {
-      uint32_t r;
-      asm volatile(
-          "{\n\t.reg .pred q;\n\tmbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\tselp.u32 %0, 1, 0, q;\n\t}"
-          : "=r"(r)
-          : "r"(smem_u32(mbar)), "r"(phase)
-          : "memory");
-      done = r != 0;
-    }
-    phase ^= 1u;
-    ok = __syncthreads_and(done) != 0;
-    if (!ok) {
-      if (tid == 0) atomicExch(D.ctr + CTR_HD_ERR, 1u);
-      break;
-    }
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t cnt = min(HDS_N, nt - t0);
-    for (uint32_t c0 = 0; c0 < cnt; c0 += 32) {
-      uint32_t v[32];
-      const uint32_t taddr = tmem + ((warp * 32u) << 16) + c0;
-      asm volatile(
-          "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-          "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-          : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-            "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-            "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-            "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-          : "r"(taddr));
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      // the 32 columns' bounds (the bound may only be larger than the
-      // final one: best and ub only decrease), then the exact distances of
-      // the survivors
+    S.p2 = dot(S.p, S.p);
+    S.best = 3.4e38f;
+    S.ub = 3.4e38f;
+    const float4* C = A.triC + tb;
+    const float4* B = A.box + 2 * (tb >> 5);
+    const uint32_t nc = (tnt + 31) / 32;
+    // one cluster against the active samples
+    auto visit = [&](uint32_t c) {
+      const uint32_t cn = min(32u, tnt - 32 * c);
+      __syncwarp();
+      cent[lane] = lane < cn ? C[32 * c + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      __syncwarp();
+      const float gmax = __uint_as_float(__ldcg(gmaxAt));
+      // the nearest centroid, its triangle first
+      float dmin = 3.4e38f;
+      uint32_t jmin = 0;
+      for (uint32_t j = 0; j < cn; j++) {
+        const float4 g = cent[j];
+        const f3 d = S.p - mk3(g.x, g.y, g.z);
+        const float d2 = dot(d, d);
+        if (d2 < dmin) { dmin = d2; jmin = j; }
+      }
+      S.ub = fminf(S.ub, dmin);
+      active = active && S.counts(gmax);
+      const unsigned any = __ballot_sync(FULLMASK, active);
+      nScreen += (unsigned long long)__popc(any) * cn;  // the same on every lane
+      if (any == 0) return;
+      auto exact = [&](uint32_t j) {
+        const float4* g = G + 3 * (size_t)(32 * c + j);
+        const float4 a = g[0], b = g[1], cc = g[2];
+        S.best = fminf(S.best, tri_sq(S.p, xyz(a), xyz(b), xyz(cc)));
+        nExact++;
+      };
+      if (active && dmin < 3.4e38f) {
+        exact(jmin);
+        active = S.counts(gmax);
+      }
+      if (__ballot_sync(FULLMASK, active) == 0) return;
+      float rs = sqrtf(S.reach());
       uint32_t keep = 0;
-#pragma unroll
-      for (uint32_t j = 0; j < 32; j++) {
-        const uint32_t k = c0 + j;
-        if (k < cnt) {
-          // |p - c|^2 as screened, and its error bound e = 2^-13 (|p|^2 +
-          // |c|^2 + 2 |p|_1 |c|_1). Derivation (u = 2^-24, bf16 unit
-          // roundoff 2^-8): the hi/lo split leaves |x - x_hi - x_lo| <=
-          // 2^-16 |x| for every coordinate of p and of -2c and for |c|^2, so
-          // the split products miss at most 2^-14 sum|p_i||c_i| + 2^-16
-          // |c|^2; the bf16 x bf16 products are exact in fp32 and the 16-term
-          // accumulation (at most 15 roundings, each at most 2^-23 relative
-          // even if the tensor core truncates) adds at most 1.8e-6 (2
-          // sum|p_i||c_i| + |c|^2); |p|^2 and |c|^2 themselves are fp32 dot
-          // products (3u) and the final add one more u. In total e_true <=
-          // 6.5e-5 sum|p_i||c_i| + 1.8e-5 |c|^2 + 2.4e-7 |p|^2, which e
-          // exceeds by 3.8x, 7x and 500x (sum|p_i||c_i| <= |p|_1 |c|_1);
-          // the fp32 rounding of e, q2 + e and the square roots below are
-          // covered by the 1e-3 relative margin of the comparison. Far from
-          // the origin |p|^2 and -2 p.c cancel and e grows with them: the
-          // screen then keeps more triangles, never a wrong one.
-          const float q2 = p2 + __uint_as_float(v[j]);
-          const float e = 1.220703125e-4f * (p2 + sCC[k] + 2.0f * p1 * sC1[k]);
-          ub = fminf(ub, q2 + e);
-          const float lo = sqrtf(fmaxf(q2 - e, 0.0f)) - sR[k];
-          const float lb2 = lo > 0.0f ? lo * lo : 0.0f;
-          const float bound = fminf(best, ub);
-          if (lb2 <= bound * 1.001f + 1e-10f * (p2 + sCC[k]) + 1e-30f) keep |= 1u << j;
-        }
+      for (uint32_t j = 0; j < cn; j++) {
+        const float4 g = cent[j];
+        const f3 d = S.p - mk3(g.x, g.y, g.z);
+        const float q = rs + g.w;
+        if (!(dot(d, d) > q * q * 1.00001f)) keep |= 1u << j;
       }
+      if (dmin < 3.4e38f) keep &= ~(1u << jmin);
+      if (!active) keep = 0;
       while (keep) {
         const uint32_t j = __ffs(keep) - 1;
         keep &= keep - 1;
-        const float4* g = A.triG + 3 * (size_t)(base + t0 + c0 + j);
-        const float4 a = g[0], b = g[1], c = g[2];
-        best = fminf(best, tri_sq(p, mk3(a.x, a.y, a.z), mk3(b.x, b.y, b.z), mk3(c.x, c.y, c.z)));
-        exact++;
+        const float4 g = cent[j];
+        const f3 d = S.p - mk3(g.x, g.y, g.z);
+        const float q = rs + g.w;
+        if (dot(d, d) > q * q * 1.00001f) continue;
+        exact(j);
+        if (!S.counts(gmax)) {
+          active = false;
+          break;
+        }
+        rs = sqrtf(S.reach());
+      }
+      __syncwarp();
+    };
+    // the tile's box and the cluster whose box is nearest to its centre
+    f3 wlo = mk3(warp_box_min(S.p.x), warp_box_min(S.p.y), warp_box_min(S.p.z));
+    f3 whi = mk3(warp_box_max(S.p.x), warp_box_max(S.p.y), warp_box_max(S.p.z));
+    uint32_t first = 0;
+    {
+      const f3 ctr = 0.5f * (wlo + whi);
+      uint32_t bk = 0xffffffffu, bc = 0;
+      for (uint32_t c = lane; c < nc; c += 32) {
+        const float4 l = B[2 * c], h = B[2 * c + 1];
+        const float dx = 0.5f * (l.x + h.x) - ctr.x, dy = 0.5f * (l.y + h.y) - ctr.y, dz = 0.5f * (l.z + h.z) - ctr.z;
+        const float v = box_gap(ctr, ctr, l, h) + 1e-2f * (dx * dx + dy * dy + dz * dz);
+        const uint32_t k = v >= 0.0f ? __float_as_uint(v) : 0u;
+        if (k < bk) { bk = k; bc = c; }
+      }
+      const uint32_t k = __reduce_min_sync(FULLMASK, bk);
+      first = __reduce_min_sync(FULLMASK, bk == k ? bc : 0xffffffffu);
+    }
+    visit(first);
+    unsigned act = __ballot_sync(FULLMASK, active);
+    float reach = 0.0f;
+    auto shrink = [&]() {  // the box and the reach of the samples left
+      const float inf = INFINITY;
+      wlo = mk3(warp_box_min(active ? S.p.x : inf), warp_box_min(active ? S.p.y : inf), warp_box_min(active ? S.p.z : inf));
+      whi = mk3(warp_box_max(active ? S.p.x : -inf), warp_box_max(active ? S.p.y : -inf), warp_box_max(active ? S.p.z : -inf));
+      reach = __uint_as_float(__reduce_max_sync(FULLMASK, active ? __float_as_uint(S.reach()) : 0u));
+    };
+    if (act) shrink();
+    for (uint32_t c0 = 0; c0 < nc && act; c0 += 32) {
+      const uint32_t c = c0 + lane;
+      float gap = 0.0f;
+      bool need = false;
+      if (c < nc && c != first) {
+        gap = box_gap(wlo, whi, B[2 * c], B[2 * c + 1]);
+        need = !(gap > reach);
+      }
+      unsigned todo = __ballot_sync(FULLMASK, need);
+      while (todo) {
+        // nearest box first
+        const uint32_t key = need ? __float_as_uint(gap) : 0xffffffffu;
+        const uint32_t k = __reduce_min_sync(FULLMASK, key);
+        const uint32_t j = __ffs(__ballot_sync(FULLMASK, key == k && need)) - 1;
+        if (lane == j) need = false;
+        const float4 l = B[2 * (c0 + j)], h = B[2 * (c0 + j) + 1];
+        if (__any_sync(FULLMASK, active && !(box_gap(S.p, S.p, l, h) > S.reach()))) {
+          visit(c0 + j);
+          const unsigned a2 = __ballot_sync(FULLMASK, active);
+          if (a2 == 0) { act = 0; break; }
+          if (a2 != act) {
+            act = a2;
+            shrink();
+          } else {
+            reach = __uint_as_float(__reduce_max_sync(FULLMASK, active ? __float_as_uint(S.reach()) : 0u));
+          }
+          need = need && !(gap > reach);
+        }
+        todo = __ballot_sync(FULLMASK, need);
       }
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    // every thread is done with this tile's radii before the next tile's
-    // rows overwrite them
-    __syncthreads();
+    const uint32_t worst = __reduce_max_sync(FULLMASK, active ? __float_as_uint(S.best) : 0u);
+    if (lane == 0 && worst != 0) atomicMax(gmaxAt, worst);
   }
-  // the tile's largest smallest distance (squared)
-  float worst = (ok && si < ns) ? best : 0.0f;
-  worst = warp_max_f(worst);
-  unsigned long long ex = warp_sum_u(exact);
-  if ((tid & 31) == 0) {
-    red[warp] = worst;
-    add_bytes(D.ctr, CTR_HD_EXACT, ex);
+  for (int o = 16; o > 0; o >>= 1) nExact += __shfl_xor_sync(FULLMASK, nExact, o);
+  if (lane == 0 && nScreen != 0) {
+    add_bytes(D.ctr, CTR_HD_EXACT, nExact);
+    add_bytes(D.ctr, CTR_HD_SCREENED, nScreen);
   }
-  __syncthreads();
-  if (tid == 0) {
-    float w = red[0];
-    for (uint32_t i = 1; i < HDS_M / 32; i++) w = fmaxf(w, red[i]);
-    if (ok) atomicMax(D.ctr + CTR_HD + pair, __float_as_uint(w));
-    const uint32_t nsTile = min(HDS_M, ns - s0);
-    add_bytes(D.ctr, CTR_HD_SCREENED, (unsigned long long)nsTile * nt);
-  }
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(HDS_N));
 }
 
-void launch_hd(const HdArgs& A, const Dev& D, cudaStream_t s) {
+void launch_hd(const HdArgs& A, const Dev& D, int nSM, cudaStream_t s) {
   if (A.nPairs == 0) return;
-  k_hd_sample<32><<<(A.nMeshes + 7) / 8, 256, 0, s>>>(A, D);
-  k_hd_prep<<<A.nMeshes, 256, 0, s>>>(A, D);
-  dim3 grid((A.maxSide + HD_TILE - 1) / HD_TILE, A.nPairs, 2);
-  k_hd_dist<<<grid, HD_TILE, 0, s>>>(A, D);
-  dim3 gs((A.maxSide + HDS_M - 1) / HDS_M, A.nPairs, 2);
-  k_hd_screen<<<gs, HDS_M, 0, s>>>(A, D);
+  k_hd_prep<<<A.nMeshes, HD_PREP, 0, s>>>(A, D);
+  k_hd_tiles<<<1, 1024, 0, s>>>(A, D);
+  k_hd_near<<<nSM * 8, HD_NEAR, 0, s>>>(A, D);
 }
 
 }  // namespace cuacd

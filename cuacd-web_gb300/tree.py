@@ -176,8 +176,9 @@ class GpuTree:
     KERNELS = ("reset", "plan", "scan", "emit", "hull", "record", "evaluate")
 
     def hd_stats(self) -> dict:
-        """The last Hausdorff batch's tensor-core screen: exact distances,
-        screened pairs and whether a tensor-core wait timed out."""
+        """The last Hausdorff batch's cluster search: exact distances and
+        sample-triangle pairs of the clusters visited (timeout is False: the
+        search waits on nothing)."""
         b = (C.c_uint64 * 3)()
         _check(load_library().cuacd_tree_hd_stats(self.h, b))
         return dict(exact=int(b[0]), screened=int(b[1]), timeout=bool(b[2]))

@@ -70,9 +70,9 @@ typedef struct {
                                warp each, larger ones on a 256-thread block
                                (0: 1024); the results do not depend on it */
   int32_t hdScreenMinTris;  /* Hausdorff target meshes with at least this many
-                               triangles go through the tensor-core screen
-                               (0: 256, < 0: never); the results do not
-                               depend on it */
+                               triangles are searched by clusters (0: 64,
+                               < 0: never, every triangle is evaluated); the
+                               results do not depend on it */
   int32_t autotune;         /* 1 (the default): when warpMaxNv is 0, the
                                warp/block thresholds of the hull and of
                                plan/emit are chosen per distribution of part
@@ -193,10 +193,10 @@ int cuacd_tree_kernel_ms(void* tree, float* ms7);
  * children once, and each child's points are read once by its hull. */
 int cuacd_tree_kernel_bytes(void* tree, uint64_t* bytes3);
 
-/* Hausdorff tensor-core screen of the last Hausdorff batch on this handle
- * (no reference counterpart): [0] exact point-triangle distances computed,
- * [1] sample-triangle pairs screened, [2] 1 when a tensor-core wait timed out
- * (the batch's distances are then incomplete). */
+/* Hausdorff cluster search of the last Hausdorff batch on this handle (no
+ * reference counterpart): [0] exact point-triangle distances computed, [1]
+ * sample-triangle pairs of the clusters visited, [2] 0 (the search waits on
+ * nothing that could time out). */
 int cuacd_tree_hd_stats(void* tree, uint64_t* out3);
 
 /* GpuTree.lastHullGpuMs (tree.ts:380): device time of the last completed
