@@ -104,7 +104,9 @@ struct HdArgs {
   uint32_t* cnt;             // per triangle: its area, then its samples
   uint32_t* soff;            // per triangle: its cell, then (sorted) its first sample
   uint32_t* perm;            // sorted triangles' indices
-  float4* triC;              // sorted triangles: centroid, radius
+  uint32_t* bad;             // per mesh: its slivers, as sorted triangles' numbers
+  uint32_t* nBad;            // per mesh: how many
+  float4* triC;              // sorted triangles: centroid, radius (negative: a sliver)
   float4* triG;              // sorted triangles: three corners
   float4* box;               // per cluster of 32 sorted triangles: low and high corner
   uint32_t* tilePre;         // prefix of the meshes' 32-sample tiles (nMeshes + 1)

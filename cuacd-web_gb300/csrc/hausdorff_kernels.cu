@@ -129,6 +129,7 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
   __shared__ uint32_t ws[32];
   __shared__ float box[6][HD_PREP / 32];
   __shared__ float sTotal;
+  __shared__ uint32_t sBad;
   const uint32_t m = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const PartDesc pd = D.parts[A.partBase + m];
   const uint32_t nt = pd.nt, cap = A.capN[m];
@@ -251,6 +252,8 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
   // the sorted triangles, the clusters' boxes and the samples' prefix
   const size_t base = A.triOff[m];
   run = 0;
+  if (tid == 0) sBad = 0;
+  __syncthreads();
   for (uint32_t c0 = 0; c0 < nt; c0 += 4 * HD_PREP) {
     const uint32_t i0 = c0 + 128 * warp + lane;
     uint32_t N[4], off[4], wsum = 0;
@@ -277,6 +280,15 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
           r = INFINITY;
           blo = mk3(-INFINITY, -INFINITY, -INFINITY);
           bhi = mk3(INFINITY, INFINITY, INFINITY);
+        }
+        // a sliver (the angle at a below 0.57 degrees) or a degenerate
+        // triangle: tri_sq may be far off its geometry (HdNear), so it is
+        // marked by a negative radius and listed
+        const f3 ab = b - a, ac = c - a, nn = cross(ab, ac);
+        const float n2 = dot(nn, nn);
+        if (!(n2 > 1e-4f * dot(ab, ab) * dot(ac, ac)) || n2 < 1.1e-20f) {
+          r = -r;
+          A.bad[base + atomicAdd(&sBad, 1u)] = i;
         }
         float4* G = A.triG + 3 * (base + i);
         G[0] = make_float4(a.x, a.y, a.z, 0.0f);
@@ -310,6 +322,7 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
       if (i0 + 32 * u < nt) soff[i0 + 32 * u] = run + before + off[u];
     run += tot;
   }
+  if (tid == 0) A.nBad[m] = sBad;  // behind the last scan's barriers
 }
 
 // tiles of 32 samples per mesh: their prefix over the meshes, and the work
@@ -347,24 +360,33 @@ __global__ void __launch_bounds__(1024) k_hd_tiles(const HdArgs A, const Dev D) 
 
 #define HD_NEAR 128u
 
-// A sample's state in the culled search. best is the smallest tri_sq so far
-// and ub the smallest squared centroid distance (a centroid is a point of
-// its triangle). The search keeps a triangle unless its bound |p - c| - r, or
-// its cluster's box, is farther than reach(): the smaller of the two with
-// a 1e-3 relative margin, and an absolute one of 3e-10 |p|^2 for distances
-// that cancel far from the origin (coordinates round to 2^-24 of |p|, so
-// squared distances below (1e-3 |p|)^2 may be off by 1e-3 of themselves).
-// Those cover the float32 error of tri_sq, of the centroid and of the
-// radius, so the triangle attaining the smallest tri_sq is always looked at.
+// A sample's state in the culled search. best is the smallest tri_sq so far;
+// ub bounds the tri_sq of some triangle from above by its centroid's distance
+// (a centroid is a point of its triangle). The search keeps a triangle unless
+// its bound |p - c| - r, or its cluster's box, is farther than reach(): the
+// smaller of the two with a 1e-3 relative margin, and an absolute one of
+// 3e-10 |p|^2 for distances that cancel far from the origin (coordinates
+// round to 2^-24 of |p|, so squared distances below (1e-3 |p|)^2 may be off by
+// 1e-3 of themselves).
+//
+// Both bounds hold for tri_sq as it is computed when the angle at a, which its
+// barycentrics and its normal are formed from, has a sine s >= 0.01: the
+// normal's direction is within about 2^-23 / s, so a plane distance is off
+// by at most 1e-5 |p - a|, which ub's margin of 2 % and 1e-7 r^2 covers (|p -
+// a| <= |p - c| + r); and the barycentrics are off by at most 2^-24 |p - a| /
+// s^2 in length, so a point taken for one above the triangle lies within 6e-4
+// |p - a| of it, 4e-7 of the squared distance. For a sliver the normal can
+// be noise and the plane distance anything, and a triangle with |n|^2 < 1e-20
+// counts by its corners alone: such triangles give no ub, and a sample that
+// could still raise the pair's largest distance is at last tested against
+// every one of them, near or far. So the distance is the exhaustive
+// search's, whichever order the tiles run in.
 struct HdNear {
   f3 p;
   float p2, best, ub;
   __device__ __forceinline__ float reach() const { return fminf(best, ub) * 1.001f + 3e-10f * p2 + 1e-30f; }
-  // whether the sample can still raise the pair's largest distance: its
-  // smallest tri_sq is at most best, and at most ub with a wider margin
-  __device__ __forceinline__ bool counts(float gmax) const {
-    return best > gmax && !(ub * 1.01f + 3e-9f * p2 < gmax);
-  }
+  // whether the sample can still raise the pair's largest distance
+  __device__ __forceinline__ bool counts(float gmax) const { return best > gmax && !(ub + 3e-9f * p2 < gmax); }
 };
 
 __device__ __forceinline__ float warp_box_min(float v) { return f_unord(__reduce_min_sync(FULLMASK, f_ord(v))); }
@@ -460,9 +482,9 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
         const float4 g = cent[j];
         const f3 d = S.p - mk3(g.x, g.y, g.z);
         const float d2 = dot(d, d);
-        if (d2 < dmin) { dmin = d2; jmin = j; }
+        if (d2 < dmin && g.w >= 0.0f) { dmin = d2; jmin = j; }
       }
-      S.ub = fminf(S.ub, dmin);
+      if (dmin < 3.4e38f) S.ub = fminf(S.ub, dmin * 1.02f + 1e-7f * cent[jmin].w * cent[jmin].w);
       active = active && S.counts(gmax);
       const unsigned any = __ballot_sync(FULLMASK, active);
       nScreen += (unsigned long long)__popc(any) * cn;  // the same on every lane
@@ -483,7 +505,7 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
       for (uint32_t j = 0; j < cn; j++) {
         const float4 g = cent[j];
         const f3 d = S.p - mk3(g.x, g.y, g.z);
-        const float q = rs + g.w;
+        const float q = rs + fabsf(g.w);
         if (!(dot(d, d) > q * q * 1.00001f)) keep |= 1u << j;
       }
       if (dmin < 3.4e38f) keep &= ~(1u << jmin);
@@ -493,7 +515,7 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
         keep &= keep - 1;
         const float4 g = cent[j];
         const f3 d = S.p - mk3(g.x, g.y, g.z);
-        const float q = rs + g.w;
+        const float q = rs + fabsf(g.w);
         if (dot(d, d) > q * q * 1.00001f) continue;
         exact(j);
         if (!S.counts(gmax)) {
@@ -560,6 +582,20 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
           need = need && !(gap > reach);
         }
         todo = __ballot_sync(FULLMASK, need);
+      }
+    }
+    // what is left against the target's slivers
+    if (act) {
+      const uint32_t nBad = A.nBad[dst];
+      if (nBad != 0) active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
+      for (uint32_t k = 0; k < nBad; k++) {
+        if ((k & 31u) == 0 && __ballot_sync(FULLMASK, active) == 0) break;
+        const float4* g = G + 3 * (size_t)A.bad[tb + k];
+        const float4 a = g[0], b = g[1], c = g[2];
+        if (active) {
+          S.best = fminf(S.best, tri_sq(S.p, xyz(a), xyz(b), xyz(c)));
+          nExact++;
+        }
       }
     }
     const uint32_t worst = __reduce_max_sync(FULLMASK, active ? __float_as_uint(S.best) : 0u);

@@ -53,3 +53,26 @@ def test_cluster_search_long_and_mixed_batch(trees):
     for i, (x, y) in enumerate(pairs):
         if x.nt == 0 or y.nt == 0:
             assert a[i] == 0.0
+
+
+@pytest.mark.parametrize("seed", [0, 1, 2])
+def test_cluster_search_slivers(trees, seed):
+    """Parts cut again and again hold slivers, whose tri_sq can be far off
+    their geometry: the distances are still the exhaustive search's, and the
+    same on every run, whichever tiles finish first."""
+    cut = pkg("decompose").plane_cut
+    rng = np.random.default_rng(seed)
+    parts = [G.noisy_icosphere(3, seed=seed), M.normalize(G.blob_mesh(6, 22 + seed, seed=seed))[0]]
+    for _ in range(4):
+        halves = []
+        for m in parts:
+            n = np.eye(3)[rng.integers(3)] if rng.random() < 0.5 else rng.normal(size=3)
+            n /= np.linalg.norm(n)
+            p = m.verts.astype(np.float64) @ n
+            try:
+                halves += cut(m, [*n, -(p.min() + rng.uniform(0.3, 0.7) * np.ptp(p))])
+            except RuntimeError:
+                halves.append(m)
+        parts = [h for h in halves if h.nt >= 4]
+    runs = [[h["hausdorff"] if h else None for h in t.hulls_with_hausdorff(parts)] for t in (trees[2], trees[2], trees[1])]
+    assert runs[0] == runs[1] == runs[2]
