@@ -68,9 +68,19 @@ struct Dev {
   uint32_t* ctr;
   unsigned long long* scanTmp;  // scan bases and per-block sums (3 + 3 * blocks)
   uint32_t* work;               // hull work counters, one per hull launch of a run
+  uint32_t* list;               // parts for the blocks, listed by the level's warp hulls
   float* ub;                    // per seed: the last level's pruning upper bound
   uint64_t vCap, tCap, eCap, sCap;
 };
+
+// Points from which parts beyond the register hull go to the blocks: in a
+// batch of hulls (pair unions, halves: convex position), where blocks win from
+// the smallest part on (152 parts of 60 points 0.34 against 0.37 ms), and in a
+// tree's levels, whose smaller children barely outgrow the register form (8
+// staircases: 1.6 ms of hulls from 129 points on, 1.7 ms from 33 on; 16 blobs
+// of 500-2,000 triangles 12.2 and 11.0 ms: the other one is a trial schedule).
+#define HAND_ON_BATCH 33u
+#define HAND_ON_TREE 129u
 
 // Launch parameters of one tree level (the reference's Params, shaders.ts:30-39)
 struct Level {
@@ -86,9 +96,10 @@ struct Level {
   uint32_t exportBase, exportStride;  // hull face export into T (u32 offsets)
   uint32_t lastLevel, hullStage, nSeeds;
   uint32_t hdDescBase;      // != 0: write a Hausdorff descriptor at part + hdDescBase
-  uint32_t workSlot;        // hull work counters of this launch: D.work[slot] (warp
-                            // groups) and D.work[16 + slot] (256-thread groups)
-  uint32_t maxNvHint;       // largest part the host knows of, or 0: read D.work[32 + workSlot]
+  uint32_t workSlot;        // hull work counters of this launch: D.work[slot] (warp groups),
+                            // D.work[16 + slot] (block groups), D.work[48 + slot] (parts in D.list)
+  uint32_t handOn;          // warps hand parts of at least this many points, beyond the
+                            // register hull, on to the blocks (0: none)
 };
 
 // Hausdorff batch: mesh m's descriptor at parts[partBase + m]; pair k is
@@ -115,9 +126,10 @@ struct HdArgs {
 
 // Physical words of one hull slab whose reference size (which fixes the face
 // limit fmax) is W words. After the W words a part of nv points needs the
-// visible list and walk queue (2 * 2048), adjacency (4 fmax), two bitmap
-// arrays (2 ceil(fmax / 32)) and two horizon maps (2 nv). With fmax <= (W -
-// 3 nv) / 16 and nv <= (W - 1024) / 3 that is below 3672 + 0.671 W.
+// visible list and walk queue (2 * 2048), adjacency (4 fmax), the faces' keys
+// and segments (4 fmax), two bitmap arrays (2 ceil(fmax / 32)) and two
+// horizon maps (2 nv). With fmax <= (W - 3 nv) / 16 the 8 fmax + 2 nv words
+// are at most W / 2 + nv / 2, and with nv <= (W - 1024) / 3 below 2 W / 3.
 __host__ __device__ constexpr uint32_t hull_slab_stride(uint32_t W) {
   return (W + 4096u + (uint32_t)(((uint64_t)W * 2) / 3) + W / 128 + 64u + 63u) & ~63u;
 }
@@ -175,6 +187,12 @@ __device__ __forceinline__ float warp_max_f(float v) {
   for (int o = 16; o > 0; o >>= 1) v = fmaxf(v, __shfl_xor_sync(FULLMASK, v, o));
   return v;
 }
+// floats as signed integers in the same order
+__device__ __forceinline__ int f_ord(float x) {
+  const int b = __float_as_int(x);
+  return b ^ ((b >> 31) & 0x7fffffff);
+}
+__device__ __forceinline__ float f_unord(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
 // inclusive scan within a warp
 __device__ __forceinline__ uint32_t warp_incl_u(uint32_t v, int lane) {
 #pragma unroll

@@ -68,14 +68,19 @@ static const uint32_t HD_SCREEN_MIN = 64;
 static const uint32_t BIG_JOB_NV = 2048;
 
 // Schedules the autotuner chooses between: the largest part a warp hulls
-// (larger ones go to blocks) and the largest parent a warp plans and emits.
+// (larger ones go to blocks), the largest parent a warp plans and emits, and
+// the points from which warps hand parts beyond the register hull on to the
+// blocks, in a tree's levels and in hull batches.
 // The kernels' outputs do not depend on which group shape handles a part,
 // so every schedule gives the same results; they differ in speed with the
 // distribution of part sizes. The first is the fixed default.
 struct Schedule {
-  uint32_t smallNv, bigJobNv;
+  uint32_t smallNv, bigJobNv, handTree, handBatch;
 };
-static const Schedule kSchedules[] = {{SMALL_NV, BIG_JOB_NV}, {512, BIG_JOB_NV}, {256, BIG_JOB_NV}, {SMALL_NV, 4096}};
+static const Schedule kSchedules[] = {{SMALL_NV, BIG_JOB_NV, HAND_ON_TREE, HAND_ON_BATCH},
+                                      {512, BIG_JOB_NV, HAND_ON_BATCH, HAND_ON_TREE},
+                                      {256, BIG_JOB_NV, 0, 0},
+                                      {SMALL_NV, 4096, 0, 0}};
 static const int kNumSchedules = (int)(sizeof(kSchedules) / sizeof(kSchedules[0]));
 // per key: device time of one run or batch under each schedule tried so far
 struct TuneEntry {
@@ -176,7 +181,7 @@ struct Tree {
     pcls.push_back(cls);
   }
   Dev D{};
-  DevBuf bV, bT, bE, bS, bCtr, bSlab, bParts, bItems, bJobs, bPlanes, bSnap, bHd, bScan, bWork, bUb;
+  DevBuf bV, bT, bE, bS, bCtr, bSlab, bParts, bItems, bJobs, bPlanes, bSnap, bHd, bScan, bWork, bUb, bList;
   uint32_t workSlots = 0;  // hull launches of the prepared run
   HostBuf hStage, hRead, hSnap, hMeta;
   uint32_t capSeeds = 0, capJobs = 0, capItems = 0, capParts = 0, capPlanes = 0;
@@ -243,7 +248,7 @@ struct Tree {
     if (cutter) cut::engine_destroy(cutter);
     if (concave) conc::engine_destroy(concave);
     if (gexec) cudaGraphExecDestroy(gexec);
-    for (DevBuf* b : {&bV, &bT, &bE, &bS, &bCtr, &bSlab, &bParts, &bItems, &bJobs, &bPlanes, &bSnap, &bHd, &bScan, &bWork, &bUb}) b->release();
+    for (DevBuf* b : {&bV, &bT, &bE, &bS, &bCtr, &bSlab, &bParts, &bItems, &bJobs, &bPlanes, &bSnap, &bHd, &bScan, &bWork, &bUb, &bList}) b->release();
     for (HostBuf* b : {&hStage, &hRead, &hSnap, &hMeta}) b->release();
     for (cudaEvent_t e : pev) cudaEventDestroy(e);
     if (ev0) cudaEventDestroy(ev0);
@@ -255,6 +260,7 @@ struct Tree {
     D.slab = (uint32_t*)bSlab.p; D.parts = (PartDesc*)bParts.p; D.items = (ItemDesc*)bItems.p;
     D.jobs = (Job*)bJobs.p; D.planes = (float4*)bPlanes.p; D.ctr = (uint32_t*)bCtr.p;
     D.scanTmp = (unsigned long long*)bScan.p; D.work = (uint32_t*)bWork.p; D.ub = (float*)bUb.p;
+    D.list = (uint32_t*)bList.p;
     D.vCap = cfg.vertexCap; D.tCap = cfg.triCap; D.eCap = cfg.edgeCap; D.sCap = cfg.scratchWords;
   }
   // tree.ts:191-213
@@ -272,6 +278,7 @@ struct Tree {
     if (nItems > 0xffffffffull / 2 || nParts > 0xffffffffull / 2) return fail(CUACD_E_CAPACITY, "tree tables exceed 32-bit indexing");
     int rc;
     if ((rc = bParts.ensure(nParts * sizeof(PartDesc)))) return rc;
+    if ((rc = bList.ensure(nParts * 4))) return rc;
     if ((rc = bItems.ensure(nItems * sizeof(ItemDesc)))) return rc;
     if ((rc = bJobs.ensure(std::max<uint64_t>(totalJobs, 1) * sizeof(Job)))) return rc;
     if ((rc = bPlanes.ensure(std::max<uint64_t>(nPlanes, 1) * 16))) return rc;
@@ -285,6 +292,7 @@ struct Tree {
   int ensurePartSlots(uint32_t n) {
     if (n <= capParts) return 0;
     int rc = bParts.ensure((size_t)n * sizeof(PartDesc));
+    if (rc == 0) rc = bList.ensure((size_t)n * 4);
     if (rc) return rc;
     capParts = n;
     gvalid = false;
@@ -308,7 +316,7 @@ struct Tree {
     }
     return 0;
   }
-  Level baseLevel() const {
+  Level baseLevel(bool batch) const {
     Level P;
     std::memset(&P, 0, sizeof(P));
     P.edgeStride = edgeStride;
@@ -316,11 +324,12 @@ struct Tree {
     P.hullSlabWords = slabWords;
     P.slabStride = slabStride;
     P.smallNv = smallNv();
+    if (cfg.warpMaxNv <= 0) P.handOn = batch ? kSchedules[sched].handBatch : kSchedules[sched].handTree;
     return P;
   }
   // hull launches of one level, warp groups then block groups; work
-  // counters `slot` and 16 + slot must be zero beforehand. Parts above
-  // warpMaxNv points take the widest blocks (1024, then 512 threads) whose
+  // counters `slot`, 16 + slot and 48 + slot must be zero beforehand. The
+  // parts that the warps list take the widest blocks (1024, then 512 threads) whose
   // resident slots hold all the level's parts in one wave (the more threads
   // per part, the shorter each insertion round), else 256-thread blocks
   // (the most parts at once).
@@ -528,12 +537,12 @@ struct Tree {
     cudaMemcpyAsync(D.planes + stateBase, snap + snapState, (16 + 4 * (size_t)nSeeds) * 16, cudaMemcpyDeviceToDevice, stream);
     mark(0);
     auto stage = [&](const std::vector<LevelLayout>& L, uint32_t mode, uint32_t headerOff) {
-      // one hull work counter per level of the stage
-      // (work[l]: the level's hull counter; work[32 + l]: its largest child)
+      // the levels' hull work counters (work[l], work[16 + l]) and lists' lengths
+      // (work[48 + l])
       cudaMemsetAsync(D.work, 0, 64 * 4, stream);
       for (uint32_t l = 0; l < L.size(); l++) {
         const LevelLayout& v = L[l];
-        Level P = baseLevel();
+        Level P = baseLevel(false);
         P.itemsInBase = v.itemsInBase; P.nItemsIn = v.nItemsIn; P.itemsOutBase = v.itemsOutBase; P.jobBase = v.jobBase;
         P.width = v.width; P.nEdgeCuts = v.nEdgeCuts; P.totalWidth = v.totalWidth;
         P.level = l; P.totalLevels = depth; P.partBase = v.partBase;
@@ -576,6 +585,8 @@ struct Tree {
     for (auto& L : tree) { s.push_back(L.nJobs); s.push_back(L.totalWidth); s.push_back(L.width); }
     for (uint32_t l = 0; l < depth; l++) s.push_back((maxSeedNv >> l) > bigJobNv());
     s.push_back(smallNv());
+    s.push_back(baseLevel(false).handOn);
+    s.push_back((uint64_t)bList.p);
     return s;
   }
   int launch() {
@@ -706,12 +717,11 @@ struct Tree {
     CK(cudaMemcpyAsync(D.parts, parts.data(), (size_t)n * sizeof(PartDesc), cudaMemcpyHostToDevice, stream));
     if (withHd) CK(cudaMemsetAsync(D.parts + n, 0, (size_t)n * sizeof(PartDesc), stream));
     CK(cudaMemsetAsync(D.ctr, 0, CTR_WORDS * 4, stream));
-    Level P = baseLevel();
+    Level P = baseLevel(true);
     P.nItemsIn = n; P.itemsOutBase = n; P.totalLevels = 1;
     P.edgePlaneBase = capJobs; P.nChildParts = n; P.nJobs = 0;
     P.exportBase = tTop; P.exportStride = stride; P.hullStage = (uint32_t)hullStage;
     P.hdDescBase = withHd ? (uint32_t)n : 0;
-    P.maxNvHint = std::max(maxNv, 1u);
     CK(cudaMemsetAsync(D.work, 0, 64 * 4, stream));
     CK(cudaEventRecord(ev0, stream));
     hullLaunch(P, 0);
@@ -1022,7 +1032,7 @@ int cuacd_tree_memory(const void* tree, uint64_t* deviceBytes, uint64_t* caps4) 
   if (!t) return fail(CUACD_E_INVALID, "cuacd_tree_memory: null tree");
   uint64_t n = cut::engine_device_bytes(t->cutter) + conc::engine_device_bytes(t->concave);
   for (const DevBuf* b : {&t->bV, &t->bT, &t->bE, &t->bS, &t->bCtr, &t->bSlab, &t->bParts, &t->bItems, &t->bJobs,
-                          &t->bPlanes, &t->bSnap, &t->bHd, &t->bScan, &t->bWork, &t->bUb})
+                          &t->bPlanes, &t->bSnap, &t->bHd, &t->bScan, &t->bWork, &t->bUb, &t->bList})
     n += b->bytes;
   if (deviceBytes) *deviceBytes = n;
   if (caps4) {

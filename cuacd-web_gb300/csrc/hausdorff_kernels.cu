@@ -84,13 +84,6 @@ static_assert(HD_CHUNK % 32 == 0 && 2 * HD_CHUNK <= HD_CELLS, "two area chunks s
 __device__ __forceinline__ uint32_t spread4(uint32_t v) {
   return (v & 1u) | ((v & 2u) << 2) | ((v & 4u) << 4) | ((v & 8u) << 6);
 }
-// floats as signed integers in the same order
-__device__ __forceinline__ int f_ord(float x) {
-  const int b = __float_as_int(x);
-  return b ^ ((b >> 31) & 0x7fffffff);
-}
-__device__ __forceinline__ float f_unord(int k) { return __int_as_float(k ^ ((k >> 31) & 0x7fffffff)); }
-
 __device__ __forceinline__ f3 centroid(f3 a, f3 b, f3 c) {
   return mk3((a.x + b.x + c.x) / 3.0f, (a.y + b.y + c.y) / 3.0f, (a.z + b.z + c.z) / 3.0f);
 }

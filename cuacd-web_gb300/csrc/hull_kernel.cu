@@ -28,7 +28,7 @@ namespace cuacd {
 
 #define HULL_VIS_MAX 2048u
 #define ALIVE 0x80000000u
-// points a warp group keeps in shared memory (3 floats each)
+// points a warp group keeps in shared memory (16 bytes each)
 #define QC_MAX 256u
 
 // k-DOP seed axes (shaders.ts:769-810): the same table, so the seeds are the
@@ -111,14 +111,17 @@ struct HullCtx {
   uint32_t* vis;   // visible face slots in slot order (HULL_VIS_MAX)
   uint32_t* q;     // walk queue (HULL_VIS_MAX)
   uint32_t* nbr;   // 4 words per face slot: the faces across its 3 edges
+  unsigned long long* fkey;  // block path, per face slot: its candidates' largest key, 0 without any
+  uint2* fseg;               // block path, per face slot: its candidates in the pool (first, count)
   uint32_t* bm;    // one bit per face slot
   uint32_t* wp;    // compaction: alive faces before each bitmap word
   uint32_t* hA;    // per point: new face whose horizon edge starts there
   uint32_t* hB;    // per point: new face whose horizon edge ends there
-  const float* qc;  // quantised points in shared memory, or null
+  const float4* qc;  // quantised points, one 16-byte load each (a warp's in shared
+                     // memory, a block's in its slab), or null
 
   __device__ __forceinline__ f3 qvert(uint32_t i) const {
-    if (qc) return mk3(qc[3 * i], qc[3 * i + 1], qc[3 * i + 2]);
+    if (qc) return xyz(qc[i]);
     f3 v = ldv(V, (size_t)vOff + 3 * (size_t)i) - qlo;
     return mk3(rintf(v.x * qs), rintf(v.y * qs), rintf(v.z * qs));
   }
@@ -142,7 +145,10 @@ struct HullCtx {
   // face_make with the grid point of corner c given
   __device__ __forceinline__ void face_make_q(uint32_t a, uint32_t b, uint32_t c, f3 pc, uint4& w0, uint4& w1,
                                               uint4& w2, uint4& w3) const {
-    f3 pa = qvert(a), pb = qvert(b);
+    face_make_abc(a, b, c, qvert(a), qvert(b), pc, w0, w1, w2, w3);
+  }
+  __device__ __forceinline__ void face_make_abc(uint32_t a, uint32_t b, uint32_t c, f3 pa, f3 pb, f3 pc, uint4& w0,
+                                                uint4& w1, uint4& w2, uint4& w3) const {
     f3 e1 = pb - pa, e2 = pc - pa;
     f3 n = cross(e1, e2);
     const float kb = 1e-6f * (l1(e1) * l1(e2));
@@ -179,6 +185,17 @@ struct HullCtx {
     if (det > bound) return det / __uint_as_float(w1.w);
     if (det < -bound) return -1.0f;
     return ((w0.x & 0x7fffffffu) == pi || w0.y == pi || w0.z == pi) ? -1.0f : 0.0f;
+  }
+  // the same decision without the ranking value's division: 1 visible, -1
+  // not, 0 when the sign needs the exact determinant
+  __device__ __forceinline__ int face_side(uint4 w0, uint4 w1, uint4 w2, f3 p, uint32_t pi) const {
+    const f3 n = mk3(__uint_as_float(w1.x), __uint_as_float(w1.y), __uint_as_float(w1.z));
+    const f3 d = p - mk3(__uint_as_float(w2.x), __uint_as_float(w2.y), __uint_as_float(w2.z));
+    const float det = dot(n, d);
+    const float bound = __uint_as_float(w0.w) * l1(d);
+    if (det > bound) return 1;
+    if (det < -bound) return -1;
+    return ((w0.x & 0x7fffffffu) == pi || w0.y == pi || w0.z == pi) ? -1 : 0;
   }
   // exact visibility of p from the face (shaders.ts:868-876): the sign of
   // N . (p - a) with the stored integer normal. With N = 2^32 h + l (l the
@@ -831,11 +848,15 @@ __device__ __noinline__ uint32_t hull_grow(const HullCtx& h, HullSm& hs, GrpSmem
 //     patch and the horizon loop is matched in shared memory. A patch of more
 //     than BIG_VIS faces falls back to hull_insert (nothing global has been
 //     written by then).
-//   * the candidates are kept per candidate slot k (point cand[k], owner
-//     and distance in the owner and dist words at k), so one coalesced pass
-//     after each insertion drops the inserted point, reassigns the points of
-//     dead faces and finds the next pick (largest distance, lowest point
-//     index); dead slots are squeezed out when they reach a quarter.
+//   * the candidates are kept per face: a face's candidate points are one
+//     segment of a pool, with the largest key (distance, then lowest point
+//     index) beside it. An insertion reads the segments of the faces it
+//     kills and appends the segments of its new faces, so its cost follows
+//     the points that change owner, and the next pick is found among the
+//     faces' keys. (One pass over every candidate's owner per round was half
+//     of a round's time.) The pool is the 2 nv words of the owner and
+//     distance arrays; when the bump pointer would pass its end the live
+//     segments are gathered to its front.
 #ifndef BIG_VIS
 #define BIG_VIS 128u
 #endif
@@ -850,61 +871,54 @@ struct BigSm {
   uint32_t hzA[3 * BIG_VIS];  // new face j: start and end of its horizon edge
   uint32_t hzB[3 * BIG_VIS];
   uint4 nrec[BIG_NREC][4];    // records of the first new faces, for the reassignment
-  uint32_t fast, ntodo;
+  uint32_t fast;
 };
 
-// Batched rounds. A round takes the next picks in key order c_0, c_1, ...,
-// walks their visible patches on the current hull in parallel (one warp
-// each) and inserts the longest prefix whose insertions, one after
-// another, give the hull the single-pick loop gives:
+// Batched rounds. A round takes picks c_0, c_1, ..., the candidates of the
+// faces with the largest keys in key order (c_j the farthest candidate not
+// owned by an earlier pick's owner face), walks their visible patches on the
+// current hull in parallel (one warp each) and inserts the longest prefix
+// whose insertions, one after another, give the hull the single-pick loop
+// gives:
 //   * the patches are disjoint and no face of a later patch borders a face
 //     of an earlier one. A new face of c_i borders only c_i's other new
 //     faces and the faces across c_i's horizon, so c_j's visible faces,
 //     horizon and new faces are the ones found on the current hull, and
 //     c_j's orphans (the points its patch owns) are the current ones;
-//   * c_j still holds the largest key once c_0 .. c_(j-1) are in: the
-//     orphans of each earlier patch get their new keys over that patch's
-//     new faces, and all of them are below c_j's key;
+//   * c_j holds the largest key once c_0 .. c_(j-1) are in: the orphans of
+//     each earlier patch get their new keys over that patch's new faces, and
+//     all of them are below c_j's key; every other candidate is owned by a
+//     face outside the earlier patches, so none of the earlier picks' owner
+//     faces, and was considered for c_j;
 //   * neither the compaction rule nor the slot limit fires at any of the
 //     steps (a round whose first step would compact runs the single-pick
 //     step).
 // c_j's new faces take the slots the single-pick loop gives them, right
 // after c_(j-1)'s, so face slots, owners and insertion order are the
 // single-pick loop's.
-// picks per round: one per warp of the block (NW warps)
 #define BAT_FACES 32u   // faces of a batched patch, one per lane
-#define BAT_NEW 36u     // its horizon edges (a connected patch of n faces has at most n + 2)
+#define BAT_NEW 32u     // its new faces, one per lane
 #define BAT_HASH_BITS 6u
-// the faces of every whole walked patch: at most NW * BAT_FACES, so the set
-// is never more than half full
 #ifndef KMAX_CAP
 #define KMAX_CAP 16u
 #endif
 template <int NW>
 struct BatDims {
-  static constexpr uint32_t BLK_BITS = NW <= 8 ? 9u : (NW <= 16 ? 10u : 11u);
-  static constexpr uint32_t NRC = NW <= 8 ? 16u : 8u;  // new-face records per step kept in shared memory
-  // picks per round: one per warp, at most KMAX_CAP (the merge of the
-  // warps' lists is serial in the picks, and later picks rarely pass the
-  // checks: on 15-28k-point blob hulls 12 and 16 measured the same, 20
-  // 1-2 % slower, 28 4-6 % slower)
+  // picks per round: one per warp, at most KMAX_CAP
   static constexpr uint32_t KMAX = NW < KMAX_CAP ? (uint32_t)NW : KMAX_CAP;
+  // the faces of every whole walked patch: at most KMAX * BAT_FACES, so the
+  // set is never more than half full
+  static constexpr uint32_t BLK_BITS = KMAX <= 8 ? 9u : (KMAX <= 16 ? 10u : 11u);
 };
-#define BAT_LIST 8u  // keys per warp list
-// candidate slots per thread in flight in the batched round's slot pass
-#ifndef SCAN_U
-#define SCAN_U 4
-#endif
-// dead candidate slots are squeezed out above 1 / SQZ_DIV of the list
-#ifndef SQZ_DIV
-#define SQZ_DIV 8u
-#endif
-// orphans listed per round (six words each in the visible list's and walk
-// queue's words); a round with more inserts its first step alone
-#ifndef TODO_CAP
-#define TODO_CAP (HULL_VIS_MAX / 3)
-#endif
+#define BAT_LIST 4u  // keys per warp list
+#define BAT_CAND 64u  // faces above the threshold
 struct BatWalk {
+  uint4 rec[BAT_NEW][4];              // its new faces' records
+  unsigned long long fk[BAT_NEW];     // the new faces' largest candidate keys
+  unsigned long long maxOrph;         // the largest of them
+  uint2 seg[BAT_FACES];               // the patch faces' candidates in the pool
+  uint32_t segPre[BAT_FACES];         // orphans of the patch before each face's
+  uint32_t cnt[BAT_NEW], pre[BAT_NEW];  // orphans a new face takes, and the ones before it
   uint32_t key[1u << BAT_HASH_BITS];  // patch face + 1; 0 = empty
   uint32_t f[BAT_FACES];              // patch faces in walk order
   uint32_t nb[BAT_FACES][3];          // faces across their edges
@@ -912,31 +926,31 @@ struct BatWalk {
   uint32_t ord[BAT_FACES];            // walk index of the k-th face in slot order
   uint32_t hA[BAT_NEW], hB[BAT_NEW];  // new face q: its horizon edge (a, b)
   uint32_t tw[BAT_NEW], df[BAT_NEW];  // the face across that edge and the patch face inside it
-  uint32_t n, nnew, ok, pick;
+  uint32_t n, nnew, ok, norph, tot;   // faces, new faces, whole patch, orphans, those with a new owner
+  uint32_t pick, cf, pad;             // cf: the patch meets an earlier one
 };
 template <int NW>
 struct BatSm {
-  static constexpr uint32_t BLK_BITS = BatDims<NW>::BLK_BITS, NRC = BatDims<NW>::NRC;
+  static constexpr uint32_t BLK_BITS = BatDims<NW>::BLK_BITS, K = BatDims<NW>::KMAX;
   union {
     BigSm big;  // the single-pick step
-    BatWalk w[NW];
+    BatWalk w[K];
   } u;
-  // per warp: its largest candidate keys in descending order with their
-  // slots and owners, their count, whether keys below the last one may be
-  // missing, and the warp's count of dead slots
-  unsigned long long wk[NW][BAT_LIST];
-  uint32_t ws[NW][BAT_LIST], wo[NW][BAT_LIST];
-  uint32_t wn[NW], wt[NW], wdead[NW];
+  // per warp: its largest face keys in descending order (0 behind them) with
+  // their faces, and the key below which keys may be missing (0: none are)
+  alignas(16) unsigned long long wk[NW * BAT_LIST];
+  uint32_t wf[NW * BAT_LIST];
+  unsigned long long wlast[NW];
   // faces of the whole walked patches (face + 1, 0 = empty) with the bit
   // mask of the walks (warps) that hold them
   uint2 btab[1u << BLK_BITS];
-  // words 0-2 of the first NRC new faces of each step
-  uint4 nrc[NW][NRC][3];
-  unsigned long long selKey[NW], maxOrph[NW];
-  uint32_t selSlot[NW], selOwn[NW];
-  uint32_t nfj[NW + 1], nalj[NW + 1];  // slot and alive counts before step j
-  uint32_t cf[NW];                     // patch j meets an earlier patch
-  uint32_t nsel, ntodo, totDead;
+  unsigned long long selKey[K];
+  uint32_t selF[K];
+  uint32_t base[K + 1], place[K + 1];  // orphans left to the block before step j; the pool's place for j's
+  uint32_t nsel, bump, live;           // picks; pool words used; candidates left
+  // the faces whose key reaches the round's threshold
+  alignas(16) unsigned long long lk[BAT_CAND];
+  uint32_t lf[BAT_CAND], nlist;
 };
 
 // open-addressing face sets in shared memory (face + 1 stored, 0 = empty)
@@ -1182,180 +1196,424 @@ __device__ __noinline__ void slot_reassign(const HullCtx& h, uint32_t i, uint32_
 __device__ __forceinline__ unsigned long long cand_key(float d, uint32_t i) {
   return ((unsigned long long)__float_as_uint(d) << 32) | (unsigned long long)(0xffffffffu - i);
 }
-// a thread's two largest candidate keys (0 = none) with slots and owners
+// a thread's two largest face keys (0 = none) with their faces
 struct Top2 {
   unsigned long long k1, k2;
-  uint32_t s1, o1, s2, o2;
+  uint32_t f1, f2;
   __device__ __forceinline__ void clear() {
     k1 = k2 = 0;
-    s1 = o1 = s2 = o2 = 0;
+    f1 = f2 = 0;
   }
-  __device__ __forceinline__ void add(unsigned long long k, uint32_t s, uint32_t o) {
+  __device__ __forceinline__ void add(unsigned long long k, uint32_t f) {
     if (k <= k2) return;
     if (k > k1) {
-      k2 = k1; s2 = s1; o2 = o1;
-      k1 = k; s1 = s; o1 = o;
+      k2 = k1; f2 = f1;
+      k1 = k; f1 = f;
     } else {
-      k2 = k; s2 = s; o2 = o;
+      k2 = k; f2 = f;
     }
   }
 };
 // every thread of the block: the warp's largest keys from its threads' two
 // largest, in descending order, for as long as the order is certain (once a
 // thread's second key is taken its third could come next, and keys below
-// the BAT_LIST-th may be missing: the list is marked truncated), and the
-// warp's count of dead slots
+// the BAT_LIST-th may be missing). One redux per key: a second one only when
+// two lanes share the largest distance.
 template <int NW>
-__device__ __forceinline__ void top2_publish(BatSm<NW>& B, const Top2& t, uint32_t dead) {
+__device__ __forceinline__ void top2_publish(BatSm<NW>& B, const Top2& t) {
   const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned long long cur = t.k1;
-  bool first = true;
-  uint32_t n = 0, trunc = 1;
-  const uint32_t dn = warp_sum_u(dead);
-  for (; n < BAT_LIST; n++) {
-    // the largest key: high words, then low words among the lanes holding
-    // the largest high word (a live key has a nonzero high word)
-    const uint32_t hi = __reduce_max_sync(FULLMASK, (uint32_t)(cur >> 32));
-    if (hi == 0) {
-      trunc = 0;
-      break;
+  uint32_t f = t.f1;
+  unsigned taken = 0;  // lanes whose first key is listed
+  unsigned long long last = 0;
+  bool more = true;  // uniform: keys may follow
+#pragma unroll
+  for (uint32_t n = 0; n < BAT_LIST; n++) {
+    const uint32_t ch = (uint32_t)(cur >> 32);
+    const uint32_t hi = more ? __reduce_max_sync(FULLMASK, ch) : 0u;
+    if (hi == 0) {  // no key left, or none certain
+      if (lane == 0) B.wk[BAT_LIST * w + n] = 0;
+      if (more) last = 0;
+      more = false;
+      continue;
     }
-    const uint32_t lo = __reduce_max_sync(FULLMASK, (uint32_t)(cur >> 32) == hi ? (uint32_t)cur : 0u);
-    const unsigned long long m = ((unsigned long long)hi << 32) | lo;
-    bool sec = false;
-    if (cur == m) {
-      B.wk[w][n] = m;
-      B.ws[w][n] = first ? t.s1 : t.s2;
-      B.wo[w][n] = first ? t.o1 : t.o2;
-      sec = !first;
-      cur = first ? t.k2 : 0ull;
-      first = false;
+    unsigned at = __ballot_sync(FULLMASK, ch == hi);
+    if (at & (at - 1)) {
+      const uint32_t lo = __reduce_max_sync(FULLMASK, ch == hi ? (uint32_t)cur : 0u);
+      at = __ballot_sync(FULLMASK, ch == hi && (uint32_t)cur == lo);
     }
-    if (__any_sync(FULLMASK, sec)) {
-      n++;
-      break;
+    const uint32_t l = __ffs(at) - 1;
+    last = ((unsigned long long)hi << 32) | __shfl_sync(FULLMASK, (uint32_t)cur, l);
+    if (lane == l) {
+      B.wk[BAT_LIST * w + n] = cur;
+      B.wf[BAT_LIST * w + n] = f;
+      cur = t.k2;
+      f = t.f2;
     }
+    if ((taken >> l) & 1u) more = false;
+    taken |= 1u << l;
+    if (lane == l && !more) cur = 0;
   }
-  if (lane == 0) {
-    B.wn[w] = n;
-    B.wt[w] = trunc;
-    B.wdead[w] = dn;
-  }
+  if (lane == 0) B.wlast[w] = last;
 }
 
-// warp 0: the block's largest keys in descending order, at most kmax, by
-// merging the warps' lists (lane w holds list w's next key). Every key of a
-// warp above the last key of its truncated list is in the list, so the
-// merge stops after taking such a last key; and the total of the dead-slot
-// counts
+// the warps that hold a list entry per lane: the block's largest keys in
+// descending order, at most kmax, each placed by its rank among the lists'
+// keys. Every key of a warp at or above its list's last key is listed, so
+// keys below the largest such bound are not taken. B.nsel is zero before.
 template <int NW>
-__device__ __noinline__ void bat_select(BatSm<NW>& B, uint32_t kmax) {
+__device__ __forceinline__ void bat_select(BatSm<NW>& B, uint32_t kmax) {
+  constexpr uint32_t N = NW * BAT_LIST;
+  const uint32_t t = threadIdx.x, lane = t & 31;
+  if (t >= N) return;
+  const unsigned long long k = B.wk[t], b = lane < NW ? B.wlast[lane] : 0ull;
+  const uint32_t bh = __reduce_max_sync(FULLMASK, (uint32_t)(b >> 32));
+  const uint32_t bl = __reduce_max_sync(FULLMASK, (uint32_t)(b >> 32) == bh ? (uint32_t)b : 0u);
+  const unsigned long long bound = ((unsigned long long)bh << 32) | bl;
+  uint32_t rank = 0;
+#pragma unroll 8
+  for (uint32_t j = 0; j < N; j += 2) {
+    const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(B.wk + j);
+    rank += (v.x > k ? 1u : 0u) + (v.y > k ? 1u : 0u);
+  }
+  const bool in = k != 0 && k >= bound && rank < kmax;
+  if (in) {
+    B.selKey[rank] = k;
+    B.selF[rank] = B.wf[t];
+  }
+  const uint32_t n = __reduce_max_sync(FULLMASK, in ? rank + 1 : 0u);
+  if (lane == 0 && n != 0) atomicMax(&B.nsel, n);
+}
+
+// ---- the candidates' pool (2 nv words from h.owner on) ----
+
+// the faces' segments one after another into h.cand, the segments' starts
+// renumbered to it; the number of candidates
+template <int NW>
+__device__ __noinline__ uint32_t pool_gather(const HullCtx& h, uint32_t nf, GrpSmem& sm) {
+  constexpr int G = 32 * NW;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t wn = lane < NW ? B.wn[lane] : 0u;
-  const bool wt = lane < NW && B.wt[lane] != 0;
-  const uint32_t dn = warp_sum_u(lane < NW ? B.wdead[lane] : 0u);
-  uint32_t pos = 0;
-  unsigned long long cur = wn > 0 ? B.wk[lane][0] : 0ull;
-  uint32_t n = 0;
-  while (n < kmax) {
-    const uint32_t hi = __reduce_max_sync(FULLMASK, (uint32_t)(cur >> 32));
-    if (hi == 0) break;
-    const uint32_t lo = __reduce_max_sync(FULLMASK, (uint32_t)(cur >> 32) == hi ? (uint32_t)cur : 0u);
-    const unsigned long long m = ((unsigned long long)hi << 32) | lo;
-    bool stop = false;
-    if (cur == m) {
-      B.selKey[n] = m;
-      B.selSlot[n] = B.ws[lane][pos];
-      B.selOwn[n] = B.wo[lane][pos];
-      pos++;
-      stop = pos == wn && wt;
-      cur = pos < wn ? B.wk[lane][pos] : 0ull;
+  const uint32_t* pool = h.owner;
+  uint32_t run = 0;
+  for (uint32_t c = 0; c * G < nf; c++) {
+    const uint32_t f = c * G + threadIdx.x;
+    const uint2 sg = f < nf ? h.fseg[f] : make_uint2(0, 0);
+    uint32_t tot;
+    const uint32_t at = run + grp_scan_u<G>(sg.y, &tot, sm);
+    unsigned some = __ballot_sync(FULLMASK, sg.y != 0);
+    while (some) {
+      const int l = __ffs(some) - 1;
+      some &= some - 1;
+      const uint32_t o = __shfl_sync(FULLMASK, sg.x, l), n = __shfl_sync(FULLMASK, sg.y, l);
+      const uint32_t t = __shfl_sync(FULLMASK, at, l);
+      for (uint32_t e = lane; e < n; e += 32) h.cand[t + e] = pool[o + e];
     }
-    n++;
-    if (__any_sync(FULLMASK, stop)) break;
+    if (f < nf) h.fseg[f].x = at;
+    run += tot;
   }
-  if (lane == 0) {
-    B.nsel = n;
-    B.totDead = dn;
+  __syncthreads();
+  return run;
+}
+
+// the live segments to the pool's front; returns the new bump pointer
+template <int NW>
+__device__ __noinline__ uint32_t pool_compact(const HullCtx& h, uint32_t nf, GrpSmem& sm, BatSm<NW>& B) {
+  const uint32_t n = pool_gather<NW>(h, nf, sm);
+  for (uint32_t k = threadIdx.x; k < n; k += 32 * NW) h.owner[k] = h.cand[k];
+  if (threadIdx.x == 0) B.bump = n;
+  __syncthreads();
+  return n;
+}
+
+// the faces' segments and keys from the list h.cand[0, ncand), its owners
+// and distances by list position (BY_SLOT) or by point; candidates without
+// an owner are dropped. The order within a segment does not matter: the
+// next pick and every reassignment are by key.
+template <int NW, bool BY_SLOT>
+__device__ __noinline__ void pool_build(const HullCtx& h, uint32_t nf, GrpSmem& sm, BatSm<NW>& B, uint32_t ncand) {
+  constexpr int G = 32 * NW;
+  const uint32_t lid = threadIdx.x, lt = lanemask_lt();
+  for (uint32_t f = lid; f < nf; f += G) {
+    h.fkey[f] = 0;
+    h.fseg[f] = make_uint2(0, 0);
   }
-  __syncwarp();
+  __syncthreads();
+  // count and largest key per face, one atomic per distinct owner in a warp
+  for (uint32_t k0 = 0; k0 < ncand; k0 += G) {
+    const uint32_t k = k0 + lid;
+    uint32_t i = 0, o = CUACD_NONE, d = 0;
+    if (k < ncand) {
+      i = h.cand[k];
+      o = h.owner[BY_SLOT ? k : i];
+      d = __float_as_uint(h.dist[BY_SLOT ? k : i]);
+    }
+    const unsigned same = __match_any_sync(FULLMASK, o);
+    const uint32_t hi = __reduce_max_sync(same, d);
+    const uint32_t lo = __reduce_max_sync(same, d == hi ? 0xffffffffu - i : 0u);
+    if (o != CUACD_NONE && (same & lt) == 0) {
+      atomicAdd(&h.fseg[o].y, __popc(same));
+      atomicMax(h.fkey + o, ((unsigned long long)hi << 32) | lo);
+    }
+  }
+  __syncthreads();
+  uint32_t run = 0;
+  for (uint32_t c = 0; c * G < nf; c++) {
+    const uint32_t f = c * G + lid;
+    const uint32_t n = f < nf ? h.fseg[f].y : 0u;
+    uint32_t tot;
+    const uint32_t at = run + grp_scan_u<G>(n, &tot, sm);
+    if (f < nf) h.fseg[f].x = at;
+    run += tot;
+  }
+  __syncthreads();
+  // the owners occupy the pool's words: the segments go through h.hA
+  for (uint32_t k0 = 0; k0 < ncand; k0 += G) {
+    const uint32_t k = k0 + lid;
+    uint32_t i = 0, o = CUACD_NONE;
+    if (k < ncand) {
+      i = h.cand[k];
+      o = h.owner[BY_SLOT ? k : i];
+    }
+    const unsigned same = __match_any_sync(FULLMASK, o);
+    const int lead = __ffs(same) - 1;
+    uint32_t at = 0;
+    if (o != CUACD_NONE && (same & lt) == 0) at = atomicAdd(&h.fseg[o].x, __popc(same));
+    at = __shfl_sync(FULLMASK, at, lead) + __popc(same & lt);
+    if (o != CUACD_NONE) h.hA[at] = i;
+  }
+  __syncthreads();
+  for (uint32_t f = lid; f < nf; f += G) h.fseg[f].x -= h.fseg[f].y;
+  for (uint32_t k = lid; k < run; k += G) h.owner[k] = h.hA[k];
+  if (lid == 0) B.bump = B.live = run;
+  __syncthreads();
+}
+
+// the single-pick step for the selection's first pick: hull_insert's
+// compaction by the whole block, big_insert (hull_insert for a patch above
+// BIG_VIS faces) by warp 0, then the points of the dead faces (all points
+// after a compaction) are reassigned
+template <int NW>
+__device__ __noinline__ void big_seq_step(const HullCtx& h, HullSm& hs, GrpSmem& sm, BatSm<NW>& B) {
+  constexpr int G = 32 * NW;
+  BigSm& bs = B.u.big;
+  const uint32_t lid = threadIdx.x, warp = lid >> 5, lane = lid & 31;
+  const uint32_t pick = 0xffffffffu - (uint32_t)(B.selKey[0] & 0xffffffffu);
+  uint32_t start = B.selF[0], ncand = 0;
+  // read before the barrier: warp 0 moves them in its insertion
+  const uint32_t nf = hs.nf;
+  const bool compact = nf + 3 * HULL_VIS_MAX > h.fmax || nf > 2 * hs.nalive + 512;
+  if (lid == 0) {
+    hs.compacted = 0;
+    hs.remapN = 0;
+  }
+  __syncthreads();
+  if (compact) {
+    // every candidate in a list with its owner, which the compaction renumbers
+    ncand = pool_gather<NW>(h, nf, sm);
+    for (uint32_t f0 = 32 * warp; f0 < nf; f0 += G) {
+      const uint2 sg = f0 + lane < nf ? h.fseg[f0 + lane] : make_uint2(0, 0);
+      unsigned some = __ballot_sync(FULLMASK, sg.y != 0);
+      while (some) {
+        const int l = __ffs(some) - 1;
+        some &= some - 1;
+        const uint32_t o = __shfl_sync(FULLMASK, sg.x, l), n = __shfl_sync(FULLMASK, sg.y, l);
+        for (uint32_t e = lane; e < n; e += 32) h.owner[o + e] = f0 + l;
+      }
+    }
+    __syncthreads();
+    start = hull_compact<G>(h, hs, sm, start, h.owner, ncand);
+  }
+  if (warp == 0) {
+    const bool fast = big_insert(h, hs, bs, pick, start);
+    if (!fast) hull_insert<32>(h, hs, sm, pick, start);
+    if (lane == 0) bs.fast = fast ? 1u : 0u;
+  }
+  __syncthreads();
+  if (hs.fail) return;
+  const uint32_t nfNow = hs.nf, newBase = hs.newBase, nvis = hs.nvis;
+  const bool compacted = hs.compacted != 0, fast = bs.fast != 0;
+  if (compacted) {
+    for (uint32_t k = lid; k < ncand; k += G) {
+      const uint32_t i = h.cand[k], own = h.owner[k];
+      uint32_t no = CUACD_NONE;
+      float nd = 0.0f;
+      if (i != pick)
+        slot_reassign(h, i, own, fast ? big_has(bs, own) : bm_test(h.bm, own), true, newBase, nfNow, nullptr, no, nd);
+      h.owner[k] = no;
+      h.dist[k] = nd;
+    }
+    __syncthreads();
+    if (!fast)
+      for (uint32_t vi = lid; vi < nvis; vi += G) h.bm[h.vis[vi] >> 5] = 0;
+    pool_build<NW, true>(h, nfNow, sm, B, ncand);
+    return;
+  }
+  // room for every candidate beyond the bump pointer, then the dead faces'
+  // points to the new faces: a warp per dead face; the new owner is kept at
+  // the point's pool position in h.hA and h.hB (2 nv words)
+  if ((uint64_t)B.bump + B.live > 2ull * h.nv) pool_compact<NW>(h, newBase, sm, B);
+  for (uint32_t f = newBase + lid; f < nfNow; f += G) {
+    h.fkey[f] = 0;
+    h.fseg[f] = make_uint2(0, 0);
+  }
+  __syncthreads();
+  const uint32_t* dead = fast ? bs.f : h.vis;
+  uint32_t* pool = h.owner;
+  for (uint32_t v = warp; v < nvis; v += NW) {
+    const uint2 sg = h.fseg[dead[v]];
+    for (uint32_t e = lane; e < sg.y; e += 32) {
+      const uint32_t i = pool[sg.x + e];
+      uint32_t no = CUACD_NONE;
+      float nd = 0.0f;
+      if (i != pick)
+        slot_reassign(h, i, 0, true, false, newBase, nfNow, fast ? bs.nrec : nullptr, no, nd);
+      h.hA[sg.x + e] = no;
+      if (no == CUACD_NONE) {
+        atomicSub(&B.live, 1u);
+      } else {
+        atomicAdd(&h.fseg[no].y, 1u);
+        atomicMax(h.fkey + no, cand_key(nd, i));
+      }
+    }
+  }
+  __syncthreads();
+  uint32_t run = B.bump;
+  for (uint32_t c = 0; newBase + c * G < nfNow; c++) {
+    const uint32_t f = newBase + c * G + lid;
+    const uint32_t n = f < nfNow ? h.fseg[f].y : 0u;
+    uint32_t tot;
+    const uint32_t at = run + grp_scan_u<G>(n, &tot, sm);
+    if (f < nfNow) h.fseg[f].x = at;
+    run += tot;
+  }
+  __syncthreads();
+  for (uint32_t v = warp; v < nvis; v += NW) {
+    const uint2 sg = h.fseg[dead[v]];
+    for (uint32_t e = lane; e < sg.y; e += 32) {
+      const uint32_t no = h.hA[sg.x + e];
+      if (no != CUACD_NONE) pool[atomicAdd(&h.fseg[no].x, 1u)] = pool[sg.x + e];
+    }
+  }
+  __syncthreads();
+  for (uint32_t f = newBase + lid; f < nfNow; f += G) h.fseg[f].x -= h.fseg[f].y;
+  for (uint32_t v = lid; v < nvis; v += G) {
+    const uint32_t f = dead[v];
+    h.fkey[f] = 0;
+    h.fseg[f] = make_uint2(0, 0);
+    if (!fast) h.bm[f >> 5] = 0;
+  }
+  if (lid == 0) B.bump = run;
+  __syncthreads();
+}
+
+// best_face over every step-th of a walk's new faces from `from` on: the
+// face's number q and the distance
+__device__ __forceinline__ void bat_best(const HullCtx& h, const BatWalk& W, f3 pt, uint32_t i, uint32_t from,
+                                         uint32_t step, uint32_t& outQ, float& outD) {
+  uint32_t bestQ = CUACD_NONE;
+  float bestD = 0.0f;
+  const uint32_t nnew = W.nnew;
+  for (uint32_t q = from; q < nnew; q += step) {
+    const uint4 w0 = W.rec[q][0], w1 = W.rec[q][1], w2 = W.rec[q][2];
+    const float dd = h.face_filter(w0, w1, w2, pt, i);
+    if (dd > bestD) { bestD = dd; bestQ = q; }
+    if (dd == 0.0f && bestQ == CUACD_NONE && h.face_exact(w2, W.rec[q][3], pt)) { bestD = 1e-30f; bestQ = q; }
+  }
+  outQ = bestQ;
+  outD = bestD;
 }
 
 // one warp: the visible patch of point pIdx on the current hull, walked
 // from its owner face `start` as big_insert walks it, in slot order, and
 // its horizon edges in the insertion's order (e = 3 * listPos + k); the
-// patch's faces also go into the block's set with the warp's bit. W.ok = 0
-// when the patch has more than BAT_FACES faces.
+// patch's faces also go into the block's set with the warp's bit. False when
+// the patch or its horizon does not fit the warp's lanes.
 template <int NW>
-__device__ __noinline__ void bat_walk(const HullCtx& h, uint32_t nf, BatSm<NW>& B, uint32_t pIdx, uint32_t start) {
+__device__ __forceinline__ bool bat_walk(const HullCtx& h, uint32_t nf, BatSm<NW>& B, BatWalk& W, uint32_t pIdx, f3 p,
+                                         uint32_t start) {
   constexpr uint32_t HB = BAT_HASH_BITS;
   const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  BatWalk& W = B.u.w[warp];
   const uint32_t lt = lanemask_lt();
-  const f3 p = h.qvert(pIdx);
+  // the faces across the start face's edges (lanes 0-2) and across theirs
+  // (lanes 3-11) together: most patches end within them, and a level of the
+  // walk below costs as much as this one
+  const uint4 nbS = *reinterpret_cast<const uint4*>(h.nbr + 4 * (size_t)start);
+  const uint32_t ring = lane < 3 ? lane : (lane - 3) / 3;
+  uint32_t g = ring == 0 ? nbS.x : (ring == 1 ? nbS.y : nbS.z);
+  if (lane >= 3 && lane < 12 && g < nf) g = h.nbr[4 * (size_t)g + (lane - 3) % 3];
   for (uint32_t j = lane; j < (1u << HB); j += 32) W.key[j] = 0;
   __syncwarp();
-  if (lane == 0) {
-    uint32_t at;
-    tab_add<HB>(W.key, start, at);
+  if (lane == 31) {
+    W.key[tab_hash<HB>(start)] = start + 1;
     W.f[0] = start;
     const uint4 w0 = h.rec(start)[0];
-    const uint4 nb = *reinterpret_cast<const uint4*>(h.nbr + 4 * (size_t)start);
+    const uint2 sg = h.fseg[start];
     W.vabc[0][0] = w0.x & 0x7fffffffu; W.vabc[0][1] = w0.y; W.vabc[0][2] = w0.z;
-    W.nb[0][0] = nb.x; W.nb[0][1] = nb.y; W.nb[0][2] = nb.z;
+    W.nb[0][0] = nbS.x; W.nb[0][1] = nbS.y; W.nb[0][2] = nbS.z;
+    W.seg[0] = sg;
   }
   __syncwarp();
+  uint4 w0 = make_uint4(0, 0, 0, 0), nb = w0;
+  uint2 sg = make_uint2(0, 0);
+  auto sees = [&](uint32_t f) -> bool {  // loads face f; whether the point sees it
+    const uint4* r = h.rec(f);
+    w0 = r[0];
+    const uint4 w1 = r[1], w2 = r[2];
+    nb = *reinterpret_cast<const uint4*>(h.nbr + 4 * (size_t)f);
+    sg = h.fseg[f];
+    if ((w0.x & ALIVE) == 0) return false;
+    const int v = h.face_side(w0, w1, w2, p, pIdx);
+    return v > 0 || (v == 0 && h.face_exact(w2, r[3], p));
+  };
+  auto keep = [&](uint32_t at) {
+    if (at >= BAT_FACES) return;
+    W.f[at] = g;
+    W.vabc[at][0] = w0.x & 0x7fffffffu; W.vabc[at][1] = w0.y; W.vabc[at][2] = w0.z;
+    W.nb[at][0] = nb.x; W.nb[at][1] = nb.y; W.nb[at][2] = nb.z;
+    W.seg[at] = sg;
+  };
   uint32_t head = 0, qn = 1;
-  bool bad = false;
-  for (;;) {
+  bool over = false;
+  static_assert(BAT_FACES >= 13, "the start face and both rings fit the patch");
+  {
+    const bool vis = lane < 12 && g < nf && sees(g);
+    const unsigned visible = __ballot_sync(FULLMASK, vis);
+    bool claimed = false;
+    if (vis && (lane < 3 || ((visible >> ring) & 1u))) {
+      uint32_t at;
+      const uint32_t rr = tab_add<HB>(W.key, g, at);
+      claimed = rr == 1;
+      over = rr == 2;
+    }
+    const unsigned m = __ballot_sync(FULLMASK, claimed);
+    if (claimed) keep(1 + __popc(m & lt));
+    head = 1 + __popc(m & 7u);  // the first ring's neighbours have been looked at
+    qn = 1 + __popc(m);
+    __syncwarp();
+  }
+  while (head < qn) {
     const uint32_t tasks = 3 * (qn - head);
     uint32_t added = 0;
-    bool over = false;
     for (uint32_t t0 = 0; t0 < tasks; t0 += 32) {
       const uint32_t t = t0 + lane;
       bool claimed = false;
-      uint32_t g = 0;
-      uint4 w0 = make_uint4(0, 0, 0, 0), nb = w0;
       if (t < tasks) {
         g = W.nb[head + t / 3][t % 3];
-        if (g < nf && !tab_has<HB>(W.key, g)) {
-          const uint4* r = h.rec(g);
-          w0 = r[0];
-          const uint4 w1 = r[1], w2 = r[2];
-          nb = *reinterpret_cast<const uint4*>(h.nbr + 4 * (size_t)g);
-          if (w0.x & ALIVE) {
-            const float v = h.face_filter(w0, w1, w2, p, pIdx);
-            if (v > 0.0f || (v == 0.0f && h.face_exact(w2, r[3], p))) {
-              uint32_t at;
-              const uint32_t rr = tab_add<HB>(W.key, g, at);
-              claimed = rr == 1;
-              over = rr == 2;
-            }
-          }
+        if (g < nf && !tab_has<HB>(W.key, g) && sees(g)) {
+          uint32_t at;
+          const uint32_t rr = tab_add<HB>(W.key, g, at);
+          claimed = rr == 1;
+          over = over || rr == 2;
         }
       }
       const unsigned m = __ballot_sync(FULLMASK, claimed);
-      const uint32_t at = qn + added + __popc(m & lt);
-      if (claimed && at < BAT_FACES) {
-        W.f[at] = g;
-        W.vabc[at][0] = w0.x & 0x7fffffffu; W.vabc[at][1] = w0.y; W.vabc[at][2] = w0.z;
-        W.nb[at][0] = nb.x; W.nb[at][1] = nb.y; W.nb[at][2] = nb.z;
-      }
+      if (claimed) keep(qn + added + __popc(m & lt));
       added += __popc(m);
     }
     __syncwarp();
     head = qn;
     qn += added;
-    if (__any_sync(FULLMASK, over) || qn > BAT_FACES) {
-      bad = true;
-      break;
-    }
-    if (head == qn) break;
-  }
-  if (bad) {
-    if (lane == 0) W.ok = 0;
-    __syncwarp();
-    return;
+    if (__any_sync(FULLMASK, over) || qn > BAT_FACES) return false;
   }
   const uint32_t n = qn;
   if (lane < n) {
@@ -1365,6 +1623,10 @@ __device__ __noinline__ void bat_walk(const HullCtx& h, uint32_t nf, BatSm<NW>& 
     W.ord[r] = lane;
     btab_add(B, fi, 1u << warp);
   }
+  const uint32_t oc = lane < n ? W.seg[lane].y : 0u;
+  const uint32_t oi = warp_incl_u(oc, (int)lane);
+  W.segPre[lane] = oi - oc;
+  if (lane == 31) W.norph = oi;
   __syncwarp();
   uint32_t nnew = 0;
   for (uint32_t c = 0; c * 32 < 3 * n; c++) {
@@ -1392,433 +1654,268 @@ __device__ __noinline__ void bat_walk(const HullCtx& h, uint32_t nf, BatSm<NW>& 
   if (lane == 0) {
     W.n = n;
     W.nnew = nnew;
-    W.ok = nnew <= BAT_NEW ? 1u : 0u;
-    W.pick = pIdx;
   }
   __syncwarp();
+  return nnew <= BAT_NEW;
 }
 
-// warp j < K: whether patch j meets an earlier walked patch (a face of
-// patch j, or a face across one of its edges, was claimed by a walk i < j);
-// the round's counters are reset
-template <int NW>
-__device__ __noinline__ void bat_conflicts(BatSm<NW>& B, uint32_t K) {
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) B.ntodo = 0;
-  if (threadIdx.x < NW) B.maxOrph[threadIdx.x] = 0;
-  if (warp >= K) return;
-  const BatWalk& W = B.u.w[warp];
-  const uint32_t below = (1u << warp) - 1u;
-  bool hit = false;
-  if (W.ok && lane < W.n) {
-    const uint32_t g[4] = {W.f[lane], W.nb[lane][0], W.nb[lane][1], W.nb[lane][2]};
-#pragma unroll
-    for (int k = 0; k < 4; k++) hit = hit || (btab_mask(B, g[k]) & below) != 0;
+// the pool position of a walk's orphan e < norph
+__device__ __forceinline__ uint32_t orphan_at(const BatWalk& W, uint32_t e) {
+  uint32_t lo = 0, hi = W.n;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (W.segPre[mid] <= e) lo = mid;
+    else hi = mid;
   }
-  hit = __any_sync(FULLMASK, hit);
-  if (lane == 0) B.cf[warp] = hit ? 1u : 0u;
+  return W.seg[lo].x + (e - W.segPre[lo]);
 }
 
-// every thread: the number of accepted steps ms, the longest prefix of the
-// walked picks whose patches are whole, disjoint and not adjacent, with
-// neither the compaction rule (steps after the first) nor the slot limit
-// firing; *base = the first new-face slot of the thread's warp's step.
-// Thread 0 stores the slot and alive counts before each step.
-template <int NW>
-__device__ __noinline__ uint32_t bat_prefix(const HullCtx& h, const HullSm& hs, BatSm<NW>& B, uint32_t K,
-                                            uint32_t* base) {
-  const uint32_t warp = threadIdx.x >> 5;
-  uint32_t nfc = hs.nf, nalc = hs.nalive, ms = 0;
-  *base = nfc;
-  for (uint32_t j = 0; j < K; j++) {
-    const BatWalk& W = B.u.w[j];
-    if (!W.ok || B.cf[j]) break;
-    if (j > 0 && (nfc + 3 * HULL_VIS_MAX > h.fmax || nfc > 2 * nalc + 512)) break;
-    if (nfc + 3 * W.n > h.fmax) break;
-    if (threadIdx.x == 0) {
-      B.nfj[j] = nfc;
-      B.nalj[j] = nalc;
-    }
-    if (j == warp) *base = nfc;
-    nfc += W.nnew;
-    nalc = nalc + W.nnew - W.n;
-    ms = j + 1;
-  }
-  if (threadIdx.x == 0) {
-    B.nfj[ms] = nfc;
-    B.nalj[ms] = nalc;
-  }
-  return ms;
+// one warp: the places of a walk's new faces' candidates and the largest key
+__device__ __forceinline__ void bat_sums(BatWalk& W) {
+  const uint32_t lane = threadIdx.x & 31;
+  const unsigned long long k = W.fk[lane];
+  const uint32_t c = W.cnt[lane];
+  const uint32_t inc = warp_incl_u(c, (int)lane);
+  W.pre[lane] = inc - c;
+  const uint32_t hi = __reduce_max_sync(FULLMASK, (uint32_t)(k >> 32));
+  const uint32_t lo = __reduce_max_sync(FULLMASK, (uint32_t)(k >> 32) == hi ? (uint32_t)k : 0u);
+  if (lane == 31) W.tot = inc;
+  if (lane == 0) W.maxOrph = ((unsigned long long)hi << 32) | lo;
 }
 
-// squeeze dead slots out of the candidate list (slot order kept); returns
-// the new count and publishes the threads' keys
+// A batched round over the selection's K picks. Each pick's warp walks its
+// patch, forms its new faces and, for up to 32 orphans, their new owners,
+// all before it is known which picks the round takes (nothing in the slab
+// changes): one barrier instead of one after each step, and a warp waits
+// for the slowest whole pick, not for the slowest walk, then the slowest
+// face set, and so on. Then the longest prefix of whole, disjoint,
+// non-adjacent patches (compaction rule and slot limit included); larger
+// orphan sets of those, spread over the block; the accepted prefix from the
+// largest new key per step; and its commit. Returns the number of
+// insertions, 0 when the single-pick step has to run.
 template <int NW>
-__device__ __noinline__ uint32_t big_squeeze(const HullCtx& h, GrpSmem& sm, BatSm<NW>& B, uint32_t ncand) {
+__device__ __noinline__ uint32_t bat_round(const HullCtx& h, HullSm& hs, GrpSmem& sm, BatSm<NW>& B, uint32_t K) {
   constexpr int G = 32 * NW;
-  const uint32_t lid = threadIdx.x;
-  uint32_t nc = 0;
-  Top2 t;
-  t.clear();
-  for (uint32_t c = 0; c * G < ncand; c++) {
-    const uint32_t k = c * G + lid;
-    uint32_t o = CUACD_NONE, i = 0;
-    float d = 0.0f;
-    if (k < ncand) {
-      o = h.owner[k];
-      i = h.cand[k];
-      d = h.dist[k];
-    }
-    uint32_t tot;
-    const uint32_t pre = grp_scan_bit<G>(o != CUACD_NONE, &tot, sm);
-    __syncthreads();
-    if (o != CUACD_NONE) {
-      const uint32_t at = nc + pre;
-      h.cand[at] = i;
-      h.owner[at] = o;
-      h.dist[at] = d;
-      t.add(cand_key(d, i), at, o);
-    }
-    nc += tot;
-    __syncthreads();
-  }
-  top2_publish(B, t, 0);
-  __syncthreads();
-  return nc;
-}
-
-// the single-pick step for the selection's first pick: hull_insert's
-// compaction by the whole block, big_insert (hull_insert for a patch above
-// BIG_VIS faces) by warp 0, then one pass over the candidate slots: the
-// inserted point leaves, points of dead faces (all points after a
-// compaction) are reassigned, and the threads' keys are published
-template <int NW>
-__device__ __noinline__ void big_seq_step(const HullCtx& h, HullSm& hs, GrpSmem& sm, BatSm<NW>& B, uint32_t ncand) {
-  constexpr int G = 32 * NW;
-  BigSm& bs = B.u.big;
-  const uint32_t lid = threadIdx.x;
-  uint32_t* cown = h.owner;
-  float* cdist = h.dist;
-  const uint32_t pick = 0xffffffffu - (uint32_t)(B.selKey[0] & 0xffffffffu);
-  const uint32_t pickSlot = B.selSlot[0];
-  uint32_t start = B.selOwn[0];
-  {
-    if (lid == 0) {
-      hs.compacted = 0;
-      hs.remapN = 0;
-      bs.ntodo = 0;
-    }
-    __syncthreads();
-    if (hs.nf + 3 * HULL_VIS_MAX > h.fmax || hs.nf > 2 * hs.nalive + 512) {
-      start = hull_compact<G>(h, hs, sm, start, cown, ncand);
-    }
-    if (threadIdx.x < 32) {
-      const bool fast = big_insert(h, hs, bs, pick, start);
-      if (!fast) hull_insert<32>(h, hs, sm, pick, start);
-      if (threadIdx.x == 0) bs.fast = fast ? 1u : 0u;
-    }
-    __syncthreads();
-    if (hs.fail) return;
-    const uint32_t nfNow = hs.nf, newBase = hs.newBase;
-    const bool compacted = hs.compacted != 0, fast = bs.fast != 0;
-    Top2 top;
-    top.clear();
-    uint32_t dead = 0;
-    bool sweep = compacted;
-    if (!compacted) {
-      // scan, four slots per thread in flight; the slots whose owner died
-      // are listed (in the walk queue's words, free after an insertion) and
-      // reassigned by the whole block afterwards
-      uint32_t* todo = h.q;
-      for (uint32_t k0 = lid; k0 < ncand; k0 += 4 * G) {
-        uint32_t ow[4], ci[4];
-        float cd[4];
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const uint32_t k = k0 + u * G;
-          const bool in = k < ncand;
-          ow[u] = in ? cown[k] : CUACD_NONE;
-          ci[u] = in ? h.cand[k] : 0u;
-          cd[u] = in ? cdist[k] : 0.0f;
-        }
-#pragma unroll
-        for (int u = 0; u < 4; u++) {
-          const uint32_t k = k0 + u * G;
-          if (k >= ncand) break;
-          const uint32_t own = ow[u];
-          if (own == CUACD_NONE) {
-            dead++;
-            continue;
-          }
-          if (k == pickSlot) {
-            cown[k] = CUACD_NONE;
-            dead++;
-            continue;
-          }
-          if (fast ? big_has(bs, own) : bm_test(h.bm, own)) {
-            const uint32_t t = atomicAdd(&bs.ntodo, 1u);
-            if (t < HULL_VIS_MAX) todo[t] = k;
-            continue;
-          }
-          const unsigned long long key = cand_key(cd[u], ci[u]);
-          top.add(key, k, own);
-        }
-      }
-      __syncthreads();
-      const uint32_t nt = bs.ntodo;
-      for (uint32_t t = lid; t < min(nt, HULL_VIS_MAX); t += G) {
-        const uint32_t k = todo[t], i = h.cand[k];
-        uint32_t own;
-        float d;
-        slot_reassign(h, i, cown[k], true, false, newBase, nfNow, fast ? bs.nrec : nullptr, own, d);
-        cown[k] = own;
-        cdist[k] = d;
-        if (own == CUACD_NONE) {
-          dead++;
-        } else {
-          const unsigned long long key = cand_key(d, i);
-          top.add(key, k, own);
-        }
-      }
-      // more than the list holds: the rest is found by a sweep
-      sweep = nt > HULL_VIS_MAX;
-      __syncthreads();
-    }
-    if (sweep) {
-      for (uint32_t k = lid; k < ncand; k += G) {
-        uint32_t own = cown[k];
-        if (own == CUACD_NONE) {
-          if (compacted) dead++;
-          continue;
-        }
-        if (compacted && k == pickSlot) {
-          cown[k] = CUACD_NONE;
-          dead++;
-          continue;
-        }
-        const bool gone = fast ? big_has(bs, own) : bm_test(h.bm, own);
-        if (!compacted && !gone) continue;
-        const uint32_t i = h.cand[k];
-        float d;
-        slot_reassign(h, i, own, gone, compacted, newBase, nfNow, fast ? bs.nrec : nullptr, own, d);
-        cown[k] = own;
-        cdist[k] = d;
-        if (own == CUACD_NONE) {
-          dead++;
-        } else {
-          const unsigned long long key = cand_key(d, i);
-          top.add(key, k, own);
-        }
-      }
-    }
-    __syncthreads();
-    if (!fast) {
-      for (uint32_t vi = lid; vi < hs.nvis; vi += G) h.bm[h.vis[vi] >> 5] = 0;
-    }
-    top2_publish(B, top, dead);
-    __syncthreads();
-  }
-}
-
-// best_face over the new faces [f0, f1) of one step (all alive), the first
-// NRC records read from shared memory
-template <uint32_t NRC>
-__device__ __forceinline__ void bat_best(const HullCtx& h, uint32_t i, uint32_t f0, uint32_t f1, const uint4 (*nrc)[3],
-                                         uint32_t& outF, float& outD) {
-  const f3 pt = h.qvert(i);
-  uint32_t bestF = CUACD_NONE;
-  float bestD = 0.0f;
-  for (uint32_t f = f0; f < f1; f++) {
-    const uint32_t q = f - f0;
-    uint4 w0, w1, w2;
-    if (q < NRC) {
-      w0 = nrc[q][0]; w1 = nrc[q][1]; w2 = nrc[q][2];
-    } else {
-      const uint4* w = h.rec(f);
-      w0 = w[0]; w1 = w[1]; w2 = w[2];
-    }
-    const float dd = h.face_filter(w0, w1, w2, pt, i);
-    if (dd > bestD) { bestD = dd; bestF = f; }
-    if (dd == 0.0f && bestF == CUACD_NONE && h.face_exact(w2, h.rec(f)[3], pt)) { bestD = 1e-30f; bestF = f; }
-  }
-  outF = bestF;
-  outD = bestD;
-}
-
-// A batched round after validation (ms >= 1 steps): the new faces of every
-// validated step at their slots while one pass over the candidate slots
-// lists the orphans of the validated patches (six words each in the
-// visible list's and walk queue's words: slot, point, owner, then new
-// owner, new distance, step), the orphans' new owners over their step's
-// new faces and the largest new key per step, the accepted prefix, then its
-// commit (twin links, dead faces, counts) and the orphans' new owners.
-// Returns the number of insertions.
-template <int NW>
-__device__ __noinline__ uint32_t bat_step(const HullCtx& h, HullSm& hs, BatSm<NW>& B, uint32_t ncand, uint32_t ms,
-                                          uint32_t myBase) {
-  constexpr int G = 32 * NW;
-  constexpr uint32_t NRC = BatSm<NW>::NRC;
   const uint32_t lid = threadIdx.x, warp = lid >> 5, lane = lid & 31;
-  const uint32_t nf0 = hs.nf;
-  uint32_t* tK = h.vis;
-  uint32_t* tI = h.vis + TODO_CAP;
-  uint32_t* tO = h.vis + 2 * TODO_CAP;
-  uint32_t* tNO = h.q;
-  uint32_t* tND = h.q + TODO_CAP;
-  uint32_t* tJ = h.q + 2 * TODO_CAP;
-  // new faces (a, b, pick) and the links among them and to the twins;
-  // records of steps that are not accepted lie above the slot count and
-  // are overwritten later
-  if (warp < ms) {
-    const BatWalk& W = B.u.w[warp];
-    const uint32_t base = myBase, nnew = W.nnew, pIdx = W.pick;
+  static_assert(BatSm<NW>::K < 32, "a lane past the last step");
+  // read before the round's barriers: thread 0 moves them at its end
+  const uint32_t nf0 = hs.nf, nal0 = hs.nalive;
+  uint32_t bump = B.bump;
+  uint32_t* pool = h.owner;
+  const bool mine = warp < K;
+  BatWalk& W = B.u.w[mine ? warp : 0];
+  // the lane's new face's links and its orphan (point, face, rank)
+  // (tslot: which of the twin's links lead to the face it replaces)
+  uint32_t j1 = 0, j2 = 0, tslot = 0, oi = 0, oq = CUACD_NONE, orank = 0;
+  if (mine) {
+    const uint32_t pIdx = 0xffffffffu - (uint32_t)(B.selKey[warp] & 0xffffffffu);
     const f3 p = h.qvert(pIdx);
-    for (uint32_t q = lane; q < nnew; q += 32) {
-      const uint32_t a = W.hA[q], b = W.hB[q], s = base + q;
-      uint4 w0, w1, w2, w3;
-      h.face_make_q(a, b, pIdx, p, w0, w1, w2, w3);
-      uint4* w = h.rec(s);
-      w[0] = w0; w[1] = w1; w[2] = w2; w[3] = w3;
-      if (q < NRC) {
-        B.nrc[warp][q][0] = w0; B.nrc[warp][q][1] = w1; B.nrc[warp][q][2] = w2;
-      }
-      // around the horizon loop: (b, p) borders the new face starting at
-      // b, (p, a) the new face ending at a
-      uint32_t j1 = 0, j2 = 0;
-      for (uint32_t r = 0; r < nnew; r++) {
-        if (W.hA[r] == b) j1 = r;
-        if (W.hB[r] == a) j2 = r;
-      }
-      uint32_t* nq = h.nbr + 4 * (size_t)s;
-      nq[0] = W.tw[q];
-      nq[1] = base + j1;
-      nq[2] = base + j2;
+    const bool ok = bat_walk(h, nf0, B, W, pIdx, p, B.selF[warp]);
+    if (lane == 0) {
+      W.ok = ok ? 1u : 0u;
+      W.pick = pIdx;
     }
-  }
-  // one pass over the slots, SCAN_U per thread in flight
-  Top2 top;
-  top.clear();
-  uint32_t dead = 0;
-  for (uint32_t k0 = lid; k0 < ncand; k0 += SCAN_U * G) {
-    uint32_t ow[SCAN_U], ci[SCAN_U];
-    float cd[SCAN_U];
-#pragma unroll
-    for (int u = 0; u < SCAN_U; u++) {
-      const uint32_t k = k0 + u * G;
-      const bool in = k < ncand;
-      ow[u] = in ? h.owner[k] : CUACD_NONE;
-      ci[u] = in ? h.cand[k] : 0u;
-      cd[u] = in ? h.dist[k] : 0.0f;
-    }
-#pragma unroll
-    for (int u = 0; u < SCAN_U; u++) {
-      const uint32_t k = k0 + u * G;
-      if (k >= ncand) break;
-      const uint32_t own = ow[u];
-      if (own == CUACD_NONE) {
-        dead++;
-        continue;
-      }
-      // the first walk holding the owner: an earlier step's patch when two
-      // hold it, and then only that step can be accepted
-      const uint32_t j = __ffs(btab_mask(B, own)) - 1u;
-      if (j < ms) {
-        const uint32_t t = atomicAdd(&B.ntodo, 1u);
-        if (t < TODO_CAP) {
-          tK[t] = k;
-          tI[t] = ci[u];
-          tO[t] = own;
-          tJ[t] = j;
+    if (ok) {
+      const uint32_t nnew = W.nnew, norph = W.norph;
+      W.cnt[lane] = 0;
+      W.fk[lane] = 0;
+      // few orphans take 8, 4 or 2 lanes each, which split the new faces;
+      // the orphan's point, the new face's corners and the twin's
+      // neighbours are loaded together
+      const uint32_t sh = norph <= 4 ? 3u : (norph <= 8 ? 2u : (norph <= 16 ? 1u : 0u));
+      const uint32_t e = lane >> sh, sub = lane & ((1u << sh) - 1u);
+      const bool has = norph <= 32 && e < norph;
+      if (has) oi = pool[orphan_at(W, e)];
+      const bool face = lane < nnew;
+      const uint32_t a = face ? W.hA[lane] : pIdx, b = face ? W.hB[lane] : pIdx;
+      const uint32_t twin = face ? W.tw[lane] : CUACD_NONE;
+      uint4 tn = make_uint4(0, 0, 0, 0);
+      if (twin < nf0) tn = *reinterpret_cast<const uint4*>(h.nbr + 4 * (size_t)twin);
+      const f3 qa = h.qvert(a), qb = h.qvert(b);
+      const f3 pt = h.qvert(oi);
+      // new face (a, b, pick), and its neighbours around the horizon loop:
+      // (b, p) borders the new face starting at b, (p, a) the one ending at a
+      if (face) {
+        const uint32_t df = W.df[lane];
+        tslot = (tn.x == df ? 1u : 0u) | (tn.y == df ? 2u : 0u) | (tn.z == df ? 4u : 0u);
+        for (uint32_t r = 0; r < nnew; r++) {
+          if (W.hA[r] == b) j1 = r;
+          if (W.hB[r] == a) j2 = r;
         }
-        continue;
+        uint4 w0, w1, w2, w3;
+        h.face_make_abc(a, b, pIdx, qa, qb, p, w0, w1, w2, w3);
+        W.rec[lane][0] = w0; W.rec[lane][1] = w1; W.rec[lane][2] = w2; W.rec[lane][3] = w3;
       }
-      top.add(cand_key(cd[u], ci[u]), k, own);
+      __syncwarp();
+      if (norph <= 32) {
+        uint32_t q = CUACD_NONE;
+        float nd = 0.0f;
+        if (has && oi != pIdx) bat_best(h, W, pt, oi, sub, 1u << sh, q, nd);
+        for (uint32_t o = 1; o < (1u << sh); o <<= 1) {
+          const float d2 = __shfl_xor_sync(FULLMASK, nd, o);
+          const uint32_t q2 = __shfl_xor_sync(FULLMASK, q, o);
+          if (d2 > nd || (d2 == nd && q2 < q)) { nd = d2; q = q2; }
+        }
+        if (sub == 0 && q != CUACD_NONE) {
+          oq = q;
+          orank = atomicAdd(W.cnt + q, 1u);
+          atomicMax(W.fk + q, cand_key(nd, oi));
+        }
+        __syncwarp();
+        bat_sums(W);
+      }
     }
   }
   __syncthreads();
-  const uint32_t nt = B.ntodo;
-  uint32_t m = 1;
-  if (nt <= TODO_CAP) {
-    for (uint32_t t = lid; t < nt; t += G) {
-      const uint32_t k = tK[t], i = tI[t], j = tJ[t];
-      uint32_t no = CUACD_NONE;
-      float nd = 0.0f;
-      if (k != B.selSlot[j]) {
-        bat_best<NRC>(h, i, B.nfj[j], B.nfj[j + 1], B.nrc[j], no, nd);
-        if (no != CUACD_NONE) atomicMax(&B.maxOrph[j], cand_key(nd, i));
-      }
-      tNO[t] = no;
-      tND[t] = __float_as_uint(nd);
+  // whether patch j meets an earlier walked patch (a face of patch j, or a
+  // face across one of its edges, was claimed by a walk i < j)
+  if (mine) {
+    const uint32_t below = (1u << warp) - 1u;
+    bool hit = false;
+    if (W.ok && lane < W.n) {
+      const uint32_t g[4] = {W.f[lane], W.nb[lane][0], W.nb[lane][1], W.nb[lane][2]};
+#pragma unroll
+      for (int k = 0; k < 4; k++) hit = hit || (btab_mask(B, g[k]) & below) != 0;
     }
-    __syncthreads();
-    // pick j is next while every earlier step's orphans stay below its key
-    unsigned long long run = B.maxOrph[0];
-    for (uint32_t j = 1; j < ms; j++) {
-      if (!(run < B.selKey[j])) break;
-      run = B.maxOrph[j] > run ? B.maxOrph[j] : run;
-      m++;
+    hit = __any_sync(FULLMASK, hit);
+    if (lane == 0) W.cf = hit ? 1u : 0u;
+  }
+  __syncthreads();
+  // the steps, step j on lane j of every warp: prefix sums of faces, orphans
+  // and new owners and the prefix maximum of the orphans' new keys, over the
+  // leading good steps (what follows the first other one is not used)
+  const BatWalk& Wj = B.u.w[lane < K ? lane : 0];
+  const bool good = lane < K && Wj.ok && !Wj.cf;
+  const uint32_t nn = good ? Wj.n | (Wj.nnew << 16) : 0u, no = good ? Wj.norph : 0u;
+  const unsigned long long sk = B.selKey[lane < K ? lane : 0];
+  uint32_t nnPre = nn, noPre = no, totPre = good ? Wj.tot : 0u;
+  unsigned long long run = good ? Wj.maxOrph : 0ull;
+  auto scan_keys = [&]() {
+#pragma unroll
+    for (int o = 1; o < (int)BatSm<NW>::K; o <<= 1) {
+      const unsigned long long u = __shfl_up_sync(FULLMASK, run, o);
+      const uint32_t c = __shfl_up_sync(FULLMASK, totPre, o);
+      if (lane >= (uint32_t)o) {
+        totPre += c;
+        run = u > run ? u : run;
+      }
+    }
+  };
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t a = __shfl_up_sync(FULLMASK, nnPre, o), b = __shfl_up_sync(FULLMASK, noPre, o);
+    if (lane >= (uint32_t)o) {
+      nnPre += a;
+      noPre += b;
     }
   }
-  // commit: the twins link to the new faces, the patches die
+  const bool large = good && no > 32;
+  const unsigned anyLarge = __ballot_sync(FULLMASK, large);
+  if (anyLarge == 0) scan_keys();
+  nnPre -= nn;
+  const uint32_t nfc = nf0 + (nnPre >> 16), nalc = nal0 + (nnPre >> 16) - (nnPre & 0xffffu);
+  const bool room = lane == 0 || (nfc + 3 * HULL_VIS_MAX <= h.fmax && nfc <= 2 * nalc + 512);
+  const unsigned okm = __ballot_sync(FULLMASK, good && room && nfc + 3 * (nn & 0xffffu) <= h.fmax);
+  const uint32_t ms = __ffs(~okm) - 1;
+  if (ms == 0) return 0;
+  if ((uint64_t)bump + __shfl_sync(FULLMASK, noPre, ms - 1) > 2ull * h.nv) {
+    bump = pool_compact<NW>(h, nf0, sm, B);
+    if (warp < ms && lane < W.n) W.seg[lane].x = h.fseg[W.f[lane]].x;
+    __syncthreads();
+  }
+  // the large orphan sets: owners and ranks of the block's orphan t in h.hA
+  // and h.hB (nv words each)
+  uint32_t TB = 0;
+  if (anyLarge) {
+    const uint32_t c = large && lane < ms ? no : 0u;
+    const uint32_t ci = warp_incl_u(c, (int)lane);
+    TB = __shfl_sync(FULLMASK, ci, 31);
+    if (lane <= ms) B.base[lane] = ci - c;  // the same values from every warp
+    __syncwarp();
+    for (uint32_t t = lid; t < TB; t += G) {
+      uint32_t j = 0, hi = ms;
+      while (hi - j > 1) {
+        const uint32_t mid = (j + hi) >> 1;
+        if (B.base[mid] <= t) j = mid;
+        else hi = mid;
+      }
+      BatWalk& X = B.u.w[j];
+      const uint32_t i = pool[orphan_at(X, t - B.base[j])];
+      uint32_t q = CUACD_NONE, r = 0;
+      if (i != X.pick) {
+        float nd;
+        bat_best(h, X, h.qvert(i), i, 0, 1, q, nd);
+        if (q != CUACD_NONE) {
+          r = atomicAdd(X.cnt + q, 1u);
+          atomicMax(X.fk + q, cand_key(nd, i));
+        }
+      }
+      h.hA[t] = q;
+      h.hB[t] = r;
+    }
+    __syncthreads();
+    if (warp < ms && W.norph > 32) bat_sums(W);
+    __syncthreads();
+    totPre = lane < ms ? Wj.tot : 0u;
+    run = lane < ms ? Wj.maxOrph : 0ull;
+    scan_keys();
+  }
+  // pick j is next while every earlier step's orphans stay below its key
+  const unsigned long long before = __shfl_up_sync(FULLMASK, run, 1);
+  const uint32_t m = __ffs(~__ballot_sync(FULLMASK, lane == 0 || (lane < ms && before < sk))) - 1;
+  const uint32_t at = bump + __shfl_up_sync(FULLMASK, totPre, 1);
+  if (lane <= ms) B.place[lane] = lane ? at : bump;  // the same values from every warp
+  __syncwarp();
+  const uint32_t first = __shfl_sync(FULLMASK, nfc, warp);  // warp < m: its first new slot
+  const uint32_t nfEnd = __shfl_sync(FULLMASK, nfc, m), nalEnd = __shfl_sync(FULLMASK, nalc, m);
+  const uint32_t gone = __shfl_sync(FULLMASK, noPre, m - 1);
+  // commit: new faces with their links, keys and segments, the twins' links,
+  // the dead faces, the orphans in their places
   if (warp < m) {
-    const BatWalk& W = B.u.w[warp];
-    const uint32_t base = B.nfj[warp];
-    for (uint32_t q = lane; q < W.nnew; q += 32) {
-      const uint32_t twin = W.tw[q], f = W.df[q], s = base + q;
+    const uint32_t at = B.place[warp];
+    if (lane < W.nnew) {
+      const uint32_t s = first + lane, twin = W.tw[lane];
+      uint4* w = h.rec(s);
+      w[0] = W.rec[lane][0]; w[1] = W.rec[lane][1]; w[2] = W.rec[lane][2]; w[3] = W.rec[lane][3];
+      *reinterpret_cast<uint4*>(h.nbr + 4 * (size_t)s) = make_uint4(twin, first + j1, first + j2, 0u);
+      h.fkey[s] = W.fk[lane];
+      h.fseg[s] = make_uint2(at + W.pre[lane], W.cnt[lane]);
       if (twin < nf0) {
         uint32_t* tq = h.nbr + 4 * (size_t)twin;
-        const uint4 tn = *reinterpret_cast<const uint4*>(tq);
-        if (tn.x == f) tq[0] = s;
-        if (tn.y == f) tq[1] = s;
-        if (tn.z == f) tq[2] = s;
+        if (tslot & 1u) tq[0] = s;
+        if (tslot & 2u) tq[1] = s;
+        if (tslot & 4u) tq[2] = s;
       }
     }
-    for (uint32_t i = lane; i < W.n; i += 32) h.F[16 * (size_t)W.f[i]] &= 0x7fffffffu;
+    if (lane < W.n) {
+      const uint32_t f = W.f[lane];
+      h.F[16 * (size_t)f] &= 0x7fffffffu;
+      h.fkey[f] = 0;
+      h.fseg[f] = make_uint2(0, 0);
+    }
+    if (oq != CUACD_NONE) pool[at + W.pre[oq] + orank] = oi;
+  }
+  for (uint32_t t = lid; t < TB; t += G) {
+    const uint32_t q = h.hA[t];
+    if (q == CUACD_NONE) continue;
+    uint32_t j = 0, hi = ms;
+    while (hi - j > 1) {
+      const uint32_t mid = (j + hi) >> 1;
+      if (B.base[mid] <= t) j = mid;
+      else hi = mid;
+    }
+    if (j >= m) continue;
+    const BatWalk& X = B.u.w[j];
+    pool[B.place[j] + X.pre[q] + h.hB[t]] = pool[orphan_at(X, t - B.base[j])];
   }
   if (lid == 0) {
+    const uint32_t end = B.place[m];
     hs.newBase = nf0;
-    hs.nf = B.nfj[m];
-    hs.nalive = B.nalj[m];
+    hs.nf = nfEnd;
+    hs.nalive = nalEnd;
+    B.bump = end;
+    B.live = B.live - gone + (end - bump);
   }
-  if (nt <= TODO_CAP) {
-    // accepted steps' orphans take their new owners (the picks leave);
-    // the others keep theirs
-    for (uint32_t t = lid; t < nt; t += G) {
-      const uint32_t k = tK[t], i = tI[t], j = tJ[t];
-      if (j < m) {
-        const uint32_t no = tNO[t];
-        const float nd = __uint_as_float(tND[t]);
-        h.owner[k] = no;
-        h.dist[k] = nd;
-        if (no == CUACD_NONE) dead++;
-        else top.add(cand_key(nd, i), k, no);
-      } else {
-        top.add(cand_key(h.dist[k], i), k, tO[t]);
-      }
-    }
-  } else {
-    // more orphans than the list holds: the first step alone, its orphans
-    // reassigned by a sweep
-    for (uint32_t k = lid; k < ncand; k += G) {
-      const uint32_t own = h.owner[k];
-      if (own == CUACD_NONE) continue;
-      const uint32_t j = __ffs(btab_mask(B, own)) - 1u;
-      if (j >= ms) continue;
-      const uint32_t i = h.cand[k];
-      if (j != 0) {
-        top.add(cand_key(h.dist[k], i), k, own);
-        continue;
-      }
-      uint32_t no = CUACD_NONE;
-      float nd = 0.0f;
-      if (k != B.selSlot[0]) bat_best<NRC>(h, i, B.nfj[0], B.nfj[1], B.nrc[0], no, nd);
-      h.owner[k] = no;
-      h.dist[k] = nd;
-      if (no == CUACD_NONE) dead++;
-      else top.add(cand_key(nd, i), k, no);
-    }
-  }
-  top2_publish(B, top, dead);
   __syncthreads();
   return m;
 }
@@ -1828,67 +1925,84 @@ __device__ __noinline__ uint32_t hull_grow_big(const HullCtx& h, HullSm& hs, Grp
                                                uint32_t maxIter) {
   constexpr int G = 32 * NW;
   const uint32_t lid = threadIdx.x, warp = lid >> 5;
-  uint32_t ncand = hs.ncand;
-  // owner and distance to candidate-slot order, in place: each chunk is read
-  // before it is written, and a later chunk reads only points cand[k] >= k
-  // (the assignment pass lists points in index order; the seed list fits
-  // one chunk)
-  Top2 top;
-  top.clear();
-  uint32_t dead = 0;
-  for (uint32_t c = 0; c * G < ncand; c++) {
-    const uint32_t k = c * G + lid;
-    uint32_t o = CUACD_NONE, i = 0;
-    float d = 0.0f;
-    if (k < ncand) {
-      i = h.cand[k];
-      o = h.owner[i];
-      d = h.dist[i];
-    }
-    __syncthreads();
-    if (k < ncand) {
-      h.owner[k] = o;
-      h.dist[k] = d;
-      if (o != CUACD_NONE) top.add(cand_key(d, i), k, o);
-      else dead++;
-    }
-    __syncthreads();
-  }
-  top2_publish(B, top, dead);
-  __syncthreads();
+  pool_build<NW, false>(h, hs.nf, sm, B, hs.ncand);
   uint32_t nIns = 0;
+  // A round's picks are the largest keys of the faces whose distance reaches
+  // tau (float bits), listed by one compare per face and placed by their
+  // rank in the list. tau follows the list's length, towards two to three
+  // times the picks; when no face reaches it (or more than the list holds)
+  // the picks come from the threads' two largest keys instead, which also
+  // finds that no candidate is left. The two give the same picks in the same
+  // order, at most a different number of them.
+  uint32_t tau = 0;
+  if (lid == 0) B.nlist = 0;
+  __syncthreads();
   while (nIns < maxIter) {
+    const uint32_t nf = hs.nf, kmax = min(BatSm<NW>::K, maxIter - nIns);
+    if (tau != 0) {
+      for (uint32_t f0 = lid; f0 < nf; f0 += 8 * G) {  // eight loads in flight
+        unsigned long long k[8];
+#pragma unroll
+        for (int u = 0; u < 8; u++) k[u] = f0 + u * G < nf ? h.fkey[f0 + u * G] : 0ull;
+#pragma unroll
+        for (int u = 0; u < 8; u++) {
+          if ((uint32_t)(k[u] >> 32) >= tau) {
+            const uint32_t at = atomicAdd(&B.nlist, 1u);
+            if (at < BAT_CAND) {
+              B.lk[at] = k[u];
+              B.lf[at] = f0 + u * G;
+            }
+          }
+        }
+      }
+    }
     for (uint32_t e = lid; e < (1u << BatSm<NW>::BLK_BITS); e += G) B.btab[e] = make_uint2(0u, 0u);
-    if (warp == 0) bat_select(B, min(BatDims<NW>::KMAX, maxIter - nIns));
+    if (lid == 0) B.nsel = 0;
     __syncthreads();
-    // squeeze dead slots out when they pass 1 / SQZ_DIV of the list
-    if (SQZ_DIV * B.totDead > ncand) {
-      ncand = big_squeeze(h, sm, B, ncand);
-      continue;
-    }
-    const uint32_t K = B.nsel;
-    if (K == 0) break;
-    uint32_t ms = 0, myBase = 0;
-    if (hs.nf + 3 * HULL_VIS_MAX <= h.fmax && hs.nf <= 2 * hs.nalive + 512) {
-      if (warp < K) bat_walk(h, hs.nf, B, 0xffffffffu - (uint32_t)(B.selKey[warp] & 0xffffffffu), B.selOwn[warp]);
+    const uint32_t nl = B.nlist;
+    uint32_t K;
+    if (nl != 0 && nl <= BAT_CAND) {
+      K = min(nl, kmax);
+      if (lid < BAT_CAND) {
+        const unsigned long long k = lid < nl ? B.lk[lid] : 0ull;
+        uint32_t rank = 0;
+        for (uint32_t j = 0; j < nl; j++) rank += B.lk[j] > k ? 1u : 0u;
+        if (lid < nl && rank < kmax) {
+          B.selKey[rank] = k;
+          B.selF[rank] = B.lf[lid];
+        }
+      }
       __syncthreads();
-      bat_conflicts(B, K);
+      const float t = __uint_as_float(tau);
+      const float by = nl <= kmax ? 0.85f : (2 * nl <= 3 * kmax ? 0.95f : (nl <= 2 * kmax ? 0.98f : (nl <= 3 * kmax ? 1.0f : 1.05f)));
+      tau = __float_as_uint(t * by);
+    } else {
+      Top2 top;
+      top.clear();
+      for (uint32_t f = lid; f < nf; f += G) top.add(h.fkey[f], f);
+      top2_publish(B, top);
       __syncthreads();
-      // the same on every thread; the slot pass reads the block's set of
-      // claimed faces, which no thread writes until the next round
-      ms = bat_prefix(h, hs, B, K, &myBase);
+      bat_select(B, kmax);
+      __syncthreads();
+      K = B.nsel;
+      if (K == 0) break;
+      tau = __float_as_uint(__uint_as_float((uint32_t)(B.selKey[K - 1] >> 32)) * 0.9f);
     }
-    if (ms == 0) {
+    if (lid == 0) B.nlist = 0;
+    uint32_t done = 0;
+    if (nf + 3 * HULL_VIS_MAX <= h.fmax && nf <= 2 * hs.nalive + 512) done = bat_round(h, hs, sm, B, K);
+    if (done == 0) {
       // the single-pick step's shared words overlay the walks' words
       __syncthreads();
-      big_seq_step(h, hs, sm, B, ncand);
-      nIns++;
-      if (hs.fail) break;
-    } else {
-      nIns += bat_step(h, hs, B, ncand, ms, myBase);
+      big_seq_step(h, hs, sm, B);
+      done = 1;
+      if (hs.fail) {
+        nIns++;
+        break;
+      }
     }
+    nIns += done;
   }
-  if (lid == 0) hs.ncand = ncand;
   __syncthreads();
   return nIns;
 }
@@ -1937,6 +2051,91 @@ __device__ __noinline__ uint32_t hull_assign_all(const HullCtx& h, GrpSmem& sm, 
     }
 #pragma unroll
     for (int k = 0; k < ASSIGN_K; k++) {
+      if (base + k * G < nv) {
+        const uint32_t i = base + k * G + lid;
+        const bool outside = i < nv && bo[k] != CUACD_NONE;
+        if (i < nv) {
+          h.owner[i] = bo[k];
+          h.dist[i] = bd[k];
+        }
+        uint32_t tot;
+        const uint32_t pre = grp_scan_bit<G>(outside, &tot, sm);
+        if (outside) h.cand[ncand + pre] = i;
+        ncand += tot;
+      }
+    }
+  }
+  return ncand;
+}
+
+// hull_assign_all for a block: the alive faces' records (at most ASSIGN_FACES
+// after the seeds: 4 + 2 for each of up to 80) in shared memory in slot
+// order, four points per thread. Almost every point lies behind almost
+// every face, so a face costs one determinant and its bound; the ranking
+// value (a division) is formed only for a point beyond the bound, and the
+// exact sign only while a point has no owner, as in best_face. Reading the
+// records of every slot, dead ones included, for each 2 points took 15 % of
+// a 30k-point hull.
+#define ASSIGN_FACES 176u
+struct AssignSm {
+  uint4 w0[ASSIGN_FACES], w1[ASSIGN_FACES], w2[ASSIGN_FACES];  // w2.w: the face's slot
+};
+template <int NW>
+__device__ __noinline__ uint32_t hull_assign_block(const HullCtx& h, GrpSmem& sm, AssignSm& A, uint32_t nf) {
+  constexpr int G = 32 * NW, PTS = 4;
+  const uint32_t lid = threadIdx.x, nv = h.nv;
+  uint32_t n = 0;
+  for (uint32_t c = 0; c * G < nf; c++) {
+    const uint32_t f = c * G + lid;
+    const uint4 w0 = f < nf ? h.rec(f)[0] : make_uint4(0, 0, 0, 0);
+    const bool al = (w0.x & ALIVE) != 0;
+    uint32_t tot;
+    const uint32_t at = n + grp_scan_bit<G>(al, &tot, sm);
+    if (al && at < ASSIGN_FACES) {
+      uint4 w2 = h.rec(f)[2];
+      w2.w = f;
+      A.w0[at] = w0;
+      A.w1[at] = h.rec(f)[1];
+      A.w2[at] = w2;
+    }
+    n += tot;
+  }
+  __syncthreads();
+  uint32_t ncand = 0;
+  for (uint32_t base = 0; base < nv; base += PTS * G) {
+    f3 p[PTS];
+    float bd[PTS];
+    uint32_t bo[PTS];
+#pragma unroll
+    for (int k = 0; k < PTS; k++) {
+      const uint32_t i = base + k * G + lid;
+      p[k] = h.qvert(i < nv ? i : 0u);
+      bd[k] = 0.0f;
+      bo[k] = CUACD_NONE;
+    }
+    for (uint32_t j = 0; j < n; j++) {
+      const uint4 w0 = A.w0[j], w1 = A.w1[j], w2 = A.w2[j];
+      const f3 nn = mk3(__uint_as_float(w1.x), __uint_as_float(w1.y), __uint_as_float(w1.z));
+      const f3 pa = mk3(__uint_as_float(w2.x), __uint_as_float(w2.y), __uint_as_float(w2.z));
+      const float kb = __uint_as_float(w0.w);
+#pragma unroll
+      for (int k = 0; k < PTS; k++) {
+        const f3 d = p[k] - pa;
+        const float det = dot(nn, d), bound = kb * l1(d);
+        if (det < -bound) continue;
+        const uint32_t i = base + k * G + lid;
+        if (det > bound) {
+          const float dd = det / __uint_as_float(w1.w);
+          if (dd > bd[k]) { bd[k] = dd; bo[k] = w2.w; }
+        } else if (bo[k] == CUACD_NONE && (w0.x & 0x7fffffffu) != i && w0.y != i && w0.z != i &&
+                   h.face_exact(h.rec(w2.w)[2], h.rec(w2.w)[3], p[k])) {
+          bd[k] = 1e-30f;
+          bo[k] = w2.w;
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < PTS; k++) {
       if (base + k * G < nv) {
         const uint32_t i = base + k * G + lid;
         const bool outside = i < nv && bo[k] != CUACD_NONE;
@@ -2003,9 +2202,82 @@ __device__ __noinline__ double hull_volume_grid(const HullCtx& h, HullSm& hs, Gr
   return ((double)th * 4294967296.0 + (double)tl) / 6.0;
 }
 
+// The 80 seeds of a block's part: eight axes at a time, so a point is read
+// five times and not twenty, each thread's extremes folded per warp with
+// redux (value, then lowest index) and the warps' by one thread per seed
+// behind a single barrier. Four block-wide reductions per two axes took 9 %
+// of a 3k-point hull.
+template <int NW>
+struct KdopSm {
+  int v[NW][80];       // ordered value: the maximum along an axis, and the negated minimum
+  uint32_t i[NW][80];  // its point, the lowest index on ties
+};
+template <int NW>
+__device__ __noinline__ void kdop_block(const HullCtx& h, HullSm& hs, KdopSm<NW>& K) {
+  constexpr int G = 32 * NW;
+  const uint32_t lid = threadIdx.x, warp = lid >> 5, lane = lid & 31;
+#pragma unroll
+  for (int a0 = 0; a0 < 40; a0 += 8) {
+    float mx[8], mn[8];
+    uint32_t ix[8], in[8];
+#pragma unroll
+    for (int a = 0; a < 8; a++) {
+      mx[a] = -1e30f;
+      mn[a] = 1e30f;
+      ix[a] = in[a] = 0;
+    }
+    for (uint32_t i = lid; i < h.nv; i += G) {
+      const f3 v = h.qvert(i);
+#pragma unroll
+      for (int a = 0; a < 8; a++) {
+        const float d = dot(mk3(c_kdop[a0 + a][0], c_kdop[a0 + a][1], c_kdop[a0 + a][2]), v);
+        if (d > mx[a]) { mx[a] = d; ix[a] = i; }
+        if (d < mn[a]) { mn[a] = d; in[a] = i; }
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < 16; a++) {
+      // -0 and 0 are the same value: adding 0 makes them the same bits
+      const int k = f_ord((a & 1 ? -mn[a >> 1] : mx[a >> 1]) + 0.0f);
+      const int best = __reduce_max_sync(FULLMASK, k);
+      const uint32_t i = __reduce_min_sync(FULLMASK, k == best ? (a & 1 ? in[a >> 1] : ix[a >> 1]) : 0xffffffffu);
+      if (lane == 0) {
+        K.v[warp][2 * a0 + a] = best;
+        K.i[warp][2 * a0 + a] = i;
+      }
+    }
+  }
+  __syncthreads();
+  if (lid < 80) {
+    int best = K.v[0][lid];
+    uint32_t i = K.i[0][lid];
+    for (int w = 1; w < NW; w++) {
+      const int k = K.v[w][lid];
+      const uint32_t j = K.i[w][lid];
+      if (k > best || (k == best && j < i)) { best = k; i = j; }
+    }
+    hs.seed[lid] = i;
+  }
+}
+
+// A part for the blocks: the warp hulls run first and list the parts above
+// smallNv points and, of the parts of at least P.handOn points (0: none),
+// those that the register hull cannot hold (more than QC_MAX points or
+// TINY_SEEDS distinct seeds, more than 32 candidates or faces). Such a part's
+// hull has many faces, and a block inserts several points a round where the
+// warp's slot-array form inserts one: 152 parts of 150 points in convex
+// position take 1.10 ms on warps and 0.45 ms on blocks, 512 pair unions of
+// 40-1,000 points 2.4-6.5 ms and 1.2 ms; staircase children of 80 points, few
+// of them on the hull, are 4 times slower on blocks, so a point count alone
+// cannot tell them apart.
+__device__ __forceinline__ void hand_on(const Level& P, const Dev& D, uint32_t idx) {
+  D.list[atomicAdd(D.work + 48 + P.workSlot, 1u)] = idx;
+}
+
+// false (warp groups): the part was handed on
 template <int G>
-__device__ void hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* slab, HullSm& hs, GrpSmem& sm,
-                         float* qcache, TinySm* ts, BatSm<(G >= 256 ? G / 32 : 8)>* bs) {
+__device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* slab, HullSm& hs, GrpSmem& sm,
+                         float4* qcache, TinySm* ts, BatSm<(G >= 256 ? G / 32 : 8)>* bs) {
   const int lid = Grp<G>::lid();
   const uint32_t partIdx = P.partBase + idx;
   PartDesc* pdp = D.parts + partIdx;
@@ -2013,19 +2285,19 @@ __device__ void hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   const float meshVol = pdp->meshVol;
   if (!(nv >= 4 && (nt > 0 || (flags & 2) != 0))) {
     if (lid == 0) pdp->hullVol = 0.0f;
-    return;
+    return true;
   }
   const uint32_t fb = (2 * nv + max(nv, 80u) + 7) & ~7u;
   const uint32_t fmax = P.hullSlabWords > fb ? (P.hullSlabWords - fb) / 16 : 0;
   if (fmax < 64) {
     if (lid == 0) { pdp->hullVol = -1.0f; pdp->flags = 3; atomicAdd(D.ctr + CTR_HULLFAIL, 1u); }
-    return;
+    return true;
   }
   // the walk's arrays after the reference's slab words must fit the slab
   // (always true for hull_slab_stride; checked so a slab is never overrun)
-  if ((uint64_t)P.hullSlabWords + 2 * HULL_VIS_MAX + 4ull * fmax + 2 * ((fmax + 31) / 32) + 2ull * nv > P.slabStride) {
+  if ((uint64_t)P.hullSlabWords + 2 * HULL_VIS_MAX + 8ull * fmax + 2 * ((fmax + 31) / 32) + 2ull * nv > P.slabStride) {
     if (lid == 0) { pdp->hullVol = -1.0f; pdp->flags = 3; atomicAdd(D.ctr + CTR_HULLFAIL, 1u); }
-    return;
+    return true;
   }
   if (lid == 0) add_bytes(D.ctr, CTR_BYTES_HULL, 12ull * nv);
   HullCtx h;
@@ -2036,12 +2308,15 @@ __device__ void hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   h.cand = slab + 2 * nv;
   h.F = slab + fb;
   // after the reference's slab words (which fix fmax): visible list, walk
-  // queue, adjacency, bitmap, word prefix, horizon maps (hull_slab_stride)
+  // queue, adjacency, the faces' keys and segments, bitmap, word prefix,
+  // horizon maps (hull_slab_stride)
   h.vis = slab + P.hullSlabWords;
   h.q = h.vis + HULL_VIS_MAX;
   h.nbr = h.q + HULL_VIS_MAX;
   const uint32_t nw = (fmax + 31) / 32;
-  h.bm = h.nbr + 4 * (size_t)fmax;
+  h.fkey = reinterpret_cast<unsigned long long*>(h.nbr + 4 * (size_t)fmax);
+  h.fseg = reinterpret_cast<uint2*>(h.fkey + fmax);
+  h.bm = h.nbr + 8 * (size_t)fmax;
   h.wp = h.bm + nw;
   h.hA = h.wp + nw;
   h.hB = h.hA + nv;
@@ -2065,16 +2340,29 @@ __device__ void hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   if (G == 32 && qcache != nullptr && nv <= QC_MAX) {
     for (uint32_t i = lid; i < nv; i += G) {
       f3 v = ldv(D.V, (size_t)vOff + 3 * (size_t)i) - lo;
-      qcache[3 * i] = rintf(v.x * h.qs);
-      qcache[3 * i + 1] = rintf(v.y * h.qs);
-      qcache[3 * i + 2] = rintf(v.z * h.qs);
+      qcache[i] = make_float4(rintf(v.x * h.qs), rintf(v.y * h.qs), rintf(v.z * h.qs), 0.0f);
     }
     h.qc = qcache;
     Grp<G>::sync();
   }
+  if constexpr (G >= 256) {
+    // the block path keeps them in the slab where its words hold them too
+    // (always when the hull bound covers the part): one 16-byte load instead
+    // of three and the rounding, in every pass and every new face
+    const uint64_t at = ((uint64_t)(h.hB - slab) + nv + 3) & ~3ull;
+    if (at + 4ull * nv <= P.slabStride) {
+      float4* qp = reinterpret_cast<float4*>(slab + at);
+      for (uint32_t i = lid; i < nv; i += G) {
+        const f3 v = h.qvert(i);
+        qp[i] = make_float4(v.x, v.y, v.z, 0.0f);
+      }
+      h.qc = qp;
+      Grp<G>::sync();
+    }
+  }
   // 80 seeds: max and min along 40 axes, lowest index on ties; seed 2a is
   // the maximum along axis a, seed 2a + 1 the minimum
-  if (h.qc != nullptr) {
+  if (G == 32 && h.qc != nullptr) {
     // one lane per axis, each scanning every point in index order
     for (uint32_t a = lid; a < 40; a += G) {
       const f3 ax = mk3(c_kdop[a][0], c_kdop[a][1], c_kdop[a][2]);
@@ -2088,35 +2376,40 @@ __device__ void hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
       hs.seed[2 * a] = ix;
       hs.seed[2 * a + 1] = in;
     }
-  } else
-  for (int ps = 0; ps < 20; ps++) {
-    const f3 a0 = mk3(c_kdop[2 * ps][0], c_kdop[2 * ps][1], c_kdop[2 * ps][2]);
-    const f3 a1 = mk3(c_kdop[2 * ps + 1][0], c_kdop[2 * ps + 1][1], c_kdop[2 * ps + 1][2]);
-    float mx0 = -1e30f, mx1 = -1e30f, mn0 = -1e30f, mn1 = -1e30f;  // mins stored negated
-    uint32_t ix0 = CUACD_NONE, ix1 = CUACD_NONE, in0 = CUACD_NONE, in1 = CUACD_NONE;
-    for (uint32_t i = lid; i < nv; i += G) {
-      f3 v = h.qvert(i);
-      float d0 = dot(a0, v), d1 = dot(a1, v);
-      am_merge(mx0, ix0, d0, i);
-      am_merge(mn0, in0, -d0, i);
-      am_merge(mx1, ix1, d1, i);
-      am_merge(mn1, in1, -d1, i);
+  } else if constexpr (G >= 256) {
+    static_assert(sizeof(KdopSm<G / 32>) <= sizeof(*bs), "the seeds' words overlay the rounds' words");
+    kdop_block<G / 32>(h, hs, *reinterpret_cast<KdopSm<G / 32>*>(bs));
+  } else {
+    for (int ps = 0; ps < 20; ps++) {
+      const f3 a0 = mk3(c_kdop[2 * ps][0], c_kdop[2 * ps][1], c_kdop[2 * ps][2]);
+      const f3 a1 = mk3(c_kdop[2 * ps + 1][0], c_kdop[2 * ps + 1][1], c_kdop[2 * ps + 1][2]);
+      float mx0 = -1e30f, mx1 = -1e30f, mn0 = -1e30f, mn1 = -1e30f;  // mins stored negated
+      uint32_t ix0 = CUACD_NONE, ix1 = CUACD_NONE, in0 = CUACD_NONE, in1 = CUACD_NONE;
+      for (uint32_t i = lid; i < nv; i += G) {
+        f3 v = h.qvert(i);
+        float d0 = dot(a0, v), d1 = dot(a1, v);
+        am_merge(mx0, ix0, d0, i);
+        am_merge(mn0, in0, -d0, i);
+        am_merge(mx1, ix1, d1, i);
+        am_merge(mn1, in1, -d1, i);
+      }
+      grp_argmax<G>(mx0, ix0, sm);
+      grp_argmax<G>(mn0, in0, sm);
+      grp_argmax<G>(mx1, ix1, sm);
+      grp_argmax<G>(mn1, in1, sm);
+      if (lid == 0) { hs.seed[4 * ps] = ix0; hs.seed[4 * ps + 1] = in0; hs.seed[4 * ps + 2] = ix1; hs.seed[4 * ps + 3] = in1; }
     }
-    grp_argmax<G>(mx0, ix0, sm);
-    grp_argmax<G>(mn0, in0, sm);
-    grp_argmax<G>(mx1, ix1, sm);
-    grp_argmax<G>(mn1, in1, sm);
-    if (lid == 0) { hs.seed[4 * ps] = ix0; hs.seed[4 * ps + 1] = in0; hs.seed[4 * ps + 2] = ix1; hs.seed[4 * ps + 3] = in1; }
   }
   Grp<G>::sync();
   if (P.hullStage == 1) {
     if (lid == 0) pdp->hullVol = 0.0f;
-    return;
+    return true;
   }
   // the register hull first when the part's points are in shared memory; a
   // hull that outgrows the warp is built again from the simplex in the
   // slot-array form (the same sequence, so the same result)
   bool tiny = G == 32 && ts != nullptr && h.qc != nullptr;
+  if (G == 32 && P.handOn && !tiny) return false;
 restart:
   // initial simplex (shaders.ts:1227-1263). The reference scans the 80 seeds
   // serially with strict comparisons, so each choice is the first seed
@@ -2175,7 +2468,7 @@ restart:
   Grp<G>::sync();
   if (!hs.ok) {
     if (lid == 0) pdp->hullVol = 0.0f;
-    return;
+    return true;
   }
   // seeds first. A point can be the extreme of several axes; its repeats in
   // the list have the same distance and index, so they never change a pick
@@ -2198,12 +2491,14 @@ restart:
   Grp<G>::sync();
   uint32_t nIns;
   bool tinyUsed = false;
+  if (G == 32 && P.handOn && nv >= P.handOn && nuniq > TINY_SEEDS) return false;
   if (tiny && nuniq <= TINY_SEEDS) {
     const uint32_t ci = (uint32_t)lid < nuniq ? h.cand[lid] : 0u;
     if (lid == 0) hs.nfRef = 4;
     __syncwarp();
     nIns = hull_tiny_grow(h, hs, *ts, 80, ci, CUACD_NONE, 0.0f, nuniq);
     if (nIns == CUACD_NONE) {
+      if (P.handOn && nv >= P.handOn) return false;
       tiny = false;
       goto restart;
     }
@@ -2253,11 +2548,21 @@ restart:
         pdp->flags = pdp->flags | 4u;
         atomicAdd(D.ctr + CTR_PRUNED, 1u);
       }
-      return;
+      return true;
     }
   }
   // every point against the rough hull; candidates = points outside it
-  const uint32_t ncand = fail0 == 0 ? hull_assign_all<G>(h, sm, nfPrev) : 0u;
+  uint32_t ncand = 0;
+  if (fail0 == 0) {
+    if constexpr (G >= 256) {
+      static_assert(sizeof(AssignSm) <= sizeof(*bs), "the assignment's records overlay the rounds' words");
+      if (hs.nalive <= ASSIGN_FACES)
+        ncand = hull_assign_block<G / 32>(h, sm, *reinterpret_cast<AssignSm*>(bs), nfPrev);
+      else ncand = hull_assign_all<G>(h, sm, nfPrev);
+    } else {
+      ncand = hull_assign_all<G>(h, sm, nfPrev);
+    }
+  }
   if (lid == 0) {
     hs.ncand = ncand;
     if (P.exportStride == 0) pdp->pad0 = ncand;
@@ -2266,6 +2571,7 @@ restart:
   const uint32_t maxIter = (P.hullStage == 2 || P.hullStage == 3 || fail0 != 0) ? 0 : nv;
   if (tinyUsed && fail0 == 0) {
     if (ncand > 32) {
+      if (P.handOn && nv >= P.handOn) return false;
       tiny = false;
       goto restart;
     }
@@ -2278,6 +2584,7 @@ restart:
     }
     const uint32_t n2 = hull_tiny_grow(h, hs, *ts, maxIter, ci, co, cd, 0u);
     if (n2 == CUACD_NONE) {
+      if (P.handOn && nv >= P.handOn) return false;
       tiny = false;
       goto restart;
     }
@@ -2301,7 +2608,7 @@ restart:
       pdp->flags = hs.fail;
       atomicAdd(D.ctr + CTR_HULLFAIL, 1u);
     }
-    return;
+    return true;
   }
   const float vol = (float)(hull_volume_grid<G>(h, hs, sm) * (double)volScale);
   if (lid == 0) { pdp->hullVol = vol; pdp->pad1 = nIns; }
@@ -2334,20 +2641,21 @@ restart:
       }
     }
   }
+  return true;
 }
 
 // Persistent groups: group s owns slab s and takes the launch's parts from a
-// counter, so parts of uneven size balance across the GPU. Warps take parts
-// with nv <= smallNv, blocks of 256, 512 or 1024 threads the others (the
-// widest whose resident blocks hold the level's parts in one wave): the
+// counter, so parts of uneven size balance across the GPU. Warps take every
+// part first and list the ones for the blocks of 256, 512 or 1024 threads
+// (the widest whose resident blocks hold the level's parts in one wave): a
 // block inserts up to one point per warp (at most 16) per round, and its
-// width serves the passes over all points and candidates, which grow with nv.
+// width serves the passes over all points, which grow with nv.
 template <int G>
 __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 ? 2 : 4))
     k_hull(const Level P, const Dev D) {
   __shared__ GrpSmem gsm[Grp<G>::PER_BLOCK];
   __shared__ HullSm hsm[Grp<G>::PER_BLOCK];
-  __shared__ float qcs[G == 32 ? 8 * 3 * QC_MAX : 1];
+  __shared__ float4 qcs[G == 32 ? 8 * QC_MAX : 1];
   __shared__ TinySm tsm[G == 32 ? 8 : 1];
   // the block path's shared words (BatSm) in the launch's dynamic shared memory
   extern __shared__ __align__(16) unsigned char hull_dyn[];
@@ -2355,21 +2663,17 @@ __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 
   const int gi = Grp<G>::gid();
   const uint32_t s = blockIdx.x * Grp<G>::PER_BLOCK + gi;
   if (s >= P.nSlabs) return;
-  if (G != 32) {
-    // leave at once when the level has no part above smallNv (the scan
-    // recorded its largest child)
-    const uint32_t mx = P.maxNvHint ? P.maxNvHint : D.work[32 + P.workSlot];
-    if (mx <= P.smallNv) return;
-  }
   uint32_t* slab = D.slab + (size_t)s * P.slabStride;
   if (G != 32) {
+    // the parts that the level's warp hulls listed
+    const uint32_t n = D.work[48 + P.workSlot];
+    if (blockIdx.x >= n) return;
     for (;;) {
-      uint32_t idx = 0;
-      if (threadIdx.x == 0) idx = atomicAdd(D.work + 16 + P.workSlot, 1u);
-      idx = grp_bcast_u<G>(idx, gsm[0]);
-      if (idx >= P.nChildParts) break;
-      if (D.parts[P.partBase + idx].nv <= P.smallNv) continue;
-      hull_one<G>(P, D, idx, slab, hsm[gi], gsm[gi], nullptr, nullptr, reinterpret_cast<BS*>(hull_dyn));
+      uint32_t k = 0;
+      if (threadIdx.x == 0) k = atomicAdd(D.work + 16 + P.workSlot, 1u);
+      k = grp_bcast_u<G>(k, gsm[0]);
+      if (k >= n) break;
+      hull_one<G>(P, D, D.list[k], slab, hsm[gi], gsm[gi], nullptr, nullptr, reinterpret_cast<BS*>(hull_dyn));
       Grp<G>::sync();
     }
     return;
@@ -2383,8 +2687,13 @@ __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 
       if (lane == 0) idx = atomicAdd(D.work + P.workSlot, 1u);
       idx = __shfl_sync(FULLMASK, idx, 0);
       if (idx >= P.nChildParts) break;
-      if (D.parts[P.partBase + idx].nv > P.smallNv) continue;
-      hull_one<G>(P, D, idx, slab, hsm[gi], gsm[gi], qcs + gi * 3 * QC_MAX, tsm + gi, nullptr);
+      const uint32_t nv = D.parts[P.partBase + idx].nv;
+      bool done = nv <= P.smallNv && !(P.handOn && nv > QC_MAX);
+      if (done) {
+        done = hull_one<G>(P, D, idx, slab, hsm[gi], gsm[gi], qcs + gi * QC_MAX, tsm + gi, nullptr);
+        if (!done && lane == 0) add_bytes(D.ctr, CTR_BYTES_HULL, 0ull - 12ull * nv);  // the block counts it
+      }
+      if (!done && lane == 0) hand_on(P, D, idx);
       Grp<G>::sync();
     }
   }
@@ -2445,7 +2754,7 @@ int set_error(int code, const char* msg);
 #define NOALLOC_PART_OFF NOALLOC_SLAB_WORDS
 #define NOALLOC_CTR_OFF (NOALLOC_PART_OFF + 16u)
 #define NOALLOC_WORK_OFF (NOALLOC_CTR_OFF + (uint32_t)CTR_WORDS)
-#define NOALLOC_WORDS (NOALLOC_WORK_OFF + 64u)
+#define NOALLOC_WORDS (NOALLOC_WORK_OFF + 65u)  // the work counters and the one-part list
 
 static __device__ __align__(256) uint32_t g_noalloc_scratch[NOALLOC_WORDS];
 
@@ -2577,7 +2886,7 @@ extern "C" int cuacd_hull_points_noalloc(const float* points, uint32_t nv, uint3
   P.smallNv = 1024;
   P.exportBase = 0;
   P.exportStride = trisCap;
-  P.maxNvHint = maxNv;
+  P.handOn = HAND_ON_BATCH;
   Dev D;
   memset(&D, 0, sizeof(D));
   D.V = const_cast<float*>(points);
@@ -2586,9 +2895,11 @@ extern "C" int cuacd_hull_points_noalloc(const float* points, uint32_t nv, uint3
   D.parts = reinterpret_cast<PartDesc*>(scratch + NOALLOC_PART_OFF);
   D.ctr = scratch + NOALLOC_CTR_OFF;
   D.work = scratch + NOALLOC_WORK_OFF;
+  D.list = scratch + NOALLOC_WORK_OFF + 64;
   k_noalloc_setup<<<1, 64, 0, s>>>(scratch, nv);
-  if (nv <= P.smallNv) k_hull<32><<<1, 256, 0, s>>>(P, D);
-  else k_hull<256><<<1, 256, sizeof(BatSm<8>), s>>>(P, D);
+  static_assert(sizeof(BatSm<8>) <= 46 * 1024, "the block's shared words need no raised limit");
+  k_hull<32><<<1, 256, 0, s>>>(P, D);
+  k_hull<256><<<1, 256, sizeof(BatSm<8>), s>>>(P, D);
   k_noalloc_finish<<<1, 1, 0, s>>>(scratch, volume, ntris, status);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(-4, cudaGetErrorString(e));

@@ -295,7 +295,6 @@ __global__ void __launch_bounds__(1024) k_scan(const Level P, const Dev D) {
     __syncthreads();
   }
   const bool keepTopo = P.lastLevel == 0;
-  uint32_t childMax = 0;
   {
     const uint32_t c = blockIdx.x;
     const uint32_t j = c * 1024 + tid;
@@ -369,7 +368,6 @@ __global__ void __launch_bounds__(1024) k_scan(const Level P, const Dev D) {
         neg.nt = keepTopo ? cnt[4] : 0; neg.eOff = keepTopo ? eOff + cnt[2] : eOff; neg.ne = keepTopo ? cnt[5] : 0;
         D.parts[posP] = pos;
         D.parts[negP] = neg;
-        childMax = max(cnt[0], cnt[3]);
         const bool bothNonEmpty = cnt[0] > 0 && cnt[1] > 0 && cnt[3] > 0 && cnt[4] > 0;
         it = parent;
         if (parent.np >= 8) {
@@ -399,10 +397,6 @@ __global__ void __launch_bounds__(1024) k_scan(const Level P, const Dev D) {
     }
     __syncthreads();
   }
-  // the level's largest child: hull launches for large parts skip levels
-  // without any
-  childMax = __reduce_max_sync(FULLMASK, childMax);
-  if (lane == 0 && childMax != 0) atomicMax(D.work + 32 + P.workSlot, childMax);
   if (tid == 0 && blockIdx.x == gridDim.x - 1) {
     // the last block holds the level's totals; the bases were read from the
     // copy k_scan_sums made, so the counters can move now
