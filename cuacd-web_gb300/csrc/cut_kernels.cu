@@ -487,7 +487,7 @@ struct Ring {  // ear-clip node arrays of one half (warp-uniform)
   double *X, *Y;
   float *Xf, *Yf;  // the coordinates rounded to float32 (the ear test's prefilter)
   float *Xl, *Yl;  // and the float32 rounding of what that rounding left out
-  uint32_t n, cap;
+  uint32_t n;
   // uniform grid over the nodes (built once the holes are bridged in), in
   // the float32 coordinates: the ear test looks only at the nodes in the
   // cells its triangle's bounding box covers (rounding is monotonic, so a
@@ -496,15 +496,15 @@ struct Ring {  // ear-clip node arrays of one half (warp-uniform)
   uint32_t *gCnt, *gStart, *gNodes;
   uint32_t gnx, gny;
   float gx0, gy0, ginvx, ginvy;
-  __device__ uint32_t cell_x(float x) const {
+  __device__ __forceinline__ uint32_t cell_x(float x) const {
     const float f = (x - gx0) * ginvx;
     return f <= 0.0f ? 0u : min(gnx - 1, (uint32_t)f);
   }
-  __device__ uint32_t cell_y(float y) const {
+  __device__ __forceinline__ uint32_t cell_y(float y) const {
     const float f = (y - gy0) * ginvy;
     return f <= 0.0f ? 0u : min(gny - 1, (uint32_t)f);
   }
-  __device__ void bridge(uint32_t a, uint32_t b) {
+  __device__ __forceinline__ void bridge(uint32_t a, uint32_t b) {
     const uint32_t a2 = n++;
     I[a2] = I[a]; X[a2] = X[a]; Y[a2] = Y[a]; Xf[a2] = Xf[a]; Yf[a2] = Yf[a]; Xl[a2] = Xl[a]; Yl[a2] = Yl[a];
     alive[a2] = 1;
@@ -521,7 +521,7 @@ struct Ring {  // ear-clip node arrays of one half (warp-uniform)
     next[bp] = b2;
     prev[b2] = bp;
   }
-  __device__ bool reflex(uint32_t k) const {
+  __device__ __forceinline__ bool reflex(uint32_t k) const {
     return orient2(X[prev[k]], Y[prev[k]], X[k], Y[k], X[next[k]], Y[next[k]]) < 0;
   }
 };
@@ -531,7 +531,7 @@ struct Ring {  // ear-clip node arrays of one half (warp-uniform)
 // them (nodes in creation order, each linked after the previous): the
 // signed area's terms in parallel and their sum in order, then every node at
 // once; returns the last node
-__device__ uint32_t ring_par(Ring& P, const double* gxy, uint32_t s, uint32_t e, bool ccw, int lane) {
+__device__ __forceinline__ uint32_t ring_par(Ring& P, const double* gxy, uint32_t s, uint32_t e, bool ccw, int lane) {
   const uint32_t base = P.n, len = e - s;
   double* terms = P.X + base;  // scratch until the nodes are written
   for (uint32_t i = lane; i < len; i += 32) {
@@ -576,7 +576,7 @@ __device__ uint32_t ring_par(Ring& P, const double* gxy, uint32_t s, uint32_t e,
 // ring position. Every value is the host's double expression on the same
 // operands. order and pos are scratch (the grid's node list and the alive
 // words, both rebuilt before the ear clipping).
-__device__ int32_t find_bridge(const Ring& P, uint32_t h, uint32_t outer, uint32_t* order, uint32_t* pos,
+__device__ __forceinline__ int32_t find_bridge(const Ring& P, uint32_t h, uint32_t outer, uint32_t* order, uint32_t* pos,
                                int lane) {
   uint32_t len = 0;
   if (lane == 0) {
@@ -672,8 +672,18 @@ __device__ int32_t find_bridge(const Ring& P, uint32_t h, uint32_t outer, uint32
 // of both (taken as 8 u (...) + 8 u^2 S (...)), the float value has the
 // double result's sign; otherwise the double orient2 is computed.
 // Returns +1, -1, or 0 for an exact double zero.
-__device__ __forceinline__ float ring_diff(const float* h, const float* l, uint32_t b, uint32_t a) {
-  return __fadd_rn(__fsub_rn(h[b], h[a]), __fsub_rn(l[b], l[a]));
+struct RingPt {  // a ring node's coordinates as float pairs
+  float xf, xl, yf, yl;
+};
+__device__ __forceinline__ RingPt ring_pt(const Ring& P, uint32_t k) {
+  RingPt r;
+  r.xf = P.Xf[k]; r.xl = P.Xl[k];
+  r.yf = P.Yf[k]; r.yl = P.Yl[k];
+  return r;
+}
+// (bh + bl) - (ah + al)
+__device__ __forceinline__ float ring_diff(float bh, float bl, float ah, float al) {
+  return __fadd_rn(__fsub_rn(bh, ah), __fsub_rn(bl, al));
 }
 
 // s + e = a + b exactly (Knuth's two-sum; no overflow in range)
@@ -685,10 +695,10 @@ __device__ __forceinline__ void two_sum(float a, float b, float& s, float& e) {
 
 // the difference of two ring coordinates as an unevaluated float pair
 // (s, r): s + e = hi_b - hi_a exactly, r = fl(e + fl(lo_b - lo_a))
-__device__ __forceinline__ void ring_diff2(const float* h, const float* l, uint32_t b, uint32_t a, float& s, float& r) {
+__device__ __forceinline__ void ring_diff2(float bh, float bl, float ah, float al, float& s, float& r) {
   float e;
-  two_sum(h[b], -h[a], s, e);
-  r = __fadd_rn(e, __fsub_rn(l[b], l[a]));
+  two_sum(bh, -ah, s, e);
+  r = __fadd_rn(e, __fsub_rn(bl, al));
 }
 
 // The second filter: orient2 in float-float arithmetic. With u = 2^-24 and
@@ -703,12 +713,12 @@ __device__ __forceinline__ void ring_diff2(const float* h, const float* l, uint3
 // (|p1| + |p2|) + 24 u^2 S sum|s| + 128 u^3 S^2 (+ 2^-140 (sum|s| + 1)) the
 // float-float value has the double result's sign. Returns +1, -1, or 2
 // when undecided.
-__device__ int orient_ff(const Ring& P, uint32_t a, uint32_t b, uint32_t c, float S) {
+__device__ __noinline__ int orient_ff(RingPt a, RingPt b, RingPt c, float S) {
   float s1, r1, s2, r2, s3, r3, s4, r4;
-  ring_diff2(P.Xf, P.Xl, b, a, s1, r1);
-  ring_diff2(P.Yf, P.Yl, c, a, s2, r2);
-  ring_diff2(P.Yf, P.Yl, b, a, s3, r3);
-  ring_diff2(P.Xf, P.Xl, c, a, s4, r4);
+  ring_diff2(b.xf, b.xl, a.xf, a.xl, s1, r1);
+  ring_diff2(c.yf, c.yl, a.yf, a.yl, s2, r2);
+  ring_diff2(b.yf, b.yl, a.yf, a.yl, s3, r3);
+  ring_diff2(c.xf, c.xl, a.xf, a.xl, s4, r4);
   const float p1 = __fmul_rn(s1, s2), q1 = __fmaf_rn(s1, s2, -p1);
   const float p2 = __fmul_rn(s3, s4), q2 = __fmaf_rn(s3, s4, -p2);
   const float c1 = __fadd_rn(__fadd_rn(__fmul_rn(s1, r2), __fmul_rn(r1, s2)), __fmul_rn(r1, r2));
@@ -730,13 +740,14 @@ __device__ int orient_ff(const Ring& P, uint32_t a, uint32_t b, uint32_t c, floa
   return 2;
 }
 
-__device__ int orient_sign(const Ring& P, uint32_t a, uint32_t b, uint32_t c) {
-  const float d1 = ring_diff(P.Xf, P.Xl, b, a), d2 = ring_diff(P.Yf, P.Yl, c, a);
-  const float d3 = ring_diff(P.Yf, P.Yl, b, a), d4 = ring_diff(P.Xf, P.Xl, c, a);
+__device__ __forceinline__ int orient_sign(const Ring& P, uint32_t a, uint32_t b, uint32_t c) {
+  const RingPt pa = ring_pt(P, a), pb = ring_pt(P, b), pc = ring_pt(P, c);
+  const float d1 = ring_diff(pb.xf, pb.xl, pa.xf, pa.xl), d2 = ring_diff(pc.yf, pc.yl, pa.yf, pa.yl);
+  const float d3 = ring_diff(pb.yf, pb.yl, pa.yf, pa.yl), d4 = ring_diff(pc.xf, pc.xl, pa.xf, pa.xl);
   const float p1 = __fmul_rn(d1, d2), p2 = __fmul_rn(d3, d4);
   const float o = __fsub_rn(p1, p2);
-  const float S = fmaxf(fmaxf(fmaxf(fabsf(P.Xf[a]), fabsf(P.Yf[a])), fmaxf(fabsf(P.Xf[b]), fabsf(P.Yf[b]))),
-                        fmaxf(fabsf(P.Xf[c]), fabsf(P.Yf[c])));
+  const float S = fmaxf(fmaxf(fmaxf(fabsf(pa.xf), fabsf(pa.yf)), fmaxf(fabsf(pb.xf), fabsf(pb.yf))),
+                        fmaxf(fabsf(pc.xf), fabsf(pc.yf)));
   if (S < 1e15f) {
     const float u = 5.9604645e-8f;
     const float eb = __fadd_rn(__fmul_rn(8.0f * u, __fadd_rn(fabsf(p1), fabsf(p2))),
@@ -749,7 +760,7 @@ __device__ int orient_sign(const Ring& P, uint32_t a, uint32_t b, uint32_t c) {
     }
     // near-collinear: the float-float filter, then double for what it
     // cannot decide (this GPU's FP64 rate is a small fraction of FP32's)
-    const int f = orient_ff(P, a, b, c, S);
+    const int f = orient_ff(pa, pb, pc, S);
     if (f != 2) return f;
   }
   const double r = orient2(P.X[a], P.Y[a], P.X[b], P.Y[b], P.X[c], P.Y[c]);
@@ -779,7 +790,7 @@ __device__ __forceinline__ int gate_sign(const Ring& P, uint32_t k) {
 // the orientation gate of the ear test at vertex k (is_ear returns false at
 // once when it fails): the triangle (prev, k, next) turns left, or is flat in
 // flat mode
-__device__ bool ear_gate(const Ring& P, uint32_t k, bool allowFlat) {
+__device__ __forceinline__ bool ear_gate(const Ring& P, uint32_t k, bool allowFlat) {
   const int sg = gate_sign(P, k);
   return sg > 0 || (sg == 0 && allowFlat);
 }
@@ -788,7 +799,7 @@ __device__ bool ear_gate(const Ring& P, uint32_t k, bool allowFlat) {
 // the nodes and vote. Each node test is the host clipper's double test; the
 // float copies decide it exactly where they can, and the double arithmetic
 // (slow on this GPU) runs only for ties and near-zero orientations
-__device__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat, int lane) {
+__device__ __forceinline__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat, int lane) {
   const uint32_t a = P.prev[k], b = k, c = P.next[k];
   const float axf = P.Xf[a], ayf = P.Yf[a], bxf = P.Xf[b], byf = P.Yf[b], cxf = P.Xf[c], cyf = P.Yf[c];
   // the ear's orientation (arPos: ar > 0; otherwise ar == 0 in flat mode)
@@ -809,9 +820,9 @@ __device__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat, int lane) {
   const uint32_t x0 = P.cell_x(fbx0), x1 = P.cell_x(fbx1);
   const uint32_t y0 = P.cell_y(fby0), y1 = P.cell_y(fby1);
   // the nodes of one row of covered cells are contiguous in the grid's node
-  // list: the lanes take 32 consecutive entries at a time (coalesced, the
-  // loads of the whole warp in flight together) and the warp stops at the
-  // first batch holding a node inside
+  // list: up to 32 rows at once, their entries spread over the lanes (an ear
+  // covers a few rows of a few entries each), and the warp stops at the
+  // first 32 entries holding a node inside
   auto inside = [&](uint32_t q) -> bool {
     if (!(P.alive[q] & 1u) || q == a || q == b || q == c) return false;
     const float qxf = P.Xf[q], qyf = P.Yf[q];
@@ -829,7 +840,17 @@ __device__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat, int lane) {
         (qxf == bxf && qyf == byf && P.X[q] == P.X[b] && P.Y[q] == P.Y[b]) ||
         (qxf == cxf && qyf == cyf && P.X[q] == P.X[c] && P.Y[q] == P.Y[c]))
       return false;
-    if (orient_sign(P, a, b, q) < 0 || orient_sign(P, b, c, q) < 0 || orient_sign(P, c, a, q) < 0) return false;
+    {
+      uint32_t u = a, v = b, t = c;
+#pragma unroll 1
+      for (int e = 0; e < 3; e++) {  // one copy of the test for the three edges
+        if (orient_sign(P, u, v, q) < 0) return false;
+        const uint32_t f = u;
+        u = v;
+        v = t;
+        t = f;
+      }
+    }
     if (!arPos) {
       // a flat ear: only nodes within the box of its two ends count
       const double qx = P.X[q], qy = P.Y[q], ax = P.X[a], ay = P.Y[a], cx = P.X[c], cy = P.Y[c];
@@ -839,12 +860,29 @@ __device__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat, int lane) {
   };
   bool hit = false;
   uint32_t hitQ = 0;
-  for (uint32_t y = y0; y <= y1 && !hit; y++) {
-    const uint32_t e0 = P.gStart[y * P.gnx + x0], e1 = P.gStart[y * P.gnx + x1 + 1];
-    for (uint32_t base = e0; base < e1; base += 32) {
-      const uint32_t e = base + (uint32_t)lane;
-      const uint32_t q = e < e1 ? P.gNodes[e] : 0u;
-      const bool h = e < e1 && inside(q);
+  for (uint32_t yb = y0; yb <= y1 && !hit; yb += 32) {
+    const uint32_t rows = min(32u, y1 - yb + 1);
+    uint32_t e0 = 0, len = 0;
+    if ((uint32_t)lane < rows) {
+      const uint32_t* g = P.gStart + (yb + (uint32_t)lane) * P.gnx;
+      e0 = g[x0];
+      len = g[x1 + 1] - e0;
+    }
+    uint32_t inc = len;
+    for (int d = 1; d < 32 && d < (int)rows; d <<= 1) {
+      const uint32_t u = __shfl_up_sync(CUT_FULL, inc, d);
+      if (lane >= d) inc += u;
+    }
+    const uint32_t total = __shfl_sync(CUT_FULL, inc, rows - 1), shift = e0 - (inc - len);
+    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+      const uint32_t t = t0 + (uint32_t)lane;
+      uint32_t e = CUT_NONE;
+      for (uint32_t r = 0; r < rows; r++) {  // the row holding entry t: the first that ends behind it
+        const uint32_t end = __shfl_sync(CUT_FULL, inc, r), sh = __shfl_sync(CUT_FULL, shift, r);
+        if (t < end && e == CUT_NONE) e = t + sh;
+      }
+      const uint32_t q = e != CUT_NONE ? P.gNodes[e] : 0u;
+      const bool h = e != CUT_NONE && inside(q);
       const uint32_t hb = __ballot_sync(CUT_FULL, h);
       if (hb) {
         hit = true;
@@ -864,7 +902,7 @@ __device__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat, int lane) {
 // the uniform grid of the ring's P.n nodes: about two nodes per cell over
 // their bounding box, nodes listed per cell (lanes split the work; the order
 // within a cell does not matter)
-__device__ void build_grid(Ring& P, int lane) {
+__device__ __forceinline__ void build_grid(Ring& P, int lane) {
   float x0 = INFINITY, y0 = INFINITY, x1 = -INFINITY, y1 = -INFINITY;
   for (uint32_t q = lane; q < P.n; q += 32) {
     x0 = fminf(x0, P.Xf[q]);
@@ -929,9 +967,40 @@ __device__ void build_grid(Ring& P, int lane) {
 
 // ear clipping of the group's ring (outer loop [0, outerEnd), holes from
 // holeStart); writes ring-index triples to out; returns the triangle count
-// (fewer than n + 2 h - 2 when the polygon could not be clipped)
-__device__ uint32_t ear_clip(Ring& P, const uint32_t* gid, const double* gxy, uint32_t nAll, const uint32_t* hs,
-                             uint32_t nHoles, uint32_t* holeL, double* holeX, uint32_t* out, int lane) {
+// (fewer than n + 2 h - 2 when the polygon could not be clipped).
+// What bounds it: one warp's instruction latency, about 4,000 cycles an ear
+// (7,400 with the window refilled for every ear, the covered grid rows visited
+// one by one and the ring behind a reference): 192 caps of about 230 edges
+// 2.07 -> 1.44 ms, 24 caps of up to 800 edges 2.97 -> 1.87 ms.
+// The ring's arrays are set up here, in shared memory when SM (their pointers
+// then are shared addresses in registers; behind a reference to one of two
+// rings every access first read its pointer from local memory, which cost a
+// third of a cap).
+template <bool SM>
+__device__ __noinline__ uint32_t ear_clip(const Ring* global, const uint32_t* gid, const double* gxy, uint32_t nAll,
+                                          const uint32_t* hs, uint32_t nHoles, uint32_t* holeL, double* holeX,
+                                          uint32_t* out, int lane) {
+  Ring P;
+  if constexpr (SM) {
+    extern __shared__ __align__(16) unsigned char capSm[];
+    double* sx = reinterpret_cast<double*>(capSm);
+    P.X = sx;
+    P.Y = sx + CAP_SM_NODES;
+    uint32_t* su = reinterpret_cast<uint32_t*>(sx + 2 * CAP_SM_NODES);
+    P.I = su;
+    P.prev = su + CAP_SM_NODES;
+    P.next = su + 2 * CAP_SM_NODES;
+    P.alive = su + 3 * CAP_SM_NODES;
+    P.gNodes = su + 4 * CAP_SM_NODES;
+    P.gCnt = su + 5 * CAP_SM_NODES;
+    P.gStart = P.gCnt + CAP_SM_NODES / 2 + 2;
+    P.Xf = reinterpret_cast<float*>(P.gStart + CAP_SM_NODES / 2 + 2);
+    P.Yf = P.Xf + CAP_SM_NODES;
+    P.Xl = P.Yf + CAP_SM_NODES;
+    P.Yl = P.Xl + CAP_SM_NODES;
+  } else {
+    P = *global;
+  }
   P.n = 0;
   const uint32_t outerEnd = nHoles == 0 ? nAll : hs[0];
   if (outerEnd < 3) return 0;
@@ -984,7 +1053,7 @@ __device__ uint32_t ear_clip(Ring& P, const uint32_t* gid, const double* gxy, ui
     if (count > P.n) return 0;  // not a ring: never for a well-formed group
   }
   uint32_t nOut = 0;
-  uint32_t ear = outer, stop = outer;
+  uint32_t stop = outer;
   bool flat = false;
   // The host clipper tests ear, next(ear), ... one at a time; most tests
   // fail at the orientation gate (reflex, or flat outside flat mode), and a
@@ -993,7 +1062,23 @@ __device__ uint32_t ear_clip(Ring& P, const uint32_t* gid, const double* gxy, ui
   // the full test runs on the gate's survivors in ring order; the first
   // that passes is the ear the host finds. Reaching `stop` ends the batch
   // there, where the host switches to flat mode (or gives up).
-  __shared__ uint32_t ring33[33];
+  //
+  // The 32 vertices stay in the lanes' registers from batch to batch (lane i
+  // holds the i-th from the current one, w32 the 33rd): a clip found at lane
+  // i moves them up by i + 1 and only as many links are followed, where
+  // following 33 dependent links took 1,400 of a batch's 8,000 cycles. A
+  // ring of at most 32 vertices is held whole and rotates in place.
+  uint32_t node = 0, w32 = 0;
+  auto fill = [&](uint32_t from) {
+    uint32_t x = from;
+    const uint32_t n = min(count, 33u);
+    for (uint32_t i = 0; i < n; i++) {
+      if ((uint32_t)lane == i) node = x;
+      w32 = x;
+      x = P.next[x];
+    }
+  };
+  fill(outer);
   // each batch clips an ear, ends a pass, or advances 32 vertices, so
   // 2 n^2 + 16 batches are never reached; the bound keeps a malformed ring
   // finite
@@ -1001,70 +1086,74 @@ __device__ uint32_t ear_clip(Ring& P, const uint32_t* gid, const double* gxy, ui
   unsigned long long steps = 0;
   while (count > 3) {
     if (++steps > maxSteps) return nOut;
-    if (lane == 0) {
-      uint32_t cv = ear;
-      for (int i = 0; i < 33; i++) {
-        ring33[i] = cv;
-        cv = P.next[cv];
-      }
-    }
-    __syncwarp();
-    // the batch: positions [0, jStop), jStop = first return to `stop`
-    uint32_t jStop = 33;
-    {
-      const bool isStop = lane >= 1 && ring33[lane] == stop;
-      const bool isStop32 = ring33[32] == stop;
-      const uint32_t bal = __ballot_sync(CUT_FULL, isStop);
-      jStop = bal ? (uint32_t)(__ffs(bal) - 1) : (isStop32 ? 32u : 33u);
+    // the batch: positions [0, jStop), jStop = first return to `stop` (a ring
+    // held whole always starts there)
+    uint32_t jStop;
+    if (count <= 32) {
+      jStop = count;
+    } else {
+      const uint32_t bal = __ballot_sync(CUT_FULL, lane >= 1 && node == stop);
+      jStop = bal ? (uint32_t)(__ffs(bal) - 1) : (w32 == stop ? 32u : 33u);
     }
     const uint32_t nTest = min(jStop, 32u);
-    const uint32_t mine = ring33[lane];
-    const bool gate = (uint32_t)lane < nTest && ear_gate(P, mine, flat);
+    const bool gate = (uint32_t)lane < nTest && ear_gate(P, node, flat);
     __syncwarp();  // the gates' memo writes before the ear tests read them
     uint32_t cand = __ballot_sync(CUT_FULL, gate);
     int found = -1;
     while (cand) {
       const int i = __ffs(cand) - 1;
       cand &= cand - 1;
-      if (is_ear(P, ring33[i], flat, lane)) {
+      if (is_ear(P, __shfl_sync(CUT_FULL, node, i), flat, lane)) {
         found = i;
         break;
       }
     }
     if (found >= 0) {
-      ear = ring33[found];
+      const uint32_t ear = __shfl_sync(CUT_FULL, node, found);
       const uint32_t a = P.prev[ear], c = P.next[ear];
-      out[3 * nOut] = P.I[a];
-      out[3 * nOut + 1] = P.I[ear];
-      out[3 * nOut + 2] = P.I[c];
+      __syncwarp();
+      if (lane < 3) out[3 * nOut + lane] = lane == 0 ? a : (lane == 1 ? ear : c);  // nodes, see below
+      if (lane == 0) {
+        P.next[a] = c;
+        P.prev[c] = a;
+        P.alive[ear] = 0;
+        P.alive[a] = 1;  // new neighbours: the memo starts over
+        P.alive[c] = 1;
+      }
       nOut++;
       __syncwarp();
-      P.next[a] = c;
-      P.prev[c] = a;
-      P.alive[ear] = 0;
-      P.alive[a] = 1;  // new neighbours: the memo starts over
-      P.alive[c] = 1;
+      const uint32_t s = (uint32_t)found + 1;
+      if (count <= 32) {
+        const uint32_t from = (uint32_t)lane + s;
+        node = __shfl_sync(CUT_FULL, node, from >= count ? from - count : from);
+      } else {
+        uint32_t v = __shfl_sync(CUT_FULL, node, ((uint32_t)lane + s) & 31u);
+        if ((uint32_t)lane + s == 32) v = w32;
+        for (uint32_t t = 1; t <= s; t++) {
+          w32 = P.next[w32];
+          if ((uint32_t)lane + s == 32 + t) v = w32;
+        }
+        node = v;
+      }
       count--;
-      ear = c;
       stop = c;
       flat = false;
-      __syncwarp();
       continue;
     }
     if (jStop <= 32) {
       // the walk reached `stop`: the host switches to flat mode or gives up
-      ear = stop;
       if (flat) return nOut;
       flat = true;
+      if (count > 32) fill(stop);
     } else {
-      ear = ring33[32];
+      fill(w32);
     }
-    __syncwarp();
   }
-  const uint32_t a = P.prev[ear], c = P.next[ear];
-  out[3 * nOut] = P.I[a];
-  out[3 * nOut + 1] = P.I[ear];
-  out[3 * nOut + 2] = P.I[c];
+  const uint32_t last = __shfl_sync(CUT_FULL, node, 0);
+  if (lane < 3) out[3 * nOut + lane] = lane == 0 ? P.prev[last] : (lane == 1 ? last : P.next[last]);
+  __syncwarp();
+  // the triples' nodes to ring indices
+  for (uint32_t k = lane; k < 3 * (nOut + 1); k += 32) out[k] = P.I[out[k]];
   return nOut + 1;
 }
 
@@ -1242,14 +1331,92 @@ __global__ void k_cut_cap(const CutDesc* __restrict__ D, const CutLayout* __rest
     bDstW = sDst;
     __syncwarp();
   }
-  // Steps 3 and 4 are sequential and each decision reads what earlier
-  // iterations wrote (hash inserts, used flags), so they run on lane 0 alone
-  // while the other lanes wait; every list walk is bounded.
   uint32_t* loopV = w + cv.loopV;
   uint32_t* loopS = w + cv.loopS;
   uint32_t nLoops = 0, nLV = 0;
   int walkFail = 0;
-  if (lane == 0) {
+  // A cut of a manifold gives every boundary vertex one out-edge. Then the
+  // lanes enter the sources at once (a source met twice shows here), the
+  // starts are the edges' sources in order, and every edge's successor is
+  // looked up at once, so the walk on lane 0 follows one link per edge and
+  // tests its used flag: the first unused out-edge of a vertex is its only
+  // one, unused, or none. (Two hash searches per edge on lane 0 took 1,300
+  // cycles an edge, 15 % of the cap.)
+  bool single = true;
+  {
+    bool twice = false;
+    for (uint32_t i = lane; i < B; i += 32) {
+      const uint32_t key = bSrcW[i];
+      uint32_t h = mix_key(key) & (shSize - 1);
+      bool entered = false;
+      for (uint32_t probe = 0; probe < shSize; probe++, h = (h + 1) & (shSize - 1)) {
+        const uint32_t k = atomicCAS(shKey + h, CUT_NONE, key);
+        if (k == CUT_NONE) {
+          shHead[h] = i;
+          entered = true;
+        }
+        if (k == CUT_NONE || k == key) break;
+      }
+      twice = twice || !entered;
+      bUsed[i] = 0;
+    }
+    single = !__any_sync(CUT_FULL, twice);
+    __syncwarp();
+  }
+  if (single) {
+    for (uint32_t i = lane; i < B; i += 32) {
+      bool ins;
+      const uint32_t h = uh_find(shKey, shSize, bDstW[i], false, &ins);
+      bNext[i] = h == CUT_NONE ? CUT_NONE : shHead[h];
+    }
+    __syncwarp();
+    if (lane == 0) {
+      loopS[0] = 0;
+      for (uint32_t e = 0; e < B && !walkFail; e++) {
+        if (bUsed[e]) continue;
+        if (nLV >= m) {
+          walkFail = CUT_SCRATCH;
+          break;
+        }
+        const uint32_t lvStart = nLV, start = bSrcW[e];
+        loopV[nLV++] = start;
+        bUsed[e] = 1;
+        uint32_t x = e, cur = bDstW[e], guard = 0;
+        while (cur != start) {
+          if (nLV >= m) {
+            walkFail = CUT_SCRATCH;
+            break;
+          }
+          loopV[nLV++] = cur;
+          x = bNext[x];
+          if (x == CUT_NONE) {
+            walkFail = CUT_OPEN_CHAIN;
+            break;
+          }
+          if (bUsed[x]) {
+            walkFail = CUT_DEAD_END;
+            break;
+          }
+          bUsed[x] = 1;
+          cur = bDstW[x];
+          if (++guard > B + 1) {
+            walkFail = CUT_CYCLE;
+            break;
+          }
+        }
+        if (walkFail) break;
+        if (nLV - lvStart >= 3) loopS[++nLoops] = nLV;
+        else nLV = lvStart;
+      }
+    }
+  } else {
+    for (uint32_t i = lane; i < shSize; i += 32) shKey[i] = CUT_NONE;
+    __syncwarp();
+  }
+  // Otherwise steps 3 and 4 are sequential and each decision reads what earlier
+  // iterations wrote (hash inserts, used flags), so they run on lane 0 alone
+  // while the other lanes wait; every list walk is bounded.
+  if (!single && lane == 0) {
     uint32_t nStarts = 0;
     for (uint32_t i = 0; i < B && !walkFail; i++) {
       bool ins;
@@ -1462,7 +1629,6 @@ __global__ void k_cut_cap(const CutDesc* __restrict__ D, const CutLayout* __rest
   Pg.alive = w + cv.ndAlive;
   Pg.X = x + cv.ndX;
   Pg.Y = x + cv.ndY;
-  Pg.cap = cv.nd;
   Pg.n = 0;
   Pg.gCnt = w + cv.gCnt;
   Pg.gStart = w + cv.gStart;
@@ -1471,26 +1637,6 @@ __global__ void k_cut_cap(const CutDesc* __restrict__ D, const CutLayout* __rest
   Pg.Yf = reinterpret_cast<float*>(w + cv.ndYf);
   Pg.Xl = reinterpret_cast<float*>(w + cv.ndXl);
   Pg.Yl = reinterpret_cast<float*>(w + cv.ndYl);
-  Ring Ps;
-  {
-    double* sx = reinterpret_cast<double*>(capSm);
-    Ps.X = sx;
-    Ps.Y = sx + CAP_SM_NODES;
-    uint32_t* su = reinterpret_cast<uint32_t*>(sx + 2 * CAP_SM_NODES);
-    Ps.I = su;
-    Ps.prev = su + CAP_SM_NODES;
-    Ps.next = su + 2 * CAP_SM_NODES;
-    Ps.alive = su + 3 * CAP_SM_NODES;
-    Ps.gNodes = su + 4 * CAP_SM_NODES;
-    Ps.gCnt = su + 5 * CAP_SM_NODES;
-    Ps.gStart = Ps.gCnt + CAP_SM_NODES / 2 + 2;
-    Ps.Xf = reinterpret_cast<float*>(Ps.gStart + CAP_SM_NODES / 2 + 2);
-    Ps.Yf = Ps.Xf + CAP_SM_NODES;
-    Ps.Xl = Ps.Yf + CAP_SM_NODES;
-    Ps.Yl = Ps.Xl + CAP_SM_NODES;
-    Ps.cap = CAP_SM_NODES;
-    Ps.n = 0;
-  }
   uint32_t* gid = w + cv.gId;
   double* gxy = x + cv.gXY;
   uint32_t* holeL = w + cv.holeL;
@@ -1520,7 +1666,8 @@ __global__ void k_cut_cap(const CutDesc* __restrict__ D, const CutLayout* __rest
     __syncwarp();
     const uint32_t expected = nAll + 2 * nHoles - 2;
     const uint32_t ringNodes = nAll + 2 * nHoles;
-    if (ringNodes > Ps.cap && ringNodes <= CAP_SM_LINK_NODES) {
+    const bool inSm = ringNodes <= CAP_SM_NODES;
+    if (!inSm && ringNodes <= CAP_SM_LINK_NODES) {
       uint32_t* su = reinterpret_cast<uint32_t*>(capSm);
       Pg.prev = su;
       Pg.next = su + CAP_SM_LINK_NODES;
@@ -1530,13 +1677,13 @@ __global__ void k_cut_cap(const CutDesc* __restrict__ D, const CutLayout* __rest
       Pg.next = w + cv.ndNext;
       Pg.alive = w + cv.ndAlive;
     }
-    Ring& P = ringNodes <= Ps.cap ? Ps : Pg;
-    if (nCap + nAll + 2 * nHoles > capMax || nAll + 2 * nHoles > P.cap) {
+    if (nCap + nAll + 2 * nHoles > capMax || ringNodes > (inSm ? CAP_SM_NODES : cv.nd)) {
       failWith(CUT_SCRATCH);
       return;
     }
     __syncwarp();
-    const uint32_t got = ear_clip(P, gid, gxy, nAll, hs, nHoles, holeL, holeX, capT + 3 * nCap, lane);
+    const uint32_t got = inSm ? ear_clip<true>(&Pg, gid, gxy, nAll, hs, nHoles, holeL, holeX, capT + 3 * nCap, lane)
+                              : ear_clip<false>(&Pg, gid, gxy, nAll, hs, nHoles, holeL, holeX, capT + 3 * nCap, lane);
     __syncwarp();
     if (got != expected) {
       if (!fan(i)) {
