@@ -74,7 +74,7 @@ struct HullSm {
 #define TINY_SEEDS 24u
 struct TinySm {
   uint32_t stage[3 * TINY_FACES];  // new face j: a, b, old lane of the face across (a, b)
-  uint8_t hA[QC_MAX];              // per point: lane of the new face starting there
+  alignas(4) uint8_t hA[QC_MAX];   // per point: lane of the new face starting there
   uint8_t hB[QC_MAX];              // per point: lane of the new face ending there
 };
 
@@ -2363,16 +2363,35 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   // 80 seeds: max and min along 40 axes, lowest index on ties; seed 2a is
   // the maximum along axis a, seed 2a + 1 the minimum
   if (G == 32 && h.qc != nullptr) {
-    // one lane per axis, each scanning every point in index order
-    for (uint32_t a = lid; a < 40; a += G) {
+    // one lane per axis for the first 32, each scanning every point in index
+    // order; the last 8 axes take 4 lanes each, a quarter of the points a lane
+    // (two full scans for 40 axes cost 4 % of a staircase child's hull)
+    auto scan = [&](uint32_t a, uint32_t i0, uint32_t i1, float& mx, float& mn, uint32_t& ix, uint32_t& in) {
       const f3 ax = mk3(c_kdop[a][0], c_kdop[a][1], c_kdop[a][2]);
-      float mx = -1e30f, mn = 1e30f;
-      uint32_t ix = 0, in = 0;
-      for (uint32_t i = 0; i < nv; i++) {
+      mx = -1e30f;
+      mn = 1e30f;
+      ix = in = 0;
+      for (uint32_t i = i0; i < i1; i++) {
         const float d = dot(ax, h.qvert(i));
         if (d > mx) { mx = d; ix = i; }
         if (d < mn) { mn = d; in = i; }
       }
+    };
+    float mx, mn;
+    uint32_t ix, in;
+    scan(lid, 0, nv, mx, mn, ix, in);
+    hs.seed[2 * lid] = ix;
+    hs.seed[2 * lid + 1] = in;
+    const uint32_t a = 32 + (lid >> 2), part = lid & 3;
+    scan(a, nv * part / 4, nv * (part + 1) / 4, mx, mn, ix, in);
+#pragma unroll
+    for (int o = 1; o < 4; o <<= 1) {  // quarters in order: a tie keeps the lower point
+      const float mx2 = __shfl_xor_sync(FULLMASK, mx, o), mn2 = __shfl_xor_sync(FULLMASK, mn, o);
+      const uint32_t ix2 = __shfl_xor_sync(FULLMASK, ix, o), in2 = __shfl_xor_sync(FULLMASK, in, o);
+      if (mx2 > mx || (mx2 == mx && ix2 < ix)) { mx = mx2; ix = ix2; }
+      if (mn2 < mn || (mn2 == mn && in2 < in)) { mn = mn2; in = in2; }
+    }
+    if (part == 0) {
       hs.seed[2 * a] = ix;
       hs.seed[2 * a + 1] = in;
     }
@@ -2474,11 +2493,25 @@ restart:
   // the list have the same distance and index, so they never change a pick
   // or an owner, and the list keeps first occurrences only.
   uint32_t nuniq = 0;
+  // (a warp marks the points it has listed, in the horizon map's bytes;
+  // comparing every pair of positions was another 4 %)
+  const bool marks = G == 32 && ts != nullptr && h.qc != nullptr;
+  if (marks) {
+    for (uint32_t w = lid; w < QC_MAX / 4; w += 32) reinterpret_cast<uint32_t*>(ts->hA)[w] = 0;
+    Grp<G>::sync();
+  }
   for (uint32_t c = 0; c * G < 80; c++) {
     const uint32_t k = c * G + lid;
     bool keep = false;
     uint32_t s = 0;
-    if (k < 80) {
+    if (marks) {
+      s = k < 80 ? hs.seed[k] : QC_MAX + lid;
+      const unsigned same = __match_any_sync(FULLMASK, s);
+      keep = k < 80 && (same & lanemask_lt()) == 0 && ts->hA[s] == 0;
+      __syncwarp();
+      if (keep) ts->hA[s] = 1;
+      __syncwarp();
+    } else if (k < 80) {
       s = hs.seed[k];
       keep = true;
       for (uint32_t j = 0; j < k; j++) if (hs.seed[j] == s) { keep = false; break; }
