@@ -27,7 +27,7 @@
 namespace cuacd {
 void launch_plan(const Level& P, const Dev& D, bool big, cudaStream_t s);
 void launch_scan(const Level& P, const Dev& D, cudaStream_t s);
-void launch_emit(const Level& P, const Dev& D, bool big, cudaStream_t s);
+void launch_emit(const Level& P, const Dev& D, bool big, bool wide, cudaStream_t s);
 void launch_record(const Level& P, const Dev& D, cudaStream_t s);
 void launch_seed_bound(const Level& P, const Dev& D, cudaStream_t s);
 void launch_evaluate(uint32_t stateBase, uint32_t headerOff, uint32_t mode, uint32_t nSeeds, uint32_t jobBase,
@@ -62,6 +62,15 @@ static const uint32_t VIS_MAX = CUACD_VIS_MAX;
 // 256-thread block (narrower blocks for mid-sized parts measured slower: the
 // passes over all points and candidates need the width)
 static const uint32_t SMALL_NV = 1024;
+// A level of at most WIDE_JOBS jobs per SM, or whose parents have WIDE_NV
+// points or more, plans and emits a job on a block, with the warp form's sums
+// (k_emit<256, 32>): a warp per job leaves the GPU idle there. Plan + emit of a
+// depth-2 run, warps against blocks: one blob of 120 points 0.58 and 0.20 ms,
+// of 1,678 points 5.2 and 1.06 ms; 16 of 220 points (1,120 and 3,360 jobs) 1.07
+// and 0.62; 64 of 818 points (13,440 jobs) 6.5 and 5.0; depth-3 staircases of 96
+// points, 8 of them 0.78 and 0.49, 40 (25,200 jobs) 1.26 and 1.48, 160 (100,800
+// jobs) 3.4 and 5.3.
+static const uint32_t WIDE_JOBS = 16, WIDE_NV = 128;
 // Hausdorff targets with at least this many triangles are searched by clusters
 static const uint32_t HD_SCREEN_MIN = 64;
 // parents with more points than this get a block per plan / emit job
@@ -526,6 +535,12 @@ struct Tree {
     return 0;
   }
 
+  // parents shrink roughly by half per level
+  bool bigLevel(uint32_t l) const { return (maxSeedNv >> l) > bigJobNv(); }
+  bool wideLevel(uint32_t l, uint32_t nJobs) const {
+    return !bigLevel(l) && (nJobs <= WIDE_JOBS * (uint32_t)nSM || (maxSeedNv >> l) >= WIDE_NV);
+  }
+
   // the whole run on the stream (tree.ts:559-594)
   void enqueue() {
     mark(-1);
@@ -550,13 +565,12 @@ struct Tree {
         P.lastLevel = l == depth - 1 ? 1u : 0u;
         P.nSeeds = cfg.pruneLastLevel ? nSeeds : 0;
         P.workSlot = l;
-        // parents shrink roughly by half per level
-        bool big = (maxSeedNv >> l) > bigJobNv();
-        launch_plan(P, D, big, stream);
+        const bool big = bigLevel(l), wide = wideLevel(l, v.nJobs);
+        launch_plan(P, D, big || wide, stream);
         mark(1);
         launch_scan(P, D, stream);
         mark(2);
-        launch_emit(P, D, big, stream);
+        launch_emit(P, D, big, wide, stream);
         mark(3);
         // the last level's pruning bound, once per seed (the parent level's
         // items are final once its record ran)
@@ -583,7 +597,8 @@ struct Tree {
                                (uint64_t)bPlanes.p, (uint64_t)bCtr.p, snapBytes, (uint64_t)bScan.p,
                                (uint64_t)bWork.p};
     for (auto& L : tree) { s.push_back(L.nJobs); s.push_back(L.totalWidth); s.push_back(L.width); }
-    for (uint32_t l = 0; l < depth; l++) s.push_back((maxSeedNv >> l) > bigJobNv());
+    for (const auto* st : {&tree, &probe})
+      for (uint32_t l = 0; l < st->size(); l++) s.push_back(bigLevel(l) | (wideLevel(l, (*st)[l].nJobs) << 1));
     s.push_back(smallNv());
     s.push_back(baseLevel(false).handOn);
     s.push_back((uint64_t)bList.p);

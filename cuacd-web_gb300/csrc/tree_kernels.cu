@@ -408,8 +408,16 @@ __global__ void __launch_bounds__(1024) k_scan(const Level P, const Dev D) {
 }
 
 // ======================= emit (shaders.ts:556-750) =======================
-template <int G>
+// G threads per job. LANES: the lanes whose compensated flux sums are combined
+// (triangle t belongs to lane t mod LANES). A level of few jobs runs its
+// mid-sized parents on blocks with a warp's 32 lanes: the flux of each
+// triangle goes through shared memory and two warps add it in the warp
+// form's order, so a part's volume has the same bits whichever form it took.
+template <int G, int LANES>
 __global__ void __launch_bounds__(256) k_emit(const Level P, const Dev D) {
+  constexpr bool STAGED = LANES < G;
+  static_assert(LANES == G || (G == 256 && LANES == 32), "a block adds its own lanes' flux or a warp's");
+  __shared__ float staged[2][STAGED ? G : 1];
   __shared__ GrpSmem gsm[Grp<G>::PER_BLOCK];
   const int gi = Grp<G>::gid(), lid = Grp<G>::lid();
   GrpSmem& sm = gsm[gi];
@@ -448,8 +456,8 @@ __global__ void __launch_bounds__(256) k_emit(const Level P, const Dev D) {
       p = ldv(D.V, (size_t)part.vOff + 3 * (size_t)i);
     }
     uint32_t totP, totN;
-    uint32_t preP = grp_scan_u<G>(fp, &totP, sm);
-    uint32_t preN = grp_scan_u<G>(fn, &totN, sm);
+    uint32_t preP = grp_scan_bit<G>(fp != 0, &totP, sm);
+    uint32_t preN = grp_scan_bit<G>(fn != 0, &totN, sm);
     if (i < part.nv) {
       uint32_t ip = CUACD_NONE, in = CUACD_NONE;
       if (fp == 1) { ip = runP + preP; stv(D.V, (size_t)posV + 3 * (size_t)ip, p); }
@@ -466,8 +474,29 @@ __global__ void __launch_bounds__(256) k_emit(const Level P, const Dev D) {
   fluxP.init();
   fluxN.init();
   uint32_t rT[2] = {0, 0}, rV[2] = {0, 0}, rE[2] = {0, 0};
+  // one term per side and chunk of a thread (the staged form adds zeros for
+  // the others, which change nothing); two barriers of the next chunk's scans
+  // lie between the adding warps' reads and the next terms
+  auto add_flux = [&](float fp, bool hasP, float fn, bool hasN) {
+    if constexpr (STAGED) {
+      staged[0][lid] = hasP ? fp : 0.0f;
+      staged[1][lid] = hasN ? fn : 0.0f;
+      __syncthreads();
+      if (lid < 64) {
+        KSum& f = lid < 32 ? fluxP : fluxN;
+        const float* x = staged[lid >> 5] + (lid & 31);
+#pragma unroll
+        for (int w = 0; w < G / 32; w++) f.add(x[32 * w]);
+      }
+    } else {
+      if (hasP) fluxP.add(fp);
+      if (hasN) fluxN.add(fn);
+    }
+  };
   for (uint32_t c = 0; c * G < part.nt; c++) {
     const uint32_t t = c * G + lid;
+    float fl[2] = {0.0f, 0.0f};
+    bool has[2] = {false, false};
     uint32_t tri[3] = {0, 0, 0};
     f3 pos3[3];
     float d[3] = {0.f, 0.f, 0.f};
@@ -543,9 +572,11 @@ __global__ void __launch_bounds__(256) k_emit(const Level P, const Dev D) {
             flux += edge_term(pts[i], pts[j2], cP, o);
           }
         }
-        if (isPos) fluxP.add(flux); else fluxN.add(flux);
+        fl[side] = flux;
+        has[side] = true;
       }
     }
+    add_flux(fl[0], has[0], fl[1], has[1]);
 #pragma unroll
     for (int side = 0; side < 2; side++) {
       rT[side] += tot[side] & 1023u;
@@ -569,34 +600,50 @@ __global__ void __launch_bounds__(256) k_emit(const Level P, const Dev D) {
       if (sp == sq) { cp = sp ? 1 : 0; cn = 1 - cp; } else { cp = 1; cn = 1; }
     }
     uint32_t totP, totN;
-    uint32_t preP = grp_scan_u<G>(cp, &totP, sm);
-    uint32_t preN = grp_scan_u<G>(cn, &totN, sm);
+    uint32_t preP = grp_scan_bit<G>(cp != 0, &totP, sm);
+    uint32_t preN = grp_scan_bit<G>(cn != 0, &totN, sm);
+    float fp = 0.0f, fn = 0.0f;
+    bool hasP = false, hasN = false;
     if (e < part.ne) {
       f3 cE = plane_point(D.planes[pid]);
       bool sp = dp >= 0.0f, sq = dq >= 0.0f;
       size_t ep = (size_t)posEo + rE[0] + preP, en = (size_t)negEo + rE[1] + preN;
       if (sp == sq) {
-        if (sp) { if (keepTopo) put_edge(D.E, ep, p, q, pid); fluxP.add(edge_term(p, q, cE, o)); }
-        else { if (keepTopo) put_edge(D.E, en, p, q, pid); fluxN.add(edge_term(p, q, cE, o)); }
+        const float f = edge_term(p, q, cE, o);
+        if (sp) { if (keepTopo) put_edge(D.E, ep, p, q, pid); fp = f; hasP = true; }
+        else { if (keepTopo) put_edge(D.E, en, p, q, pid); fn = f; hasN = true; }
       } else {
         float tt = dp / (dp - dq);
         f3 x = p + tt * (q - p);
+        const float f0 = edge_term(p, x, cE, o), f1 = edge_term(x, q, cE, o);
         if (sp) {
           if (keepTopo) { put_edge(D.E, ep, p, x, pid); put_edge(D.E, en, x, q, pid); }
-          fluxP.add(edge_term(p, x, cE, o));
-          fluxN.add(edge_term(x, q, cE, o));
+          fp = f0;
+          fn = f1;
         } else {
           if (keepTopo) { put_edge(D.E, en, p, x, pid); put_edge(D.E, ep, x, q, pid); }
-          fluxN.add(edge_term(p, x, cE, o));
-          fluxP.add(edge_term(x, q, cE, o));
+          fn = f0;
+          fp = f1;
         }
+        hasP = hasN = true;
       }
     }
+    add_flux(fp, hasP, fn, hasN);
     rE[0] += totP;
     rE[1] += totN;
   }
-  double vp = grp_sum_d<G>(fluxP.value(), sm);
-  double vn = grp_sum_d<G>(fluxN.value(), sm);
+  double vp, vn;
+  if constexpr (STAGED) {
+    const double v = warp_sum_d(lid < 32 ? fluxP.value() : fluxN.value());
+    if (lid == 0) sm.d[0] = v;
+    if (lid == 32) sm.d[1] = v;
+    __syncthreads();
+    vp = sm.d[0];
+    vn = sm.d[1];
+  } else {
+    vp = grp_sum_d<G>(fluxP.value(), sm);
+    vn = grp_sum_d<G>(fluxN.value(), sm);
+  }
   if (lid == 0) {
     unsigned long long b = 12ull * part.nv + 12ull * part.nt + 32ull * part.ne + 12ull * (J->cnt[0] + J->cnt[3]);
     if (keepTopo) b += 12ull * (J->cnt[1] + J->cnt[4]) + 32ull * (J->cnt[2] + J->cnt[5]);
@@ -760,10 +807,11 @@ void launch_scan(const Level& P, const Dev& D, cudaStream_t s) {
   k_scan_sums<<<blocks, 1024, 0, s>>>(P, D);
   k_scan<<<blocks, 1024, 0, s>>>(P, D);
 }
-void launch_emit(const Level& P, const Dev& D, bool big, cudaStream_t s) {
+void launch_emit(const Level& P, const Dev& D, bool big, bool wide, cudaStream_t s) {
   if (P.nJobs == 0) return;
-  if (big) k_emit<256><<<P.nJobs, 256, 0, s>>>(P, D);
-  else k_emit<32><<<(P.nJobs + 7) / 8, 256, 0, s>>>(P, D);
+  if (big) k_emit<256, 256><<<P.nJobs, 256, 0, s>>>(P, D);
+  else if (wide) k_emit<256, 32><<<P.nJobs, 256, 0, s>>>(P, D);
+  else k_emit<32, 32><<<(P.nJobs + 7) / 8, 256, 0, s>>>(P, D);
 }
 void launch_record(const Level& P, const Dev& D, cudaStream_t s) {
   if (P.nJobs == 0) return;
