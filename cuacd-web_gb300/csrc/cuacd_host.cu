@@ -33,6 +33,7 @@ void launch_seed_bound(const Level& P, const Dev& D, cudaStream_t s);
 void launch_evaluate(uint32_t stateBase, uint32_t headerOff, uint32_t mode, uint32_t nSeeds, uint32_t jobBase,
                      uint32_t edgePlaneBase, uint32_t edgeStride, const Dev& D, cudaStream_t s);
 void launch_hull(const Level& P, const Dev& D, int width, cudaStream_t s);
+void launch_hd_area(uint32_t nMeshes, uint32_t maxNt, const Dev& D, double2* out, cudaStream_t s);
 void launch_hd(const HdArgs& A, const Dev& D, int nSM, cudaStream_t s);
 int hull_blocks_per_sm(int width);
 }  // namespace cuacd
@@ -73,6 +74,10 @@ static const uint32_t SMALL_NV = 1024;
 static const uint32_t WIDE_JOBS = 16, WIDE_NV = 128;
 // Hausdorff targets with at least this many triangles are searched by clusters
 static const uint32_t HD_SCREEN_MIN = 64;
+// Hausdorff batches of at least this many triangles have the areas that their
+// sample capacities follow from added on the device (k_hd_area, about 40 us
+// with its readback); smaller ones on the host, at 3.4 ns a triangle
+static const uint64_t HD_AREA_MIN = 16384;
 // parents with more points than this get a block per plan / emit job
 static const uint32_t BIG_JOB_NV = 2048;
 
@@ -714,14 +719,15 @@ struct Tree {
     uint32_t stride = doExport ? 3 * 2 * std::min<uint32_t>((uint32_t)cfg.hullMaxVerts, maxNv) : 0;
     if ((uint64_t)tTop + (uint64_t)n * stride > cfg.triCap) return fail(CUACD_E_CAPACITY, "hull export exceeds triangle pool");
     // sample scratch of the fused Hausdorff (tree.ts:686-698)
+    CK(cudaMemcpyAsync(D.parts, parts.data(), (size_t)n * sizeof(PartDesc), cudaMemcpyHostToDevice, stream));
     std::vector<uint32_t> capN;
     if (withHd) {
+      std::vector<uint64_t> res;
+      if ((rc = sampleRes(m, (uint32_t)n, res))) return rc;
       capN.resize(2 * n);
       uint64_t off = 0;
       for (int k = 0; k < n; k++) {
-        double area = mesh_area(host_side(m, (size_t)k));
-        uint64_t res = std::max<uint64_t>(1000, (uint64_t)std::floor(2000.0 * area));
-        uint64_t cap = 2 * (2 * res + std::max<uint64_t>(m[k].nt, 2ull * m[k].nv) + 16);
+        uint64_t cap = 2 * (2 * res[k] + std::max<uint64_t>(m[k].nt, 2ull * m[k].nv) + 16);
         if (3 * (off + cap) > cfg.scratchWords) return fail(CUACD_E_SCRATCH, "hausdorff sample scratch exceeds capacity");
         uint32_t ca = (uint32_t)(cap / 2), cb = (uint32_t)(cap - cap / 2);
         capN[k] = ca;
@@ -729,7 +735,6 @@ struct Tree {
         off += cap;
       }
     }
-    CK(cudaMemcpyAsync(D.parts, parts.data(), (size_t)n * sizeof(PartDesc), cudaMemcpyHostToDevice, stream));
     if (withHd) CK(cudaMemsetAsync(D.parts + n, 0, (size_t)n * sizeof(PartDesc), stream));
     CK(cudaMemsetAsync(D.ctr, 0, CTR_WORDS * 4, stream));
     Level P = baseLevel(true);
@@ -831,6 +836,45 @@ struct Tree {
     }
     return area;
   }
+  // res[k] = max(1000, floor(2000 * mesh_area)) of every mesh, the samples its
+  // capacity follows from. The meshes lie in the pools and D.parts. A large
+  // batch's areas are added on the device, with a bound on how far they are
+  // from mesh_area's (its serial sum is off by nt rounding errors at most);
+  // a mesh whose floor that leaves open is added here.
+  int sampleRes(const cuacd_mesh* m, uint32_t n, std::vector<uint64_t>& res) {
+    auto samples = [](double area) { return std::max<uint64_t>(1000, (uint64_t)std::floor(2000.0 * area)); };
+    uint64_t nt = 0;
+    uint32_t maxNt = 0;
+    for (uint32_t k = 0; k < n; k++) {
+      nt += m[k].nt;
+      maxNt = std::max(maxNt, m[k].nt);
+    }
+    res.resize(n);
+    const double2* area = nullptr;
+    if (nt >= HD_AREA_MIN) {
+      const size_t bytes = n * sizeof(double2);
+      int rc;
+      if ((rc = bHd.ensure(bytes)) || (rc = hMeta.ensure(bytes))) return rc;
+      CK(cudaMemsetAsync(bHd.p, 0, bytes, stream));
+      launch_hd_area(n, maxNt, D, (double2*)bHd.p, stream);
+      CK(cudaGetLastError());
+      CK(cudaMemcpyAsync(hMeta.p, bHd.p, bytes, cudaMemcpyDeviceToHost, stream));
+      CK(cudaStreamSynchronize(stream));
+      area = (const double2*)hMeta.p;
+    }
+    for (uint32_t k = 0; k < n; k++) {
+      if (area) {
+        const double off = area[k].y + 3e-16 * m[k].nt * area[k].x;
+        const double lo = std::max(0.0, area[k].x - off), hi = area[k].x + off;
+        if (hi < 1e15 && samples(lo) == samples(hi)) {  // false for NaN and infinity
+          res[k] = samples(lo);
+          continue;
+        }
+      }
+      res[k] = samples(mesh_area(host_side(m, k)));
+    }
+    return 0;
+  }
   // triCap: per mesh, an upper bound on its triangles
   int runHd(uint32_t nPairs, uint32_t partBase, const std::vector<uint32_t>& capN, const std::vector<uint32_t>& triCap) {
     const uint32_t nm = 2 * nPairs;
@@ -908,21 +952,20 @@ struct Tree {
     for (int k = 0; k < n; k++) { all[k] = a[k]; all[n + k] = b[k]; }
     std::vector<PartDesc> parts;
     if ((rc = uploadMeshes(all.data(), 2 * n, parts))) return rc;
-    auto bound = [](const cuacd_mesh& m) {
-      uint64_t res = std::max<uint64_t>(1000, (uint64_t)std::floor(2000.0 * mesh_area(m)));
-      return 2 * res + m.nt + 16;
-    };
+    CK(cudaMemcpyAsync(D.parts, parts.data(), 2ull * n * sizeof(PartDesc), cudaMemcpyHostToDevice, stream));
+    std::vector<uint64_t> res;
+    if ((rc = sampleRes(all.data(), 2 * (uint32_t)n, res))) return rc;
+    auto bound = [&](int k) { return 2 * res[k] + all[k].nt + 16; };
     std::vector<uint32_t> capN(2 * n);
     uint64_t off = 0;
     for (int k = 0; k < n; k++) {
-      uint64_t cap = 2 * std::max(bound(a[k]), bound(b[k]));
+      uint64_t cap = 2 * std::max(bound(k), bound(n + k));
       if (3 * (off + cap) > cfg.scratchWords) return fail(CUACD_E_SCRATCH, "hausdorff sample scratch exceeds capacity");
       uint32_t ca = (uint32_t)(cap / 2), cb = (uint32_t)(cap - cap / 2);
       capN[k] = ca;
       capN[n + k] = cb;
       off += cap;
     }
-    CK(cudaMemcpyAsync(D.parts, parts.data(), 2ull * n * sizeof(PartDesc), cudaMemcpyHostToDevice, stream));
     CK(cudaMemsetAsync(D.ctr + CTR_HD, 0, 4ull * n, stream));
     CK(cudaEventRecord(ev0, stream));
     std::vector<uint32_t> triCap(2 * n);
