@@ -398,9 +398,8 @@ int engine_run(Engine* e, cudaStream_t s, const cuacd_mesh* meshes, int nMeshes,
     const bool dv = is_device_ptr(m.verts), dt = is_device_ptr(m.tris);
     if ((m.nv && m.nt && dv != dt) || (!m.nv && dt) || (!m.nt && dv))
       return set_error(CUACD_E_INVALID, "concave: a mesh's buffers must both be host or both be device memory");
-    if (!dt)
-      for (uint64_t k = 0; k < 3ull * m.nt; k++)
-        if (m.tris[k] >= m.nv) return set_error(CUACD_E_INVALID, "concave: triangle index out of range");
+    if (!dt && !indices_below(m.tris, 3ull * m.nt, m.nv))
+      return set_error(CUACD_E_INVALID, "concave: triangle index out of range");
     MeshDesc& d = desc[i];
     d.vOff = (uint32_t)totV;
     d.nv = m.nv;

@@ -411,12 +411,27 @@ struct Tree {
     }
     if (anyHost && totV) CK(cudaMemcpyAsync(D.V, hv, totV * 4, cudaMemcpyHostToDevice, stream));
     if (anyHost && totT) CK(cudaMemcpyAsync(D.T, ht, totT * 4, cudaMemcpyHostToDevice, stream));
-    for (uint32_t k = 0; k < n; k++) {
+    // device meshes one by one; neighbours in the cut engine's buffers, which
+    // become neighbours here, in one copy (192 halves were 384 copies)
+    const float* cv = nullptr;
+    const uint32_t* ct = nullptr;
+    size_t cvWords = 0, ctWords = 0;
+    if (cutter) cut::engine_outputs(cutter, &cv, &cvWords, &ct, &ctWords);
+    auto follows = [](const auto* a, size_t words, const auto* b, size_t next, const auto* buf, size_t bufWords) {
+      return buf && b == a + words && a >= buf && b + next <= buf + bufWords;
+    };
+    for (uint32_t k = 0, e; k < n; k = e) {
+      e = k + 1;
       if (!dev[k]) continue;
-      if (m[k].nv)
-        CK(cudaMemcpyAsync(D.V + parts[k].vOff, m[k].verts, 12ull * m[k].nv, cudaMemcpyDeviceToDevice, stream));
-      if (m[k].nt)
-        CK(cudaMemcpyAsync(D.T + parts[k].tOff, m[k].tris, 12ull * m[k].nt, cudaMemcpyDeviceToDevice, stream));
+      size_t vw = 3ull * m[k].nv, tw = 3ull * m[k].nt;
+      for (; e < n && dev[e] && follows(m[k].verts, vw, m[e].verts, 3ull * m[e].nv, cv, cvWords) &&
+             follows(m[k].tris, tw, m[e].tris, 3ull * m[e].nt, ct, ctWords);
+           e++) {
+        vw += 3ull * m[e].nv;
+        tw += 3ull * m[e].nt;
+      }
+      if (vw) CK(cudaMemcpyAsync(D.V + parts[k].vOff, m[k].verts, 4 * vw, cudaMemcpyDeviceToDevice, stream));
+      if (tw) CK(cudaMemcpyAsync(D.T + parts[k].tOff, m[k].tris, 4 * tw, cudaMemcpyDeviceToDevice, stream));
     }
     vTop = vt;
     tTop = tt;
@@ -1190,6 +1205,23 @@ int cuacd_cuts_half(const void* halves, int cut, int side, const float** verts, 
   return st;
 }
 
+int cuacd_cuts_all(const void* halves, int32_t* status, const float** verts, uint32_t* nv, const uint32_t** tris,
+                   uint32_t* nt) {
+  const cut::Halves* h = (const cut::Halves*)halves;
+  if (!h || !status || !verts || !nv || !tris || !nt) return fail(CUACD_E_INVALID, "cuacd_cuts_all: invalid argument");
+  for (size_t c = 0; c < h->status.size(); c++) {
+    status[c] = h->status[c];
+    for (size_t k = 2 * c; k < 2 * c + 2; k++) {
+      const bool ok = h->status[c] == 0;
+      verts[k] = ok ? h->V + 3 * h->vOff[k] : nullptr;
+      tris[k] = ok ? h->T + 3 * h->tOff[k] : nullptr;
+      nv[k] = ok ? h->nv[k] : 0;
+      nt[k] = ok ? h->nt[k] : 0;
+    }
+  }
+  return CUACD_OK;
+}
+
 int cuacd_cuts_half_device(const void* halves, int cut, int side, const float** verts, const uint32_t** tris) {
   const cut::Halves* h = (const cut::Halves*)halves;
   if (!h || cut < 0 || (size_t)cut >= h->status.size() || side < 0 || side > 1)
@@ -1213,13 +1245,18 @@ int cuacd_tree_eval_cuts(void* tree, const cuacd_mesh* mesh, const double* plane
   cut::Halves* h = (cut::Halves*)hv;
   float ms = h->gpuMs;
   // every half of every cut that split, hulled with its Hausdorff distance
-  std::vector<cuacd_mesh> halves;
+  std::vector<cuacd_mesh> halves, twins;  // on the device, and their host copies
   std::vector<int> owner;
   for (int k = 0; k < n; k++) {
     if (h->status[k] != 0) continue;
     for (int sd = 0; sd < 2; sd++) {
       const size_t i = 2 * (size_t)k + sd;
-      halves.push_back(cuacd_mesh{h->V + 3 * h->vOff[i], h->T + 3 * h->tOff[i], h->nv[i], h->nt[i]});
+      twins.push_back(cuacd_mesh{h->V + 3 * h->vOff[i], h->T + 3 * h->tOff[i], h->nv[i], h->nt[i]});
+      halves.push_back(twins.back());
+      if (h->nv[i] && h->nt[i]) {
+        halves.back().verts = h->dV + 3 * h->vOff[i];
+        halves.back().tris = h->dT + 3 * h->tOff[i];
+      }
       owner.push_back(2 * k + sd);
     }
   }
@@ -1230,6 +1267,7 @@ int cuacd_tree_eval_cuts(void* tree, const cuacd_mesh* mesh, const double* plane
   size_t batch = std::min<size_t>(nh, CUACD_HD_MAX_PAIRS);
   for (size_t s0 = 0; s0 < nh;) {
     const size_t m = std::min(batch, nh - s0);
+    t->twins.assign(twins.begin() + s0, twins.begin() + s0 + m);
     rc = t->hulls(halves.data() + s0, (int)m, 0, nullptr, 0, vol.data() + s0, nt.data() + s0, st.data() + s0,
                   hd.data() + s0);
     if (rc == CUACD_E_SCRATCH && m > 1) {  // halve the batch, as merge.ts:405 does

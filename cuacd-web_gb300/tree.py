@@ -80,6 +80,8 @@ def load_library():
                                         C.c_int, P(C.c_void_p)]
     L.cuacd_cuts_half.argtypes = [C.c_void_p, C.c_int, C.c_int, P(P(C.c_float)), P(C.c_uint32), P(P(C.c_uint32)),
                                   P(C.c_uint32)]
+    L.cuacd_cuts_all.argtypes = [C.c_void_p, P(C.c_int32), P(P(C.c_float)), P(C.c_uint32), P(P(C.c_uint32)),
+                                 P(C.c_uint32)]
     L.cuacd_cuts_gpu_ms.restype = C.c_float
     L.cuacd_cuts_gpu_ms.argtypes = [C.c_void_p]
     L.cuacd_cuts_free.argtypes = [C.c_void_p]
@@ -251,11 +253,11 @@ class GpuTree:
         _check(load_library().cuacd_tree_hull_meshes(self.h, ma.arr, n, hull_stage, None if no_export else A.uptr(tris),
                                                      stride, A.fptr(vol), A.uptr(nt), _int32p(status)))
         out = []
-        for i in range(n):
-            if status[i] != 0:
+        for i, (st, k, vo) in enumerate(zip(status.tolist(), nt.tolist(), vol.tolist())):
+            if st != 0:
                 out.append(None)
             else:
-                out.append(dict(tris=tris[i * stride: i * stride + 3 * nt[i]].reshape(-1, 3).copy(), volume=float(vol[i])))
+                out.append(dict(tris=tris[i * stride: i * stride + 3 * k].reshape(-1, 3).copy(), volume=vo))
         return out, status
 
     # ---- GpuTree.hullsWithHausdorff (tree.ts:671-756) ----
@@ -278,12 +280,11 @@ class GpuTree:
                                                               A.uptr(nt), A.fptr(hd), _int32p(status)))
         self.last_hull_fails = [int(s) for s in status]
         out = []
-        for i in range(n):
-            if status[i] != 0:
+        for i, (st, k, vo, h) in enumerate(zip(status.tolist(), nt.tolist(), vol.tolist(), hd.tolist())):
+            if st != 0:
                 out.append(None)
             else:
-                out.append(dict(tris=tris[i * stride: i * stride + 3 * nt[i]].reshape(-1, 3).copy(), volume=float(vol[i]),
-                                hausdorff=float(hd[i])))
+                out.append(dict(tris=tris[i * stride: i * stride + 3 * k].reshape(-1, 3).copy(), volume=vo, hausdorff=h))
         return out
 
     # ---- GpuTree.hausdorff (tree.ts:318-372) ----
@@ -321,23 +322,26 @@ class GpuTree:
         out = []
         try:
             self.last_cut_ms = float(L.cuacd_cuts_gpu_ms(h))
-            for k in range(n):
-                halves = []
-                st = 0
-                for side in (0, 1):
-                    v = C.POINTER(C.c_float)()
-                    t = C.POINTER(C.c_uint32)()
-                    nv = C.c_uint32()
-                    nt = C.c_uint32()
-                    st = L.cuacd_cuts_half(h, k, side, C.byref(v), C.byref(nv), C.byref(t), C.byref(nt))
-                    if st < 0:
-                        _check(st)
-                    if st != 0:
-                        break
-                    vv = np.ctypeslib.as_array(v, shape=(nv.value * 3,)).copy() if nv.value else np.zeros(0, np.float32)
-                    tt = np.ctypeslib.as_array(t, shape=(nt.value * 3,)).copy() if nt.value else np.zeros(0, np.uint32)
-                    halves.append(Mesh(vv.reshape(-1, 3), tt.reshape(-1, 3)))
-                out.append((st, halves[0], halves[1]) if st == 0 else (st, None, None))
+            status = np.zeros(max(n, 1), np.int32)
+            verts, tris = np.zeros((2, max(2 * n, 1)), np.uintp)
+            nv, nt = np.zeros((2, max(2 * n, 1)), np.uint32)
+            pp = C.POINTER(C.POINTER(C.c_float)), C.POINTER(C.POINTER(C.c_uint32))
+            _check(L.cuacd_cuts_all(h, _int32p(status), verts.ctypes.data_as(pp[0]), A.uptr(nv),
+                                    tris.ctypes.data_as(pp[1]), A.uptr(nt)))
+            # one view of the buffer all halves lie in; each half is a copy of its own
+            used = nv > 0
+            lo = int(verts[used].min()) if used.any() else 0
+            end = int((tris + 12 * nt.astype(np.uintp))[used].max()) if used.any() else 0
+            words = np.frombuffer((C.c_uint32 * ((end - lo) // 4)).from_address(lo), np.uint32) if end > lo else None
+
+            def rows(p, k, dtype):
+                return words[(p - lo) // 4: (p - lo) // 4 + 3 * k].view(dtype).reshape(-1, 3).copy() if k else \
+                    np.zeros((0, 3), dtype)
+
+            halves = [Mesh(rows(pv, kv, np.float32), rows(pt, kt, np.uint32))
+                      for pv, kv, pt, kt in zip(verts.tolist(), nv.tolist(), tris.tolist(), nt.tolist())]
+            for k, st in enumerate(status[:n].tolist()):
+                out.append((0, halves[2 * k], halves[2 * k + 1]) if st == 0 else (st, None, None))
         finally:
             L.cuacd_cuts_free(h)
         return out

@@ -298,6 +298,11 @@ int cuacd_tree_plane_cuts(void* tree, const cuacd_mesh* meshes, int nMeshes, con
  * scratch bound was exceeded; or a negative error. */
 int cuacd_cuts_half(const void* halves, int cut, int side, const float** verts, uint32_t* nv, const uint32_t** tris,
                     uint32_t* nt);
+/* Every half of the batch at once: status of the nCuts cuts as above, and the
+ * arrays of half `side` of cut k at entry 2k + side (null and 0 where the cut
+ * failed). All of them lie in one allocation, the vertices first. */
+int cuacd_cuts_all(const void* halves, int32_t* status, const float** verts, uint32_t* nv, const uint32_t** tris,
+                   uint32_t* nt);
 /* The same half in device memory (no counterpart in the reference): the
  * GPU cut's output buffers keep every half of the batch until the next
  * cuacd_tree_plane_cuts (or cuacd_tree_eval_cuts) on the same handle, also
