@@ -2276,8 +2276,8 @@ __device__ __forceinline__ void hand_on(const Level& P, const Dev& D, uint32_t i
 
 // false (warp groups): the part was handed on
 template <int G>
-__device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* slab, HullSm& hs, GrpSmem& sm,
-                         float4* qcache, TinySm* ts, BatSm<(G >= 256 ? G / 32 : 8)>* bs) {
+__device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* slab, HullCtx& ctx, HullSm& hs,
+                         GrpSmem& sm, float4* qcache, TinySm* ts, BatSm<(G >= 256 ? G / 32 : 8)>* bs) {
   const int lid = Grp<G>::lid();
   const uint32_t partIdx = P.partBase + idx;
   PartDesc* pdp = D.parts + partIdx;
@@ -2300,27 +2300,27 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
     return true;
   }
   if (lid == 0) add_bytes(D.ctr, CTR_BYTES_HULL, 12ull * nv);
-  HullCtx h;
-  h.qc = nullptr;
-  h.V = D.V; h.vOff = vOff; h.nv = nv; h.fmax = fmax;
-  h.owner = slab;
-  h.dist = reinterpret_cast<float*>(slab + nv);
-  h.cand = slab + 2 * nv;
-  h.F = slab + fb;
+  HullCtx c;
+  c.qc = nullptr;
+  c.V = D.V; c.vOff = vOff; c.nv = nv; c.fmax = fmax;
+  c.owner = slab;
+  c.dist = reinterpret_cast<float*>(slab + nv);
+  c.cand = slab + 2 * nv;
+  c.F = slab + fb;
   // after the reference's slab words (which fix fmax): visible list, walk
   // queue, adjacency, the faces' keys and segments, bitmap, word prefix,
   // horizon maps (hull_slab_stride)
-  h.vis = slab + P.hullSlabWords;
-  h.q = h.vis + HULL_VIS_MAX;
-  h.nbr = h.q + HULL_VIS_MAX;
+  c.vis = slab + P.hullSlabWords;
+  c.q = c.vis + HULL_VIS_MAX;
+  c.nbr = c.q + HULL_VIS_MAX;
   const uint32_t nw = (fmax + 31) / 32;
-  h.fkey = reinterpret_cast<unsigned long long*>(h.nbr + 4 * (size_t)fmax);
-  h.fseg = reinterpret_cast<uint2*>(h.fkey + fmax);
-  h.bm = h.nbr + 8 * (size_t)fmax;
-  h.wp = h.bm + nw;
-  h.hA = h.wp + nw;
-  h.hB = h.hA + nv;
-  for (uint32_t w = lid; w < nw; w += G) h.bm[w] = 0;
+  c.fkey = reinterpret_cast<unsigned long long*>(c.nbr + 4 * (size_t)fmax);
+  c.fseg = reinterpret_cast<uint2*>(c.fkey + fmax);
+  c.bm = c.nbr + 8 * (size_t)fmax;
+  c.wp = c.bm + nw;
+  c.hA = c.wp + nw;
+  c.hB = c.hA + nv;
+  for (uint32_t w = lid; w < nw; w += G) c.bm[w] = 0;
   // quantisation grid: 2^21 cells across the largest extent
   f3 lo = mk3(1e30f, 1e30f, 1e30f), hi = mk3(-1e30f, -1e30f, -1e30f);
   for (uint32_t i = lid; i < nv; i += G) {
@@ -2332,34 +2332,37 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   hi.x = grp_max_f<G>(hi.x, sm); hi.y = grp_max_f<G>(hi.y, sm); hi.z = grp_max_f<G>(hi.z, sm);
   const f3 ext = hi - lo;
   const float scale = fmaxf(fmaxf(fmaxf(ext.x, ext.y), ext.z), 1e-30f);
-  h.qlo = lo;
-  h.qs = 2097152.0f / scale;
+  c.qlo = lo;
+  c.qs = 2097152.0f / scale;
   const float cell = scale / 2097152.0f;
   const float volScale = (cell * cell) * cell;
   // small parts keep their quantised points in shared memory
   if (G == 32 && qcache != nullptr && nv <= QC_MAX) {
     for (uint32_t i = lid; i < nv; i += G) {
       f3 v = ldv(D.V, (size_t)vOff + 3 * (size_t)i) - lo;
-      qcache[i] = make_float4(rintf(v.x * h.qs), rintf(v.y * h.qs), rintf(v.z * h.qs), 0.0f);
+      qcache[i] = make_float4(rintf(v.x * c.qs), rintf(v.y * c.qs), rintf(v.z * c.qs), 0.0f);
     }
-    h.qc = qcache;
-    Grp<G>::sync();
+    c.qc = qcache;
   }
   if constexpr (G >= 256) {
     // the block path keeps them in the slab where its words hold them too
     // (always when the hull bound covers the part): one 16-byte load instead
     // of three and the rounding, in every pass and every new face
-    const uint64_t at = ((uint64_t)(h.hB - slab) + nv + 3) & ~3ull;
+    const uint64_t at = ((uint64_t)(c.hB - slab) + nv + 3) & ~3ull;
     if (at + 4ull * nv <= P.slabStride) {
       float4* qp = reinterpret_cast<float4*>(slab + at);
       for (uint32_t i = lid; i < nv; i += G) {
-        const f3 v = h.qvert(i);
+        const f3 v = c.qvert(i);
         qp[i] = make_float4(v.x, v.y, v.z, 0.0f);
       }
-      h.qc = qp;
-      Grp<G>::sync();
+      c.qc = qp;
     }
   }
+  // what every step below reads, one copy per group: a copy per thread in local
+  // memory (the steps are calls) took 200 KB of an SM's L1
+  if (lid == 0) ctx = c;
+  const HullCtx& h = ctx;
+  Grp<G>::sync();
   // 80 seeds: max and min along 40 axes, lowest index on ties; seed 2a is
   // the maximum along axis a, seed 2a + 1 the minimum
   if (G == 32 && h.qc != nullptr) {
@@ -2473,8 +2476,9 @@ restart:
       if (lid == 2) h.face_write(2, b, i3, c);
       if (lid == 3) h.face_write(3, c, i3, a);
       // faces across each edge of the tetrahedron
-      const uint4 nb[4] = {make_uint4(1, 2, 3, 0), make_uint4(3, 2, 0, 0), make_uint4(1, 3, 0, 0), make_uint4(2, 1, 0, 0)};
-      *reinterpret_cast<uint4*>(h.nbr + 4 * lid) = nb[lid];
+      *reinterpret_cast<uint4*>(h.nbr + 4 * lid) =
+          lid == 0 ? make_uint4(1, 2, 3, 0)
+                   : (lid == 1 ? make_uint4(3, 2, 0, 0) : (lid == 2 ? make_uint4(1, 3, 0, 0) : make_uint4(2, 1, 0, 0)));
     }
     if (lid == 0) {
       hs.fail = 0;
@@ -2688,6 +2692,7 @@ __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 
     k_hull(const Level P, const Dev D) {
   __shared__ GrpSmem gsm[Grp<G>::PER_BLOCK];
   __shared__ HullSm hsm[Grp<G>::PER_BLOCK];
+  __shared__ HullCtx hcx[Grp<G>::PER_BLOCK];
   __shared__ float4 qcs[G == 32 ? 8 * QC_MAX : 1];
   __shared__ TinySm tsm[G == 32 ? 8 : 1];
   // the block path's shared words (BatSm) in the launch's dynamic shared memory
@@ -2706,7 +2711,7 @@ __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 
       if (threadIdx.x == 0) k = atomicAdd(D.work + 16 + P.workSlot, 1u);
       k = grp_bcast_u<G>(k, gsm[0]);
       if (k >= n) break;
-      hull_one<G>(P, D, D.list[k], slab, hsm[gi], gsm[gi], nullptr, nullptr, reinterpret_cast<BS*>(hull_dyn));
+      hull_one<G>(P, D, D.list[k], slab, hcx[gi], hsm[gi], gsm[gi], nullptr, nullptr, reinterpret_cast<BS*>(hull_dyn));
       Grp<G>::sync();
     }
     return;
@@ -2723,7 +2728,7 @@ __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 
       const uint32_t nv = D.parts[P.partBase + idx].nv;
       bool done = nv <= P.smallNv && !(P.handOn && nv > QC_MAX);
       if (done) {
-        done = hull_one<G>(P, D, idx, slab, hsm[gi], gsm[gi], qcs + gi * QC_MAX, tsm + gi, nullptr);
+        done = hull_one<G>(P, D, idx, slab, hcx[gi], hsm[gi], gsm[gi], qcs + gi * QC_MAX, tsm + gi, nullptr);
         if (!done && lane == 0) add_bytes(D.ctr, CTR_BYTES_HULL, 0ull - 12ull * nv);  // the block counts it
       }
       if (!done && lane == 0) hand_on(P, D, idx);
