@@ -66,11 +66,11 @@ static const uint32_t SMALL_NV = 1024;
 // A level of at most WIDE_JOBS jobs per SM, or whose parents have WIDE_NV
 // points or more, plans and emits a job on a block, with the warp form's sums
 // (k_emit<256, 32>): a warp per job leaves the GPU idle there. Plan + emit of a
-// depth-2 run, warps against blocks: one blob of 120 points 0.58 and 0.20 ms,
-// of 1,678 points 5.2 and 1.06 ms; 16 of 220 points (1,120 and 3,360 jobs) 1.07
-// and 0.62; 64 of 818 points (13,440 jobs) 6.5 and 5.0; depth-3 staircases of 96
-// points, 8 of them 0.78 and 0.49, 40 (25,200 jobs) 1.26 and 1.48, 160 (100,800
-// jobs) 3.4 and 5.3.
+// run, warps against blocks: depth 2, one blob of 120 points 0.33 and 0.14 ms,
+// of 1,678 points 2.46 and 0.49; 16 of 220 points (1,120 and 3,360 jobs) 0.55
+// and 0.34; 64 (13,440 jobs) of 254 points 0.89 and 0.86, of 818 points 3.04 and
+// 2.38; depth-3 staircases of 96 points, 8 of them 0.46 and 0.34, 40 (25,200
+// jobs) 0.71 and 0.97, 160 (100,800 jobs) 1.92 and 3.44.
 static const uint32_t WIDE_JOBS = 16, WIDE_NV = 128;
 // Hausdorff targets with at least this many triangles are searched by clusters
 static const uint32_t HD_SCREEN_MIN = 64;
