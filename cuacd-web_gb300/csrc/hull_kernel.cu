@@ -99,11 +99,7 @@ __device__ __forceinline__ int orient_filtered(f3 n, f3 e1, f3 e2, f3 d) {
 }
 
 struct HullCtx {
-  const float* V;
-  uint32_t vOff, nv;
-  f3 qlo;
-  float qs;
-  uint32_t fmax;
+  uint32_t nv, fmax;
   uint32_t* owner;
   float* dist;
   uint32_t* cand;
@@ -117,14 +113,10 @@ struct HullCtx {
   uint32_t* wp;    // compaction: alive faces before each bitmap word
   uint32_t* hA;    // per point: new face whose horizon edge starts there
   uint32_t* hB;    // per point: new face whose horizon edge ends there
-  const float4* qc;  // quantised points, one 16-byte load each (a warp's in shared
-                     // memory, a block's in its slab), or null
+  const float4* qc;  // quantised points, one 16-byte load each: a warp's small
+                     // part's in shared memory, else in the slab
 
-  __device__ __forceinline__ f3 qvert(uint32_t i) const {
-    if (qc) return xyz(qc[i]);
-    f3 v = ldv(V, (size_t)vOff + 3 * (size_t)i) - qlo;
-    return mk3(rintf(v.x * qs), rintf(v.y * qs), rintf(v.z * qs));
-  }
+  __device__ __forceinline__ f3 qvert(uint32_t i) const { return xyz(qc[i]); }
   __device__ __forceinline__ uint4* rec(uint32_t f) const { return reinterpret_cast<uint4*>(F + 16 * (size_t)f); }
   __device__ __forceinline__ bool alive(uint32_t f) const { return (F[16 * (size_t)f] & ALIVE) != 0; }
   __device__ __forceinline__ void abc(uint32_t f, uint32_t& a, uint32_t& b, uint32_t& c) const {
@@ -603,6 +595,7 @@ __device__ __noinline__ uint32_t hull_tiny_grow(const HullCtx& h, HullSm& hs, Ti
     const bool live = lane < nalive;
     const uint32_t V = __ballot_sync(FULLMASK, live && tiny_eval(h, F, pp, pick) > 0.0f);
     uint32_t C = 1u << start;
+#pragma unroll 1
     for (uint32_t it = 0; it < TINY_FACES; it++) {
       const bool nin = (((C >> (F.nb0 & 31u)) | (C >> (F.nb1 & 31u)) | (C >> (F.nb2 & 31u))) & 1u) != 0;
       const uint32_t C2 = C | __ballot_sync(FULLMASK, ((V >> lane) & 1u) && nin);
@@ -2163,6 +2156,7 @@ __device__ __noinline__ double hull_volume_grid(const HullCtx& h, HullSm& hs, Gr
   const long long ox = (long long)of.x, oy = (long long)of.y, oz = (long long)of.z;
   __int128 v6 = 0;
   const uint32_t nf = hs.nf;
+#pragma unroll 1
   for (uint32_t f = lid; f < nf; f += G) {
     if (!h.alive(f)) continue;
     uint32_t a, b, c;
@@ -2293,16 +2287,15 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
     if (lid == 0) { pdp->hullVol = -1.0f; pdp->flags = 3; atomicAdd(D.ctr + CTR_HULLFAIL, 1u); }
     return true;
   }
-  // the walk's arrays after the reference's slab words must fit the slab
-  // (always true for hull_slab_stride; checked so a slab is never overrun)
-  if ((uint64_t)P.hullSlabWords + 2 * HULL_VIS_MAX + 8ull * fmax + 2 * ((fmax + 31) / 32) + 2ull * nv > P.slabStride) {
+  // the walk's arrays and the grid points after the reference's slab words
+  // must fit the slab (they always do; checked so a slab is never overrun)
+  if (hull_slab_words(P.hullSlabWords, fmax, nv) > P.slabStride) {
     if (lid == 0) { pdp->hullVol = -1.0f; pdp->flags = 3; atomicAdd(D.ctr + CTR_HULLFAIL, 1u); }
     return true;
   }
   if (lid == 0) add_bytes(D.ctr, CTR_BYTES_HULL, 12ull * nv);
   HullCtx c;
-  c.qc = nullptr;
-  c.V = D.V; c.vOff = vOff; c.nv = nv; c.fmax = fmax;
+  c.nv = nv; c.fmax = fmax;
   c.owner = slab;
   c.dist = reinterpret_cast<float*>(slab + nv);
   c.cand = slab + 2 * nv;
@@ -2323,6 +2316,7 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   for (uint32_t w = lid; w < nw; w += G) c.bm[w] = 0;
   // quantisation grid: 2^21 cells across the largest extent
   f3 lo = mk3(1e30f, 1e30f, 1e30f), hi = mk3(-1e30f, -1e30f, -1e30f);
+#pragma unroll (G == 32 ? 1 : 4)
   for (uint32_t i = lid; i < nv; i += G) {
     f3 p = ldv(D.V, (size_t)vOff + 3 * (size_t)i);
     lo = vmin3(lo, p);
@@ -2332,31 +2326,19 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   hi.x = grp_max_f<G>(hi.x, sm); hi.y = grp_max_f<G>(hi.y, sm); hi.z = grp_max_f<G>(hi.z, sm);
   const f3 ext = hi - lo;
   const float scale = fmaxf(fmaxf(fmaxf(ext.x, ext.y), ext.z), 1e-30f);
-  c.qlo = lo;
-  c.qs = 2097152.0f / scale;
+  const float qs = 2097152.0f / scale;
   const float cell = scale / 2097152.0f;
   const float volScale = (cell * cell) * cell;
-  // small parts keep their quantised points in shared memory
-  if (G == 32 && qcache != nullptr && nv <= QC_MAX) {
+  // the points on the grid, a warp's small part's in shared memory
+  {
+    const bool inSm = G == 32 && nv <= QC_MAX;
+    float4* qp = inSm ? qcache : reinterpret_cast<float4*>(slab + (((uint64_t)(c.hB - slab) + nv + 3) & ~3ull));
+#pragma unroll (G == 32 ? 1 : 4)
     for (uint32_t i = lid; i < nv; i += G) {
-      f3 v = ldv(D.V, (size_t)vOff + 3 * (size_t)i) - lo;
-      qcache[i] = make_float4(rintf(v.x * c.qs), rintf(v.y * c.qs), rintf(v.z * c.qs), 0.0f);
+      const f3 v = ldv(D.V, (size_t)vOff + 3 * (size_t)i) - lo;
+      qp[i] = make_float4(rintf(v.x * qs), rintf(v.y * qs), rintf(v.z * qs), 0.0f);
     }
-    c.qc = qcache;
-  }
-  if constexpr (G >= 256) {
-    // the block path keeps them in the slab where its words hold them too
-    // (always when the hull bound covers the part): one 16-byte load instead
-    // of three and the rounding, in every pass and every new face
-    const uint64_t at = ((uint64_t)(c.hB - slab) + nv + 3) & ~3ull;
-    if (at + 4ull * nv <= P.slabStride) {
-      float4* qp = reinterpret_cast<float4*>(slab + at);
-      for (uint32_t i = lid; i < nv; i += G) {
-        const f3 v = c.qvert(i);
-        qp[i] = make_float4(v.x, v.y, v.z, 0.0f);
-      }
-      c.qc = qp;
-    }
+    c.qc = qp;
   }
   // what every step below reads, one copy per group: a copy per thread in local
   // memory (the steps are calls) took 200 KB of an SM's L1
@@ -2365,62 +2347,37 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   Grp<G>::sync();
   // 80 seeds: max and min along 40 axes, lowest index on ties; seed 2a is
   // the maximum along axis a, seed 2a + 1 the minimum
-  if (G == 32 && h.qc != nullptr) {
+  if constexpr (G == 32) {
     // one lane per axis for the first 32, each scanning every point in index
     // order; the last 8 axes take 4 lanes each, a quarter of the points a lane
     // (two full scans for 40 axes cost 4 % of a staircase child's hull)
-    auto scan = [&](uint32_t a, uint32_t i0, uint32_t i1, float& mx, float& mn, uint32_t& ix, uint32_t& in) {
+#pragma unroll 1
+    for (uint32_t pass = 0; pass < 2; pass++) {
+      const uint32_t part = pass ? lid & 3 : 0, parts = pass ? 4 : 1, a = pass ? 32 + (lid >> 2) : lid;
       const f3 ax = mk3(c_kdop[a][0], c_kdop[a][1], c_kdop[a][2]);
-      mx = -1e30f;
-      mn = 1e30f;
-      ix = in = 0;
-      for (uint32_t i = i0; i < i1; i++) {
+      float mx = -1e30f, mn = 1e30f;
+      uint32_t ix = 0, in = 0;
+      const uint32_t i1 = nv * (part + 1) / parts;
+      for (uint32_t i = nv * part / parts; i < i1; i++) {
         const float d = dot(ax, h.qvert(i));
         if (d > mx) { mx = d; ix = i; }
         if (d < mn) { mn = d; in = i; }
       }
-    };
-    float mx, mn;
-    uint32_t ix, in;
-    scan(lid, 0, nv, mx, mn, ix, in);
-    hs.seed[2 * lid] = ix;
-    hs.seed[2 * lid + 1] = in;
-    const uint32_t a = 32 + (lid >> 2), part = lid & 3;
-    scan(a, nv * part / 4, nv * (part + 1) / 4, mx, mn, ix, in);
 #pragma unroll
-    for (int o = 1; o < 4; o <<= 1) {  // quarters in order: a tie keeps the lower point
-      const float mx2 = __shfl_xor_sync(FULLMASK, mx, o), mn2 = __shfl_xor_sync(FULLMASK, mn, o);
-      const uint32_t ix2 = __shfl_xor_sync(FULLMASK, ix, o), in2 = __shfl_xor_sync(FULLMASK, in, o);
-      if (mx2 > mx || (mx2 == mx && ix2 < ix)) { mx = mx2; ix = ix2; }
-      if (mn2 < mn || (mn2 == mn && in2 < in)) { mn = mn2; in = in2; }
+      for (uint32_t o = 1; o < 4; o <<= 1) {  // quarters in order: a tie keeps the lower point
+        const float mx2 = __shfl_xor_sync(FULLMASK, mx, o), mn2 = __shfl_xor_sync(FULLMASK, mn, o);
+        const uint32_t ix2 = __shfl_xor_sync(FULLMASK, ix, o), in2 = __shfl_xor_sync(FULLMASK, in, o);
+        if (pass && (mx2 > mx || (mx2 == mx && ix2 < ix))) { mx = mx2; ix = ix2; }
+        if (pass && (mn2 < mn || (mn2 == mn && in2 < in))) { mn = mn2; in = in2; }
+      }
+      if (part == 0) {
+        hs.seed[2 * a] = ix;
+        hs.seed[2 * a + 1] = in;
+      }
     }
-    if (part == 0) {
-      hs.seed[2 * a] = ix;
-      hs.seed[2 * a + 1] = in;
-    }
-  } else if constexpr (G >= 256) {
+  } else {
     static_assert(sizeof(KdopSm<G / 32>) <= sizeof(*bs), "the seeds' words overlay the rounds' words");
     kdop_block<G / 32>(h, hs, *reinterpret_cast<KdopSm<G / 32>*>(bs));
-  } else {
-    for (int ps = 0; ps < 20; ps++) {
-      const f3 a0 = mk3(c_kdop[2 * ps][0], c_kdop[2 * ps][1], c_kdop[2 * ps][2]);
-      const f3 a1 = mk3(c_kdop[2 * ps + 1][0], c_kdop[2 * ps + 1][1], c_kdop[2 * ps + 1][2]);
-      float mx0 = -1e30f, mx1 = -1e30f, mn0 = -1e30f, mn1 = -1e30f;  // mins stored negated
-      uint32_t ix0 = CUACD_NONE, ix1 = CUACD_NONE, in0 = CUACD_NONE, in1 = CUACD_NONE;
-      for (uint32_t i = lid; i < nv; i += G) {
-        f3 v = h.qvert(i);
-        float d0 = dot(a0, v), d1 = dot(a1, v);
-        am_merge(mx0, ix0, d0, i);
-        am_merge(mn0, in0, -d0, i);
-        am_merge(mx1, ix1, d1, i);
-        am_merge(mn1, in1, -d1, i);
-      }
-      grp_argmax<G>(mx0, ix0, sm);
-      grp_argmax<G>(mn0, in0, sm);
-      grp_argmax<G>(mx1, ix1, sm);
-      grp_argmax<G>(mn1, in1, sm);
-      if (lid == 0) { hs.seed[4 * ps] = ix0; hs.seed[4 * ps + 1] = in0; hs.seed[4 * ps + 2] = ix1; hs.seed[4 * ps + 3] = in1; }
-    }
   }
   Grp<G>::sync();
   if (P.hullStage == 1) {
@@ -2430,7 +2387,7 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   // the register hull first when the part's points are in shared memory; a
   // hull that outgrows the warp is built again from the simplex in the
   // slot-array form (the same sequence, so the same result)
-  bool tiny = G == 32 && ts != nullptr && h.qc != nullptr;
+  bool tiny = G == 32 && nv <= QC_MAX;
   if (G == 32 && P.handOn && !tiny) return false;
 restart:
   // initial simplex (shaders.ts:1227-1263). The reference scans the 80 seeds
@@ -2443,6 +2400,7 @@ restart:
     const f3 d01 = p1 - p0;
     float best = 0.0f;
     uint32_t bk = CUACD_NONE;
+#pragma unroll 1
     for (uint32_t k = lid; k < 80; k += G) {
       const f3 c = cross(d01, h.qvert(hs.seed[k]) - p0);
       const float v = dot(c, c);
@@ -2457,6 +2415,7 @@ restart:
       const f3 n = cross(d01, e2);
       float bd = 0.0f;
       uint32_t k3 = CUACD_NONE;
+#pragma unroll 1
       for (uint32_t k = lid; k < 80; k += G) {
         const f3 dk = h.qvert(hs.seed[k]) - p0;
         const float v = fabsf(dot(n, dk));
@@ -2471,10 +2430,7 @@ restart:
     if (lid < 4 && i3 != CUACD_NONE) {
       uint32_t a = i0, b = i1, c = i2;
       if (bs > 0) { b = i2; c = i1; }
-      if (lid == 0) h.face_write(0, a, b, c);
-      if (lid == 1) h.face_write(1, a, i3, b);
-      if (lid == 2) h.face_write(2, b, i3, c);
-      if (lid == 3) h.face_write(3, c, i3, a);
+      h.face_write(lid, lid < 2 ? a : (lid == 2 ? b : c), lid ? i3 : b, lid == 0 || lid == 2 ? c : (lid == 1 ? b : a));
       // faces across each edge of the tetrahedron
       *reinterpret_cast<uint4*>(h.nbr + 4 * lid) =
           lid == 0 ? make_uint4(1, 2, 3, 0)
@@ -2499,11 +2455,12 @@ restart:
   uint32_t nuniq = 0;
   // (a warp marks the points it has listed, in the horizon map's bytes;
   // comparing every pair of positions was another 4 %)
-  const bool marks = G == 32 && ts != nullptr && h.qc != nullptr;
+  const bool marks = G == 32 && nv <= QC_MAX;
   if (marks) {
     for (uint32_t w = lid; w < QC_MAX / 4; w += 32) reinterpret_cast<uint32_t*>(ts->hA)[w] = 0;
     Grp<G>::sync();
   }
+#pragma unroll 1
   for (uint32_t c = 0; c * G < 80; c++) {
     const uint32_t k = c * G + lid;
     bool keep = false;
@@ -2687,6 +2644,12 @@ restart:
 // (the widest whose resident blocks hold the level's parts in one wave): a
 // block inserts up to one point per warp (at most 16) per round, and its
 // width serves the passes over all points, which grow with nv.
+// The warp kernel is bound by instruction fetch: its 32 warps an SM are at
+// different steps, and half of their waiting was for instructions. So its
+// short loops stay rolled, the simplex's four faces are one piece of code, and
+// the points on the grid always lie in one array (a second way to read them
+// was part of every point access): 218 to 169 KB of code, 75,000 staircase
+// children 0.74 to 0.58 ms.
 template <int G>
 __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 ? 2 : 4))
     k_hull(const Level P, const Dev D) {
