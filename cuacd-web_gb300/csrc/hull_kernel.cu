@@ -2150,24 +2150,26 @@ __device__ __noinline__ uint32_t hull_assign_block(const HullCtx& h, GrpSmem& sm
 template <int G>
 __device__ __noinline__ double hull_volume_grid(const HullCtx& h, HullSm& hs, GrpSmem& sm) {
   const int lid = Grp<G>::lid();
-  uint32_t a0, b0, c0;
-  h.abc(0, a0, b0, c0);
-  const f3 of = h.qvert(a0);
-  const long long ox = (long long)of.x, oy = (long long)of.y, oz = (long long)of.z;
-  __int128 v6 = 0;
+  // six times the volume over a face's own corner a and exact normal N: the
+  // sum of (a - o) . N, N = 2^32 h + l as in face_exact, its parts apart (the
+  // low part's carry folded in, so both stay far below 2^63)
+  const uint4 r0 = h.rec(0)[2];
+  const f3 of = mk3(__uint_as_float(r0.x), __uint_as_float(r0.y), __uint_as_float(r0.z));
+  long long A = 0, B = 0;
   const uint32_t nf = hs.nf;
 #pragma unroll 1
   for (uint32_t f = lid; f < nf; f += G) {
-    if (!h.alive(f)) continue;
-    uint32_t a, b, c;
-    h.abc(f, a, b, c);
-    f3 pa = h.qvert(a), pb = h.qvert(b), pc = h.qvert(c);
-    long long ax = (long long)pa.x - ox, ay = (long long)pa.y - oy, az = (long long)pa.z - oz;
-    long long bx = (long long)pb.x - ox, by = (long long)pb.y - oy, bz = (long long)pb.z - oz;
-    long long cx = (long long)pc.x - ox, cy = (long long)pc.y - oy, cz = (long long)pc.z - oz;
-    long long nx = by * cz - bz * cy, ny = bz * cx - bx * cz, nz = bx * cy - by * cx;
-    v6 += (__int128)ax * nx + (__int128)ay * ny + (__int128)az * nz;
+    const uint4* r = h.rec(f);
+    if ((r[0].x & ALIVE) == 0) continue;
+    const uint4 w2 = r[2], w3 = r[3];
+    const long long dx = (long long)(__uint_as_float(w2.x) - of.x), dy = (long long)(__uint_as_float(w2.y) - of.y),
+                    dz = (long long)(__uint_as_float(w2.z) - of.z);
+    A += (short)(w3.z & 0xffffu) * dx + (short)(w3.z >> 16) * dy + (short)w3.w * dz;
+    B += (long long)w2.w * dx + (long long)w3.x * dy + (long long)w3.y * dz;
+    A += B >> 32;
+    B &= 0xffffffffll;
   }
+  const __int128 v6 = (__int128)A * 4294967296ll + B;
   // group sum of the 128-bit partials
   unsigned long long lo = (unsigned long long)v6;
   long long hi = (long long)(v6 >> 64);
@@ -2406,7 +2408,7 @@ restart:
       const float v = dot(c, c);
       if (v > best) { best = v; bk = k; }
     }
-    grp_argmax<G>(best, bk, sm);
+    grp_argmax_pos<G>(best, bk, sm);
     uint32_t i3 = CUACD_NONE, i2 = CUACD_NONE;
     int bs = 0;
     if (bk != CUACD_NONE) {
@@ -2421,7 +2423,7 @@ restart:
         const float v = fabsf(dot(n, dk));
         if (v > bd && orient_filtered(n, d01, e2, dk) != 0) { bd = v; k3 = k; }
       }
-      grp_argmax<G>(bd, k3, sm);
+      grp_argmax_pos<G>(bd, k3, sm);
       if (k3 != CUACD_NONE) {
         i3 = hs.seed[k3];
         bs = orient_filtered(n, d01, e2, h.qvert(i3) - p0);
