@@ -111,6 +111,7 @@ struct HdArgs {
   uint32_t* ns;              // per mesh: sample count
   uint32_t partBase;
   uint32_t screenMin;        // targets with at least this many triangles are searched by clusters
+  uint32_t orderedMin;       // in targets with at least this many, a sliver counts when it is within reach
   const uint32_t* triOff;    // per mesh: first entry of its triangles below (a multiple of 32)
   uint32_t* cnt;             // per triangle: its area, then its samples
   uint32_t* soff;            // per triangle: its cell, then (sorted) its first sample

@@ -74,6 +74,10 @@ static const uint32_t SMALL_NV = 1024;
 static const uint32_t WIDE_JOBS = 16, WIDE_NV = 128;
 // Hausdorff targets with at least this many triangles are searched by clusters
 static const uint32_t HD_SCREEN_MIN = 64;
+// In those with at least this many, slivers count only within reach of the
+// triangles before them (HdReach); smaller targets have every one counted, as
+// their exhaustive search does.
+static const uint32_t HD_ORDERED_MIN = 256;
 // Hausdorff batches of at least this many triangles have the areas that their
 // sample capacities follow from added on the device (k_hd_area, about 40 us
 // with its readback); smaller ones on the host, at 3.4 ns a triangle
@@ -932,6 +936,7 @@ struct Tree {
     A.perm = (uint32_t*)(d + permOff);
     A.partBase = partBase;
     A.screenMin = cfg.hdScreenMinTris == 0 ? HD_SCREEN_MIN : (cfg.hdScreenMinTris < 0 ? 0xffffffffu : (uint32_t)cfg.hdScreenMinTris);
+    A.orderedMin = cfg.hdScreenMinTris == 0 ? HD_ORDERED_MIN : A.screenMin;
     launch_hd(A, D, nSM, stream);
     hdStatsPending = true;
     return 0;

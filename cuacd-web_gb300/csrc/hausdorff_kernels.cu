@@ -21,8 +21,8 @@
 // What bounds it: dependent loads and divergence in k_hd_near. Against a
 // tensor-core bound of every sample-triangle pair, whose epilogue was bound by
 // instruction issue: 24 cut halves of 1.5-30k triangles with their hulls
-// 11.4 -> 0.86 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.66 ms, 192
-// pairs of 160-6,000 triangles 5.8 + 0.71 -> 0.50 ms.
+// 11.4 -> 1.28 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.82 ms, 192
+// pairs of 160-6,000 triangles 5.8 + 0.71 -> 0.90 ms.
 #include <algorithm>
 
 #include "cuacd_dev.cuh"
@@ -315,8 +315,9 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
         const float n2 = dot(nn, nn);
         if (!(n2 > 1e-4f * dot(ab, ab) * dot(ac, ac)) || n2 < 1.1e-20f) {
           r = -r;
-          A.bad[base + atomicAdd(&sBad, 1u)] = i;
+          sBad = 1;
         }
+        cnt[t] = i | (r < 0.0f ? 0x80000000u : 0u);  // its samples have been read
         float4* G = A.triG + 3 * (base + i);
         G[0] = make_float4(a.x, a.y, a.z, 0.0f);
         G[1] = make_float4(b.x, b.y, b.z, 0.0f);
@@ -349,7 +350,16 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
       if (i0 + 32 * u < nt) soff[i0 + 32 * u] = run + before + off[u];
     run += tot;
   }
-  if (tid == 0) A.nBad[m] = sBad;  // behind the last scan's barriers
+  // the slivers in the triangles' own order (behind the last scan's barriers)
+  run = 0;
+  for (uint32_t c0 = 0; sBad != 0 && c0 < nt; c0 += HD_PREP) {
+    const uint32_t v = c0 + tid < nt ? cnt[c0 + tid] : 0u;
+    uint32_t tot;
+    const uint32_t at = run + prep_scan(v >> 31, ws, &tot) - 1;
+    if (v >> 31) A.bad[base + at] = v & 0x7fffffffu;
+    run += tot;
+  }
+  if (tid == 0) A.nBad[m] = run;
 }
 
 // tiles of 32 samples per mesh: their prefix over the meshes, and the work
@@ -404,16 +414,40 @@ __global__ void __launch_bounds__(1024) k_hd_tiles(const HdArgs A, const Dev D) 
 // s^2 in length, so a point taken for one above the triangle lies within 6e-4
 // |p - a| of it, 4e-7 of the squared distance. For a sliver the normal can
 // be noise and the plane distance anything, and a triangle with |n|^2 < 1e-20
-// counts by its corners alone: such triangles give no ub, and a sample that
-// could still raise the pair's largest distance is at last tested against
-// every one of them, near or far. So the distance is the exhaustive
-// search's, whichever order the tiles run in.
+// counts by its corners alone: such triangles give no ub, and the samples that
+// could still raise the pair's largest distance meet them at last, in the
+// triangles' order. In a target below A.orderedMin triangles every one counts,
+// as in an exhaustive search; in a larger one it counts within reach (HdReach)
+// only. Parts that have been cut again and again hold hundreds of slivers, and
+// with every one counted the noise of far ones made the distances of 9 parts
+// in 90 decompositions up to 32 % smaller than they are in 64 bits. Either way
+// the distance does not depend on the order in which the tiles run.
 struct HdNear {
   f3 p;
   float p2, best, ub;
+  uint32_t at;  // the triangle that gave best (the first of equal ones)
   __device__ __forceinline__ float reach() const { return fminf(best, ub) * 1.001f + 3e-10f * p2 + 1e-30f; }
   // whether the sample can still raise the pair's largest distance
   __device__ __forceinline__ bool counts(float gmax) const { return best > gmax && !(ub + 3e-9f * p2 < gmax); }
+};
+
+// A sliver's reach: what a search of the triangles in order, by centroids, lets
+// through. With a margin e of 2^-13 (|p|^2 + |c|^2 + 2 |p|_1 |c|_1) on squared
+// centroid distances, triangle t counts when its bound (sqrt(|p - c|^2 - e) -
+// r)^2 is not above the smallest tri_sq before t's 32 triangles or the smallest
+// |p - c|^2 + e up to t. For any other triangle the rule changes nothing, as
+// one that is out of reach is not the nearest.
+struct HdReach {
+  float lb, ub, slack;
+  __device__ __forceinline__ HdReach(f3 p, float p2, float p1, float4 c4) {
+    const f3 c = mk3(c4.x, c4.y, c4.z), d = p - c;
+    const float c2 = dot(c, c), q = dot(d, d), e = 1.220703125e-4f * (p2 + c2 + 2.0f * p1 * l1(c));
+    const float lo = sqrtf(fmaxf(q - e, 0.0f)) - fabsf(c4.w);
+    lb = lo > 0.0f ? lo * lo : 0.0f;
+    ub = q + e;
+    slack = 1e-10f * (p2 + c2) + 1e-30f;
+  }
+  __device__ __forceinline__ bool within(float bound) const { return lb <= bound * 1.001f + slack; }
 };
 
 __device__ __forceinline__ float warp_box_min(float v) { return f_unord(__reduce_min_sync(FULLMASK, f_ord(v))); }
@@ -492,6 +526,9 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
     S.p2 = dot(S.p, S.p);
     S.best = 3.4e38f;
     S.ub = 3.4e38f;
+    S.at = 0xffffffffu;
+    const bool ordered = tnt >= A.orderedMin;
+    const uint32_t* order = A.perm + tb;
     const float4* C = A.triC + tb;
     const float4* B = A.box + 2 * (tb >> 5);
     const uint32_t nc = (tnt + 31) / 32;
@@ -519,7 +556,12 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
       auto exact = [&](uint32_t j) {
         const float4* g = G + 3 * (size_t)(32 * c + j);
         const float4 a = g[0], b = g[1], cc = g[2];
-        S.best = fminf(S.best, tri_sq(S.p, xyz(a), xyz(b), xyz(cc)));
+        const float v = tri_sq(S.p, xyz(a), xyz(b), xyz(cc));
+        if (ordered && v <= S.best) {
+          const uint32_t t = order[32 * c + j];
+          S.at = v < S.best ? t : min(S.at, t);
+        }
+        S.best = fminf(S.best, v);
         nExact++;
       };
       if (active && dmin < 3.4e38f) {
@@ -533,7 +575,7 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
         const float4 g = cent[j];
         const f3 d = S.p - mk3(g.x, g.y, g.z);
         const float q = rs + fabsf(g.w);
-        if (!(dot(d, d) > q * q * 1.00001f)) keep |= 1u << j;
+        if (!(dot(d, d) > q * q * 1.00001f) && !(ordered && g.w < 0.0f)) keep |= 1u << j;
       }
       if (dmin < 3.4e38f) keep &= ~(1u << jmin);
       if (!active) keep = 0;
@@ -612,9 +654,60 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
       }
     }
     // what is left against the target's slivers
-    if (act) {
-      const uint32_t nBad = A.nBad[dst];
-      if (nBad != 0) active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
+    const uint32_t nBad = act ? A.nBad[dst] : 0u;
+    if (nBad != 0 && ordered) {
+      const float p1 = l1(S.p);
+      // smallest distance before the current 32 triangles, slivers counted; a
+      // bound by the slivers' centroids
+      const float nearest = S.best;
+      float before = nearest, sub = 3.4e38f;
+      uint32_t group = 0xffffffffu;
+      active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
+      for (uint32_t k = 0; k < nBad; k++) {
+        if ((k & 31u) == 0 && __ballot_sync(FULLMASK, active) == 0) break;
+        const uint32_t i = A.bad[tb + k], t = order[i];
+        const float4* g = G + 3 * (size_t)i;
+        const float4 a = g[0], b = g[1], c = g[2];
+        if ((t >> 5) != group) {
+          group = t >> 5;
+          before = S.best;
+        }
+        const HdReach R(S.p, S.p2, p1, C[i]);
+        sub = fminf(sub, R.ub);
+        const float v = tri_sq(S.p, xyz(a), xyz(b), xyz(c));
+        nExact += active ? 1u : 0u;
+        const bool lower = active && v < S.best;
+        bool in = lower && R.within(fminf(before, sub));
+        // out of reach of the nearest triangle of all, but not of the slivers
+        // so far: in if it is within reach of the triangles before it
+        unsigned ask = __ballot_sync(FULLMASK, lower && !in && R.within(sub) && S.at >= (t & ~31u));
+        while (ask) {
+          const uint32_t l = __ffs(ask) - 1;
+          ask &= ask - 1;
+          const f3 p = mk3(__shfl_sync(FULLMASK, S.p.x, l), __shfl_sync(FULLMASK, S.p.y, l), __shfl_sync(FULLMASK, S.p.z, l));
+          const float p2 = dot(p, p), pl = l1(p);
+          float low = 3.4e38f;
+          for (uint32_t j = lane; j < tnt; j += 32) {
+            const uint32_t s = order[j];
+            if (s > t) continue;
+            const float4 cj = C[j];
+            const HdReach Q(p, p2, pl, cj);
+            low = fminf(low, Q.ub);
+            if (s >= (t & ~31u) || cj.w < 0.0f || !Q.within(low)) continue;
+            const float4* h = G + 3 * (size_t)j;
+            low = fminf(low, tri_sq(p, xyz(h[0]), xyz(h[1]), xyz(h[2])));
+          }
+          low = f_unord(__reduce_min_sync(FULLMASK, f_ord(low)));
+          // a sliver counted before has made its distance the bound
+          if (lane == l) in = R.within(before < nearest ? fminf(low, before) : low);
+        }
+        if (in) {
+          S.best = v;
+          active = S.counts(__uint_as_float(__ldcg(gmaxAt)));
+        }
+      }
+    } else if (nBad != 0) {
+      active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
       for (uint32_t k = 0; k < nBad; k++) {
         if ((k & 31u) == 0 && __ballot_sync(FULLMASK, active) == 0) break;
         const float4* g = G + 3 * (size_t)A.bad[tb + k];
