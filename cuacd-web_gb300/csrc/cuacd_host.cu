@@ -15,6 +15,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include "../../include/cuacd.h"
@@ -72,6 +73,14 @@ static const uint32_t SMALL_NV = 1024;
 // 2.38; depth-3 staircases of 96 points, 8 of them 0.46 and 0.34, 40 (25,200
 // jobs) 0.71 and 0.97, 160 (100,800 jobs) 1.92 and 3.44.
 static const uint32_t WIDE_JOBS = 16, WIDE_NV = 128;
+// Levels and batches whose largest part has more points take 512- and
+// 1024-thread hull blocks (where they fit in one wave): the passes over all
+// points grow with a part, a round's barriers with the block. 150 parts of 700,
+// 1,000, 1,400, 2,000 and 3,000 points on 1024 threads 0.68, 0.58, 0.78, 1.24
+// and 1.19 ms, on 512 0.63, 0.52, 0.75, 1.24 and 1.23, on 256 0.58, 0.50, 0.75,
+// 1.25 and 1.27; one part of 150 points 0.40, 0.35 and 0.35, of 12,000 2.00, 2.13
+// and 2.76.
+static const uint32_t MID_HULL_NV = 1024, WIDE_HULL_NV = 2048;
 // Hausdorff targets with at least this many triangles are searched by clusters
 static const uint32_t HD_SCREEN_MIN = 64;
 // In those with at least this many, slivers count only within reach of the
@@ -347,19 +356,20 @@ struct Tree {
   }
   // hull launches of one level, warp groups then block groups; work
   // counters `slot`, 16 + slot and 48 + slot must be zero beforehand. The
-  // parts that the warps list take the widest blocks (1024, then 512 threads) whose
-  // resident slots hold all the level's parts in one wave (the more threads
-  // per part, the shorter each insertion round), else 256-thread blocks
-  // (the most parts at once).
-  void hullLaunch(Level P, uint32_t slot) {
+  // parts that the warps list take the widest blocks (1024, then 512 threads) that
+  // a largest part of about maxNv points makes worth it and whose resident slots
+  // hold all the level's parts in one wave, else 256-thread blocks (the most
+  // parts at once).
+  void hullLaunch(Level P, uint32_t slot, uint32_t maxNv) {
     P.workSlot = slot;
     P.nSlabs = nSlabsSmall;
     launch_hull(P, D, 32, stream);
     int width = 256;
     uint32_t slabs = nSlabsBig;
-    for (const auto& [w, bps] : {std::pair<int, int>{1024, bpsXL}, {512, bpsWide}}) {
+    for (const auto& [w, bps, above] : {std::tuple<int, int, uint32_t>{1024, bpsXL, WIDE_HULL_NV},
+                                        {512, bpsWide, MID_HULL_NV}}) {
       const uint32_t cap = (uint32_t)(nSM * bps);
-      if (bps > 0 && P.nChildParts <= cap) {
+      if (bps > 0 && maxNv > above && P.nChildParts <= cap) {
         width = w;
         slabs = std::min(nSlabsBig, cap);
         break;
@@ -599,7 +609,7 @@ struct Tree {
         // the last level's pruning bound, once per seed (the parent level's
         // items are final once its record ran)
         if (P.lastLevel && P.level > 0 && P.nSeeds > 0 && P.nItemsIn > 0) launch_seed_bound(P, D, stream);
-        hullLaunch(P, l);
+        hullLaunch(P, l, maxSeedNv >> l);
         mark(4);
         launch_record(P, D, stream);
         mark(5);
@@ -622,7 +632,9 @@ struct Tree {
                                (uint64_t)bWork.p};
     for (auto& L : tree) { s.push_back(L.nJobs); s.push_back(L.totalWidth); s.push_back(L.width); }
     for (const auto* st : {&tree, &probe})
-      for (uint32_t l = 0; l < st->size(); l++) s.push_back(bigLevel(l) | (wideLevel(l, (*st)[l].nJobs) << 1));
+      for (uint32_t l = 0; l < st->size(); l++)
+        s.push_back(bigLevel(l) | (wideLevel(l, (*st)[l].nJobs) << 1) | (((maxSeedNv >> l) > MID_HULL_NV) << 2) |
+                    (((maxSeedNv >> l) > WIDE_HULL_NV) << 3));
     s.push_back(smallNv());
     s.push_back(baseLevel(false).handOn);
     s.push_back((uint64_t)bList.p);
@@ -763,7 +775,7 @@ struct Tree {
     P.hdDescBase = withHd ? (uint32_t)n : 0;
     CK(cudaMemsetAsync(D.work, 0, 64 * 4, stream));
     CK(cudaEventRecord(ev0, stream));
-    hullLaunch(P, 0);
+    hullLaunch(P, 0, maxNv);
     if (withHd) {
       std::vector<uint32_t> triCap(2 * n);
       for (int k = 0; k < n; k++) {
