@@ -100,14 +100,21 @@ static const uint32_t BIG_JOB_NV = 2048;
 // blocks, in a tree's levels and in hull batches.
 // The kernels' outputs do not depend on which group shape handles a part,
 // so every schedule gives the same results; they differ in speed with the
-// distribution of part sizes. The first is the fixed default.
+// distribution of part sizes. The first is the fixed default. All but one hand
+// parts on: without it in the last two, 24 blobs of 8,000 triangles decomposed in
+// 96.9, 95.2, 99.6 and 126.5 ms a pass while trying schedule 0 to 3, with it in
+// 96.1, 94.4, 94.3 and 97.4. The last one keeps trees of small seeds on warps,
+// whose few outgrown children cost a second launch per level otherwise (160
+// staircases 10.4, 10.4, 10.4 and 9.0 ms).
 struct Schedule {
-  uint32_t smallNv, bigJobNv, handTree, handBatch;
+  uint32_t smallNv, bigJobNv, handSmallTree, handTree, handBatch;
 };
-static const Schedule kSchedules[] = {{SMALL_NV, BIG_JOB_NV, HAND_ON_TREE, HAND_ON_BATCH},
-                                      {512, BIG_JOB_NV, HAND_ON_BATCH, HAND_ON_TREE},
-                                      {256, BIG_JOB_NV, 0, 0},
-                                      {SMALL_NV, 4096, 0, 0}};
+// trees whose seeds have at most this many points count as small
+static const uint32_t SMALL_TREE_NV = 256;
+static const Schedule kSchedules[] = {{SMALL_NV, BIG_JOB_NV, HAND_ON_TREE, HAND_ON_TREE, HAND_ON_BATCH},
+                                      {512, BIG_JOB_NV, HAND_ON_BATCH, HAND_ON_BATCH, HAND_ON_TREE},
+                                      {256, BIG_JOB_NV, HAND_ON_TREE, HAND_ON_TREE, HAND_ON_BATCH},
+                                      {SMALL_NV, 4096, 0, 257, 129}};
 static const int kNumSchedules = (int)(sizeof(kSchedules) / sizeof(kSchedules[0]));
 // per key: device time of one run or batch under each schedule tried so far
 struct TuneEntry {
@@ -351,7 +358,8 @@ struct Tree {
     P.hullSlabWords = slabWords;
     P.slabStride = slabStride;
     P.smallNv = smallNv();
-    if (cfg.warpMaxNv <= 0) P.handOn = batch ? kSchedules[sched].handBatch : kSchedules[sched].handTree;
+    const Schedule& s = kSchedules[sched];
+    if (cfg.warpMaxNv <= 0) P.handOn = batch ? s.handBatch : (maxSeedNv <= SMALL_TREE_NV ? s.handSmallTree : s.handTree);
     return P;
   }
   // hull launches of one level, warp groups then block groups; work
