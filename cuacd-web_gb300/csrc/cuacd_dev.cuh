@@ -131,10 +131,9 @@ struct HdArgs {
 // and segments (4 fmax), two bitmap arrays (2 ceil(fmax / 32)) and two
 // horizon maps (2 nv). With fmax <= (W - 3 nv) / 16 the 8 fmax + 2 nv words
 // are at most W / 2 + nv / 2, and with nv <= (W - 1024) / 3 below 2 W / 3.
-// The points on the grid (4 nv words) follow; where the hull bound is far
-// below the part's points they need more than that (hull_slab_words).
+// The points on the grid (4 nv words) follow where they fit.
 __host__ __device__ constexpr uint64_t hull_slab_words(uint32_t W, uint32_t fmax, uint32_t nv) {
-  return (uint64_t)W + 4096u + 8ull * fmax + 2ull * ((fmax + 31) / 32) + 6ull * nv + 3;
+  return (uint64_t)W + 4096u + 8ull * fmax + 2ull * ((fmax + 31) / 32) + 2ull * nv;
 }
 __host__ __device__ constexpr uint32_t hull_slab_stride(uint32_t W) {
   return (W + 4096u + (uint32_t)(((uint64_t)W * 2) / 3) + W / 128 + 64u + 63u) & ~63u;

@@ -99,7 +99,11 @@ __device__ __forceinline__ int orient_filtered(f3 n, f3 e1, f3 e2, f3 d) {
 }
 
 struct HullCtx {
-  uint32_t nv, fmax;
+  const float* V;
+  uint32_t vOff, nv;
+  f3 qlo;
+  float qs;
+  uint32_t fmax;
   uint32_t* owner;
   float* dist;
   uint32_t* cand;
@@ -114,9 +118,17 @@ struct HullCtx {
   uint32_t* hA;    // per point: new face whose horizon edge starts there
   uint32_t* hB;    // per point: new face whose horizon edge ends there
   const float4* qc;  // quantised points, one 16-byte load each: a warp's small
-                     // part's in shared memory, else in the slab
+                     // part's in shared memory, else in the slab; null for a
+                     // block's part whose points do not fit it (a child far
+                     // larger than the run's seeds, or a small hull bound)
 
-  __device__ __forceinline__ f3 qvert(uint32_t i) const { return xyz(qc[i]); }
+  __device__ __noinline__ f3 qvert_far(uint32_t i) const {
+    const f3 v = ldv(V, (size_t)vOff + 3 * (size_t)i) - qlo;
+    return mk3(rintf(v.x * qs), rintf(v.y * qs), rintf(v.z * qs));
+  }
+  __device__ __forceinline__ f3 qvert(uint32_t i) const { return qc ? xyz(qc[i]) : qvert_far(i); }
+  // where a warp holds the part: its points always lie in qc
+  __device__ __forceinline__ f3 qnear(uint32_t i) const { return xyz(qc[i]); }
   __device__ __forceinline__ uint4* rec(uint32_t f) const { return reinterpret_cast<uint4*>(F + 16 * (size_t)f); }
   __device__ __forceinline__ bool alive(uint32_t f) const { return (F[16 * (size_t)f] & ALIVE) != 0; }
   __device__ __forceinline__ void abc(uint32_t f, uint32_t& a, uint32_t& b, uint32_t& c) const {
@@ -566,7 +578,7 @@ __device__ __noinline__ uint32_t hull_tiny_grow(const HullCtx& h, HullSm& hs, Ti
       R &= R - 1;
       const uint32_t pr = __shfl_sync(FULLMASK, ci, r);
       float v = -1.0f;
-      if (lane >= lo && lane < nalive) v = tiny_eval(h, F, h.qvert(pr), pr);
+      if (lane >= lo && lane < nalive) v = tiny_eval(h, F, h.qnear(pr), pr);
       const uint32_t vk = v > 0.0f ? __float_as_uint(v) : 0u;
       const uint32_t best = __reduce_max_sync(FULLMASK, vk);
       const unsigned at = __ballot_sync(FULLMASK, best != 0u && vk == best);
@@ -583,7 +595,7 @@ __device__ __noinline__ uint32_t hull_tiny_grow(const HullCtx& h, HullSm& hs, Ti
     const uint32_t pick = __reduce_min_sync(FULLMASK, key == mk ? ci : CUACD_NONE);
     const unsigned holder = __ballot_sync(FULLMASK, key == mk && ci == pick);
     const uint32_t start = __shfl_sync(FULLMASK, co, __ffs(holder) - 1);
-    const f3 pp = h.qvert(pick);
+    const f3 pp = h.qnear(pick);
     nIns++;
     // the slot-array form compacts here (hull_insert's condition)
     bool compacted = false;
@@ -646,7 +658,7 @@ __device__ __noinline__ uint32_t hull_tiny_grow(const HullCtx& h, HullSm& hs, Ti
     } else if (lane < nS + nnew) {
       const uint32_t j = lane - nS;
       const uint32_t a = ts.stage[3 * j], b = ts.stage[3 * j + 1], tw = ts.stage[3 * j + 2];
-      h.face_make(a, b, pick, F.w0, F.w1, F.w2, F.w3);
+      h.face_make_abc(a, b, pick, h.qnear(a), h.qnear(b), pp, F.w0, F.w1, F.w2, F.w3);
       F.nb0 = __popc(S & ((1u << tw) - 1u));
       F.nb1 = ts.hA[b];
       F.nb2 = ts.hB[a];
@@ -2020,7 +2032,7 @@ __device__ __noinline__ uint32_t hull_assign_all(const HullCtx& h, GrpSmem& sm, 
 #pragma unroll
     for (int k = 0; k < ASSIGN_K; k++) {
       const uint32_t i = base + k * G + lid;
-      p[k] = h.qvert(i < nv ? i : 0u);
+      p[k] = G == 32 ? h.qnear(i < nv ? i : 0u) : h.qvert(i < nv ? i : 0u);
       bd[k] = 0.0f;
       bo[k] = CUACD_NONE;
     }
@@ -2289,15 +2301,15 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
     if (lid == 0) { pdp->hullVol = -1.0f; pdp->flags = 3; atomicAdd(D.ctr + CTR_HULLFAIL, 1u); }
     return true;
   }
-  // the walk's arrays and the grid points after the reference's slab words
-  // must fit the slab (they always do; checked so a slab is never overrun)
+  // the walk's arrays after the reference's slab words must fit the slab
+  // (always true for hull_slab_stride; checked so a slab is never overrun)
   if (hull_slab_words(P.hullSlabWords, fmax, nv) > P.slabStride) {
     if (lid == 0) { pdp->hullVol = -1.0f; pdp->flags = 3; atomicAdd(D.ctr + CTR_HULLFAIL, 1u); }
     return true;
   }
   if (lid == 0) add_bytes(D.ctr, CTR_BYTES_HULL, 12ull * nv);
   HullCtx c;
-  c.nv = nv; c.fmax = fmax;
+  c.V = D.V; c.vOff = vOff; c.nv = nv; c.fmax = fmax;
   c.owner = slab;
   c.dist = reinterpret_cast<float*>(slab + nv);
   c.cand = slab + 2 * nv;
@@ -2329,18 +2341,23 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   const f3 ext = hi - lo;
   const float scale = fmaxf(fmaxf(fmaxf(ext.x, ext.y), ext.z), 1e-30f);
   const float qs = 2097152.0f / scale;
+  c.qlo = lo;
+  c.qs = qs;
   const float cell = scale / 2097152.0f;
   const float volScale = (cell * cell) * cell;
   // the points on the grid, a warp's small part's in shared memory
   {
     const bool inSm = G == 32 && nv <= QC_MAX;
-    float4* qp = inSm ? qcache : reinterpret_cast<float4*>(slab + (((uint64_t)(c.hB - slab) + nv + 3) & ~3ull));
+    const uint64_t at = ((uint64_t)(c.hB - slab) + nv + 3) & ~3ull;
+    const bool fits = inSm || at + 4ull * nv <= P.slabStride;
+    if (G == 32 && !fits) return false;  // a block reads its points where they are
+    float4* qp = inSm ? qcache : reinterpret_cast<float4*>(slab + at);
 #pragma unroll (G == 32 ? 1 : 4)
-    for (uint32_t i = lid; i < nv; i += G) {
+    for (uint32_t i = lid; fits && i < nv; i += G) {
       const f3 v = ldv(D.V, (size_t)vOff + 3 * (size_t)i) - lo;
       qp[i] = make_float4(rintf(v.x * qs), rintf(v.y * qs), rintf(v.z * qs), 0.0f);
     }
-    c.qc = qp;
+    c.qc = fits ? qp : nullptr;
   }
   // what every step below reads, one copy per group: a copy per thread in local
   // memory (the steps are calls) took 200 KB of an SM's L1
@@ -2361,7 +2378,7 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
       uint32_t ix = 0, in = 0;
       const uint32_t i1 = nv * (part + 1) / parts;
       for (uint32_t i = nv * part / parts; i < i1; i++) {
-        const float d = dot(ax, h.qvert(i));
+        const float d = dot(ax, h.qnear(i));
         if (d > mx) { mx = d; ix = i; }
         if (d < mn) { mn = d; in = i; }
       }
@@ -2397,14 +2414,15 @@ restart:
   // position reaching the maximum: here every lane scans its positions in
   // order and the group argmax breaks ties by the lowest position.
   {
+    auto at = [&](uint32_t i) -> f3 { return G == 32 ? h.qnear(i) : h.qvert(i); };
     const uint32_t i0 = hs.seed[1], i1 = hs.seed[0];
-    const f3 p0 = h.qvert(i0), p1 = h.qvert(i1);
+    const f3 p0 = at(i0), p1 = at(i1);
     const f3 d01 = p1 - p0;
     float best = 0.0f;
     uint32_t bk = CUACD_NONE;
 #pragma unroll 1
     for (uint32_t k = lid; k < 80; k += G) {
-      const f3 c = cross(d01, h.qvert(hs.seed[k]) - p0);
+      const f3 c = cross(d01, at(hs.seed[k]) - p0);
       const float v = dot(c, c);
       if (v > best) { best = v; bk = k; }
     }
@@ -2413,20 +2431,20 @@ restart:
     int bs = 0;
     if (bk != CUACD_NONE) {
       i2 = hs.seed[bk];
-      const f3 e2 = h.qvert(i2) - p0;
+      const f3 e2 = at(i2) - p0;
       const f3 n = cross(d01, e2);
       float bd = 0.0f;
       uint32_t k3 = CUACD_NONE;
 #pragma unroll 1
       for (uint32_t k = lid; k < 80; k += G) {
-        const f3 dk = h.qvert(hs.seed[k]) - p0;
+        const f3 dk = at(hs.seed[k]) - p0;
         const float v = fabsf(dot(n, dk));
         if (v > bd && orient_filtered(n, d01, e2, dk) != 0) { bd = v; k3 = k; }
       }
       grp_argmax_pos<G>(bd, k3, sm);
       if (k3 != CUACD_NONE) {
         i3 = hs.seed[k3];
-        bs = orient_filtered(n, d01, e2, h.qvert(i3) - p0);
+        bs = orient_filtered(n, d01, e2, at(i3) - p0);
       }
     }
     if (lid < 4 && i3 != CUACD_NONE) {
@@ -2643,15 +2661,16 @@ restart:
 // Persistent groups: group s owns slab s and takes the launch's parts from a
 // counter, so parts of uneven size balance across the GPU. Warps take every
 // part first and list the ones for the blocks of 256, 512 or 1024 threads
-// (the widest whose resident blocks hold the level's parts in one wave): a
-// block inserts up to one point per warp (at most 16) per round, and its
-// width serves the passes over all points, which grow with nv.
+// (wider ones for larger parts, where their resident blocks hold the level's
+// parts in one wave): a block inserts up to one point per warp (at most 16) per
+// round, and its width serves the passes over all points, which grow with nv.
 // The warp kernel is bound by instruction fetch: its 32 warps an SM are at
 // different steps, and half of their waiting was for instructions. So its
 // short loops stay rolled, the simplex's four faces are one piece of code, and
-// the points on the grid always lie in one array (a second way to read them
-// was part of every point access): 218 to 169 KB of code, 75,000 staircase
-// children 0.74 to 0.58 ms.
+// its points on the grid always lie in one array (a second way to read them
+// was part of every point access; a part whose points fit neither shared memory
+// nor the slab goes to a block): 218 to 167 KB of code, 50,400 staircase children
+// 0.74 to 0.58 ms.
 template <int G>
 __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 ? 2 : 4))
     k_hull(const Level P, const Dev D) {
