@@ -661,6 +661,7 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
       // bound by the slivers' centroids
       const float nearest = S.best;
       float before = nearest, sub = 3.4e38f;
+      float prefix = 3.4e38f;  // the last answer to the question below: later ones are no larger
       uint32_t group = 0xffffffffu;
       active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
       for (uint32_t k = 0; k < nBad; k++) {
@@ -680,7 +681,7 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
         bool in = lower && R.within(fminf(before, sub));
         // out of reach of the nearest triangle of all, but not of the slivers
         // so far: in if it is within reach of the triangles before it
-        unsigned ask = __ballot_sync(FULLMASK, lower && !in && R.within(sub) && S.at >= (t & ~31u));
+        unsigned ask = __ballot_sync(FULLMASK, lower && !in && R.within(fminf(sub, prefix)) && S.at >= (t & ~31u));
         while (ask) {
           const uint32_t l = __ffs(ask) - 1;
           ask &= ask - 1;
@@ -699,7 +700,10 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
           }
           low = f_unord(__reduce_min_sync(FULLMASK, f_ord(low)));
           // a sliver counted before has made its distance the bound
-          if (lane == l) in = R.within(before < nearest ? fminf(low, before) : low);
+          if (lane == l) {
+            prefix = low;
+            in = R.within(before < nearest ? fminf(low, before) : low);
+          }
         }
         if (in) {
           S.best = v;
