@@ -66,16 +66,22 @@ typedef struct {
   uint64_t scratchWords;
   uint64_t hullBudgetBytes; /* bytes of hull scratch slabs in flight */
   int32_t pruneLastLevel;   /* last-level branch and bound (tree.ts:29-30) */
-  int32_t warpMaxNv;        /* hulls of parts up to this many points run on one
-                               warp each, larger ones on a 256-thread block
-                               (0: 1024); the results do not depend on it */
+  int32_t warpMaxNv;        /* hulls of parts up to this many points start on
+                               one warp each, larger ones on a block of 256 to
+                               1024 threads (0: 1024, and warps hand parts that
+                               outgrow their register hull on to the blocks);
+                               the results do not depend on it */
   int32_t hdScreenMinTris;  /* Hausdorff target meshes with at least this many
                                triangles are searched by clusters (0: 64,
-                               < 0: never, every triangle is evaluated); the
-                               results do not depend on it */
+                               < 0: never, every triangle is evaluated). The
+                               results do not depend on it but for slivers (an
+                               angle below 0.57 degrees), whose float distance
+                               can be noise: one out of reach does not count in
+                               targets of 256 triangles and more (or of this
+                               many, when set) */
   int32_t autotune;         /* 1 (the default): when warpMaxNv is 0, the
-                               warp/block thresholds of the hull and of
-                               plan/emit are chosen per distribution of part
+                               warp/block thresholds of the hull, of handing on
+                               and of plan/emit are chosen per distribution of part
                                sizes (log2 buckets of the largest, median and
                                total point counts and of the part count): the
                                first runs or hull batches of each distribution
