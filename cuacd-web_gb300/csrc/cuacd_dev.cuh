@@ -111,16 +111,17 @@ struct HdArgs {
   uint32_t* ns;              // per mesh: sample count
   uint32_t partBase;
   uint32_t screenMin;        // targets with at least this many triangles are searched by clusters
-  uint32_t orderedMin;       // in targets with at least this many, a sliver counts when it is within reach
+  uint32_t orderedMin;       // in targets with at least this many, with slivers, what is within reach counts
   const uint32_t* triOff;    // per mesh: first entry of its triangles below (a multiple of 32)
-  uint32_t* cnt;             // per triangle: its area, then its samples
+  uint32_t* cnt;             // per triangle: its area, its samples, then its sorted number (bit 31: a sliver)
   uint32_t* soff;            // per triangle: its cell, then (sorted) its first sample
   uint32_t* perm;            // sorted triangles' indices
-  uint32_t* bad;             // per mesh: its slivers, as sorted triangles' numbers
-  uint32_t* nBad;            // per mesh: how many
+  uint32_t* slivers;         // per mesh: 1 when it has slivers
   float4* triC;              // sorted triangles: centroid, radius (negative: a sliver)
   float4* triG;              // sorted triangles: three corners
-  float4* box;               // per cluster of 32 sorted triangles: low and high corner
+  float4* box;               // per cluster of 32 sorted triangles: low and high corner (w: has slivers)
+  float4* triO;              // where that matters: the centroids and radii in the triangles' own order
+  float4* boxO;              // and per 32 of them, their box (w of the low corner: the largest radius)
   uint32_t* tilePre;         // prefix of the meshes' 32-sample tiles (nMeshes + 1)
   uint32_t* work;            // next tile
 };

@@ -17,12 +17,15 @@
 //   k_hd_near   a warp per 32 samples: the clusters whose box may hold a
 //               nearest triangle, nearest box first, a centroid test per
 //               triangle, tri_sq for the survivors; a sample whose distance
-//               cannot exceed the pair's largest one so far is dropped.
+//               cannot exceed the pair's largest one so far is dropped. In a
+//               target with slivers the samples that are left, and those
+//               whose nearest triangle a sliver may rule out, go through its
+//               triangles in order (hd_ordered).
 // What bounds it: dependent loads and divergence in k_hd_near. Against a
 // tensor-core bound of every sample-triangle pair, whose epilogue was bound by
 // instruction issue: 24 cut halves of 1.5-30k triangles with their hulls
-// 11.4 -> 1.28 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.82 ms, 192
-// pairs of 160-6,000 triangles 5.8 + 0.71 -> 0.90 ms.
+// 11.4 -> 1.64 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.96 ms, 192
+// pairs of 160-6,000 triangles 5.8 + 0.71 -> 1.12 ms.
 #include <algorithm>
 
 #include "cuacd_dev.cuh"
@@ -70,6 +73,12 @@ __device__ __forceinline__ float tri_sq(f3 p, f3 a, f3 b, f3 c) {
   }
   return fminf(seg_sq(p, a, b), fminf(seg_sq(p, b, c), seg_sq(p, c, a)));
 }
+
+// the same as a call, for the few evaluations outside the search's loop:
+// k_hd_near waits for instructions more than for anything else (5.8 of 12.1
+// cycles an instruction with eight copies of tri_sq), so the search has one
+// copy of its visit and of tri_sq
+__device__ __noinline__ float tri_sq_at(f3 p, const float4* g) { return tri_sq(p, xyz(g[0]), xyz(g[1]), xyz(g[2])); }
 
 // ---------------------------------------------------------------------------
 // prep
@@ -289,6 +298,7 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
       const uint32_t i = i0 + 32 * u;
       N[u] = 0;
       f3 blo = mk3(3.4e38f, 3.4e38f, 3.4e38f), bhi = mk3(-3.4e38f, -3.4e38f, -3.4e38f);
+      bool sliver = false;
       if (i < nt) {
         const uint32_t t = perm[i];
         f3 a, b, c;
@@ -310,14 +320,15 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
         }
         // a sliver (the angle at a below 0.57 degrees) or a degenerate
         // triangle: tri_sq may be far off its geometry (HdNear), so it is
-        // marked by a negative radius and listed
+        // marked by a negative radius
         const f3 ab = b - a, ac = c - a, nn = cross(ab, ac);
         const float n2 = dot(nn, nn);
         if (!(n2 > 1e-4f * dot(ab, ab) * dot(ac, ac)) || n2 < 1.1e-20f) {
           r = -r;
+          sliver = true;
           sBad = 1;
         }
-        cnt[t] = i | (r < 0.0f ? 0x80000000u : 0u);  // its samples have been read
+        cnt[t] = i | (sliver ? 0x80000000u : 0u);  // its samples have been read
         float4* G = A.triG + 3 * (base + i);
         G[0] = make_float4(a.x, a.y, a.z, 0.0f);
         G[1] = make_float4(b.x, b.y, b.z, 0.0f);
@@ -331,10 +342,11 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
         const float4 h = make_float4(f_unord(__reduce_max_sync(FULLMASK, f_ord(bhi.x))),
                                      f_unord(__reduce_max_sync(FULLMASK, f_ord(bhi.y))),
                                      f_unord(__reduce_max_sync(FULLMASK, f_ord(bhi.z))), 0.0f);
+        const bool has = __any_sync(FULLMASK, sliver);
         if (lane == 0) {
           float4* B = A.box + 2 * (size_t)((base + i) >> 5);
           B[0] = l;
-          B[1] = h;
+          B[1] = make_float4(h.x, h.y, h.z, has ? 1.0f : 0.0f);
         }
       }
       const uint32_t inc = warp_incl_u(N[u], lane);
@@ -350,16 +362,31 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
       if (i0 + 32 * u < nt) soff[i0 + 32 * u] = run + before + off[u];
     run += tot;
   }
-  // the slivers in the triangles' own order (behind the last scan's barriers)
-  run = 0;
-  for (uint32_t c0 = 0; sBad != 0 && c0 < nt; c0 += HD_PREP) {
-    const uint32_t v = c0 + tid < nt ? cnt[c0 + tid] : 0u;
-    uint32_t tot;
-    const uint32_t at = run + prep_scan(v >> 31, ws, &tot) - 1;
-    if (v >> 31) A.bad[base + at] = v & 0x7fffffffu;
-    run += tot;
+  if (tid == 0) A.slivers[m] = sBad;
+  // a target with slivers: its triangles' centroids in their own order, with a
+  // box and the largest radius per 32 (behind the last scan's barriers)
+  if (sBad == 0 || nt < A.orderedMin) return;
+  for (uint32_t t0 = 32 * warp; t0 < nt; t0 += HD_PREP) {
+    const uint32_t t = t0 + lane;
+    float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (t < nt) {
+      c = A.triC[base + (cnt[t] & 0x7fffffffu)];
+      A.triO[base + t] = c;
+    }
+    const int lo3 = f_ord(3.4e38f), hi3 = f_ord(-3.4e38f);
+    const float4 l = make_float4(f_unord(__reduce_min_sync(FULLMASK, t < nt ? f_ord(c.x) : lo3)),
+                                 f_unord(__reduce_min_sync(FULLMASK, t < nt ? f_ord(c.y) : lo3)),
+                                 f_unord(__reduce_min_sync(FULLMASK, t < nt ? f_ord(c.z) : lo3)),
+                                 __uint_as_float(__reduce_max_sync(FULLMASK, __float_as_uint(fabsf(c.w)))));
+    const float4 h = make_float4(f_unord(__reduce_max_sync(FULLMASK, t < nt ? f_ord(c.x) : hi3)),
+                                 f_unord(__reduce_max_sync(FULLMASK, t < nt ? f_ord(c.y) : hi3)),
+                                 f_unord(__reduce_max_sync(FULLMASK, t < nt ? f_ord(c.z) : hi3)), 0.0f);
+    if (lane == 0) {
+      float4* B = A.boxO + 2 * (size_t)((base + t0) >> 5);
+      B[0] = l;
+      B[1] = h;
+    }
   }
-  if (tid == 0) A.nBad[m] = run;
 }
 
 // tiles of 32 samples per mesh: their prefix over the meshes, and the work
@@ -414,29 +441,46 @@ __global__ void __launch_bounds__(1024) k_hd_tiles(const HdArgs A, const Dev D) 
 // s^2 in length, so a point taken for one above the triangle lies within 6e-4
 // |p - a| of it, 4e-7 of the squared distance. For a sliver the normal can
 // be noise and the plane distance anything, and a triangle with |n|^2 < 1e-20
-// counts by its corners alone: such triangles give no ub, and the samples that
-// could still raise the pair's largest distance meet them at last, in the
-// triangles' order. In a target below A.orderedMin triangles every one counts,
-// as in an exhaustive search; in a larger one it counts within reach (HdReach)
-// only. Parts that have been cut again and again hold hundreds of slivers, and
+// counts by its corners alone: such triangles give no ub here. In a target
+// below A.orderedMin triangles every one counts, as in an exhaustive search;
+// in a larger one what counts is decided in the triangles' order (HdReach,
+// hd_ordered). Parts that have been cut again and again are mostly slivers, and
 // with every one counted the noise of far ones made the distances of 9 parts
 // in 90 decompositions up to 32 % smaller than they are in 64 bits. Either way
 // the distance does not depend on the order in which the tiles run.
 struct HdNear {
   f3 p;
   float p2, best, ub;
-  uint32_t at;  // the triangle that gave best (the first of equal ones)
+  // the smallest |p - c|^2 of the slivers met, and the sorted numbers of that
+  // sliver and of the triangles that gave best and ub
+  float sliver;
+  uint32_t atSliver, atBest, atUb;
   __device__ __forceinline__ float reach() const { return fminf(best, ub) * 1.001f + 3e-10f * p2 + 1e-30f; }
   // whether the sample can still raise the pair's largest distance
   __device__ __forceinline__ bool counts(float gmax) const { return best > gmax && !(ub + 3e-9f * p2 < gmax); }
+  // for a sample that cannot: the triangle that shows it, and its lower bound
+  __device__ __forceinline__ uint32_t shows(float gmax) const { return best > gmax ? atUb : atBest; }
+  __device__ __forceinline__ float lower(float4 c) const {
+    const f3 d = p - mk3(c.x, c.y, c.z);
+    const float lo = sqrtf(dot(d, d)) - fabsf(c.w);
+    return lo > 0.0f ? lo * lo : 0.0f;
+  }
+  __device__ __forceinline__ void meet(float d2, uint32_t i) {
+    if (d2 < sliver) {
+      sliver = d2;
+      atSliver = i;
+    }
+  }
 };
 
-// A sliver's reach: what a search of the triangles in order, by centroids, lets
-// through. With a margin e of 2^-13 (|p|^2 + |c|^2 + 2 |p|_1 |c|_1) on squared
-// centroid distances, triangle t counts when its bound (sqrt(|p - c|^2 - e) -
-// r)^2 is not above the smallest tri_sq before t's 32 triangles or the smallest
-// |p - c|^2 + e up to t. For any other triangle the rule changes nothing, as
-// one that is out of reach is not the nearest.
+// What counts in a target with slivers, of at least A.orderedMin triangles: what
+// a search of the triangles in order, 32 at a time, lets through by their
+// centroids. With a margin e of 2^-13 (|p|^2 + |c|^2 + 2 |p|_1 |c|_1) on squared
+// centroid distances, a triangle counts when its bound (sqrt(|p - c|^2 - e) -
+// r)^2 is not above the smallest tri_sq of the 32s before and not above the
+// smallest |p - c|^2 + e up to its own. Of ordinary triangles alone, one that
+// is out of reach is not the nearest; but a sliver's tri_sq can lie on either
+// side of its bounds, so it decides what comes after it.
 struct HdReach {
   float lb, ub, slack;
   __device__ __forceinline__ HdReach(f3 p, float p2, float p1, float4 c4) {
@@ -460,10 +504,77 @@ __device__ __forceinline__ float box_gap(f3 alo, f3 ahi, float4 blo, float4 bhi)
   return dx * dx + dy * dy + dz * dz;
 }
 
+// One warp: the smallest tri_sq of the triangles that count for the point p, or
+// any value not above gmax once it is known not to be. 32 triangles are passed
+// over when the box of their centroids and their largest radius put every lower
+// bound above the smallest distance and upper bound so far: then none counts, and
+// no upper bound is smaller. (e is at least 3.7 times what |p - c|^2 is off
+// by, so 1.5 e and the margins below cover both.) What bounds it: dependent
+// loads, 1,024 triangles a step where all are passed over. Every sliver
+// against every sample in turn, 1,200 cycles a sliver, took 740 ms for 96
+// unions of parts cut 30 times with their hulls (1.3 M triangles, two thirds
+// slivers); this takes 11 ms, and the tensor-core bound took 43.
+__device__ __noinline__ float hd_ordered(const float4* O, const float4* B, const float4* G, const uint32_t* at,
+                                         uint32_t tnt, f3 p, float gmax, uint32_t& exact, uint32_t& met) {
+  const uint32_t lane = threadIdx.x & 31;
+  const float p2 = dot(p, p), p1 = l1(p);
+  const uint32_t nb = (tnt + 31) / 32;
+  float best = 3.4e38f, up = 3.4e38f;
+  uint32_t nExact = 0, nMet = 0;
+  for (uint32_t g0 = 0; g0 < nb; g0 += 32) {
+    const uint32_t g = g0 + lane;
+    float lb = 0.0f, slack = 0.0f;
+    if (g < nb) {
+      const float4 l = B[2 * g], h = B[2 * g + 1];
+      const f3 c = mk3(fmaxf(fabsf(l.x), fabsf(h.x)), fmaxf(fabsf(l.y), fabsf(h.y)), fmaxf(fabsf(l.z), fabsf(h.z)));
+      const float c2 = dot(c, c), e = 1.83e-4f * (p2 + c2 + 2.0f * p1 * l1(c));
+      const float lo = sqrtf(fmaxf(0.9999f * box_gap(p, p, l, h) - e, 0.0f)) - 1.0001f * l.w;
+      lb = lo > 0.0f ? lo * lo : 0.0f;
+      slack = 1.1e-10f * (p2 + c2) + 2e-30f;
+    }
+    auto near = [&]() { return g < nb && !(lb > fminf(best, up) * 1.0011f + slack); };
+    unsigned todo = __ballot_sync(FULLMASK, near());
+    while (todo) {
+      const uint32_t j = __ffs(todo) - 1;
+      const uint32_t t = 32 * (g0 + j) + lane;
+      float lbT = 3.4e38f, ubT = 3.4e38f, slackT = 0.0f;
+      uint32_t i = 0;
+      if (t < tnt) {
+        i = at[t] & 0x7fffffffu;
+        const HdReach R(p, p2, p1, O[t]);
+        lbT = R.lb;
+        ubT = fminf(ubT, R.ub);
+        slackT = R.slack;
+      }
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const float u = __shfl_up_sync(FULLMASK, ubT, o);
+        if ((int)lane >= o) ubT = fminf(ubT, u);
+      }
+      ubT = fminf(ubT, up);  // the smallest upper bound up to the lane's triangle
+      float v = 3.4e38f;
+      if (t < tnt && lbT <= fminf(best, ubT) * 1.001f + slackT) {
+        v = fminf(v, tri_sq_at(p, G + 3 * (size_t)i));
+        nExact++;
+      }
+      nMet += 32;
+      up = __shfl_sync(FULLMASK, ubT, 31);
+      best = fminf(best, __uint_as_float(__reduce_min_sync(FULLMASK, __float_as_uint(v))));
+      if (best <= gmax) break;
+      todo = __ballot_sync(FULLMASK, near()) & ~((2u << j) - 1u);
+    }
+    if (best <= gmax) break;
+  }
+  exact = nExact;
+  met = nMet;
+  return best;
+}
+
 // Warps take tiles of 32 samples from the work list. Targets below
 // A.screenMin triangles are searched exhaustively; for them the sort's boxes
-// save nothing that the extra steps do not cost.
-__global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D) {
+// save nothing that the extra steps do not cost. Seven blocks an SM: 192 halves
+// of 96 icosphere cuts 0.96 ms, with six 0.98, with five 1.03.
+__global__ void __launch_bounds__(HD_NEAR, 7) k_hd_near(const HdArgs A, const Dev D) {
   __shared__ float4 sCent[HD_NEAR / 32][32];
   const uint32_t lane = threadIdx.x & 31;
   float4* cent = sCent[threadIdx.x >> 5];
@@ -524,11 +635,16 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
       continue;
     }
     S.p2 = dot(S.p, S.p);
-    S.best = 3.4e38f;
-    S.ub = 3.4e38f;
-    S.at = 0xffffffffu;
-    const bool ordered = tnt >= A.orderedMin;
-    const uint32_t* order = A.perm + tb;
+    S.best = S.ub = S.sliver = 3.4e38f;
+    S.atSliver = S.atBest = S.atUb = 0;
+    const bool slivers = A.slivers[dst] != 0, ordered = slivers && tnt >= A.orderedMin;
+    uint32_t why = 0;  // of a sample dropped: the triangle that shows why
+    auto settle = [&](float gmax) {
+      if (active && !S.counts(gmax)) {
+        active = false;
+        why = S.shows(gmax);
+      }
+    };
     const float4* C = A.triC + tb;
     const float4* B = A.box + 2 * (tb >> 5);
     const uint32_t nc = (tnt + 31) / 32;
@@ -548,50 +664,59 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
         const float d2 = dot(d, d);
         if (d2 < dmin && g.w >= 0.0f) { dmin = d2; jmin = j; }
       }
-      if (dmin < 3.4e38f) S.ub = fminf(S.ub, dmin * 1.02f + 1e-7f * cent[jmin].w * cent[jmin].w);
-      active = active && S.counts(gmax);
+      const float rmin = cent[jmin].w, ubMin = dmin * 1.02f + 1e-7f * rmin * rmin;
+      if (dmin < 3.4e38f && ubMin < S.ub) {
+        S.ub = ubMin;
+        S.atUb = 32 * c + jmin;
+      }
+      settle(gmax);
+      unsigned of = ordered ? __ballot_sync(FULLMASK, cent[lane].w < 0.0f) : 0u;
+      while (of) {
+        const uint32_t j = __ffs(of) - 1;
+        of &= of - 1;
+        const f3 d = S.p - xyz(cent[j]);
+        S.meet(dot(d, d), 32 * c + j);
+      }
       const unsigned any = __ballot_sync(FULLMASK, active);
       nScreen += (unsigned long long)__popc(any) * cn;  // the same on every lane
       if (any == 0) return;
-      auto exact = [&](uint32_t j) {
-        const float4* g = G + 3 * (size_t)(32 * c + j);
-        const float4 a = g[0], b = g[1], cc = g[2];
-        const float v = tri_sq(S.p, xyz(a), xyz(b), xyz(cc));
-        if (ordered && v <= S.best) {
-          const uint32_t t = order[32 * c + j];
-          S.at = v < S.best ? t : min(S.at, t);
+      // pass 0: the nearest centroid's; pass 1: those within reach then
+      uint32_t keep = active && dmin < 3.4e38f ? 1u << jmin : 0u;
+      float rs = 3.4e38f;
+#pragma unroll 1
+      for (int pass = 0; pass < 2; pass++) {
+        if (pass) {
+          if (__ballot_sync(FULLMASK, active) == 0) return;
+          rs = sqrtf(S.reach());
+          keep = 0;
+          for (uint32_t j = 0; j < cn; j++) {
+            const float4 g = cent[j];
+            const f3 d = S.p - mk3(g.x, g.y, g.z);
+            const float q = rs + fabsf(g.w);
+            if (!(dot(d, d) > q * q * 1.00001f) && !(ordered && g.w < 0.0f)) keep |= 1u << j;
+          }
+          if (dmin < 3.4e38f) keep &= ~(1u << jmin);
+          if (!active) keep = 0;
         }
-        S.best = fminf(S.best, v);
-        nExact++;
-      };
-      if (active && dmin < 3.4e38f) {
-        exact(jmin);
-        active = S.counts(gmax);
-      }
-      if (__ballot_sync(FULLMASK, active) == 0) return;
-      float rs = sqrtf(S.reach());
-      uint32_t keep = 0;
-      for (uint32_t j = 0; j < cn; j++) {
-        const float4 g = cent[j];
-        const f3 d = S.p - mk3(g.x, g.y, g.z);
-        const float q = rs + fabsf(g.w);
-        if (!(dot(d, d) > q * q * 1.00001f) && !(ordered && g.w < 0.0f)) keep |= 1u << j;
-      }
-      if (dmin < 3.4e38f) keep &= ~(1u << jmin);
-      if (!active) keep = 0;
-      while (keep) {
-        const uint32_t j = __ffs(keep) - 1;
-        keep &= keep - 1;
-        const float4 g = cent[j];
-        const f3 d = S.p - mk3(g.x, g.y, g.z);
-        const float q = rs + fabsf(g.w);
-        if (dot(d, d) > q * q * 1.00001f) continue;
-        exact(j);
-        if (!S.counts(gmax)) {
-          active = false;
-          break;
+        while (keep) {
+          const uint32_t j = __ffs(keep) - 1;
+          keep &= keep - 1;
+          const float4 m = cent[j];
+          const f3 d = S.p - mk3(m.x, m.y, m.z);
+          const float q = rs + fabsf(m.w);
+          if (dot(d, d) > q * q * 1.00001f) continue;
+          const float4* g = G + 3 * (size_t)(32 * c + j);
+          const float4 a = g[0], b = g[1], cc = g[2];
+          const float v = tri_sq(S.p, xyz(a), xyz(b), xyz(cc));
+          if (v < S.best) {
+            S.best = v;
+            S.atBest = 32 * c + j;
+          }
+          nExact++;
+          settle(gmax);
+          if (!active) break;
+          if (pass) rs = sqrtf(S.reach());
         }
-        rs = sqrtf(S.reach());
       }
       __syncwarp();
     };
@@ -612,113 +737,118 @@ __global__ void __launch_bounds__(HD_NEAR) k_hd_near(const HdArgs A, const Dev D
       const uint32_t k = __reduce_min_sync(FULLMASK, bk);
       first = __reduce_min_sync(FULLMASK, bk == k ? bc : 0xffffffffu);
     }
-    visit(first);
-    unsigned act = __ballot_sync(FULLMASK, active);
-    float reach = 0.0f;
-    auto shrink = [&]() {  // the box and the reach of the samples left
-      const float inf = INFINITY;
-      wlo = mk3(warp_box_min(active ? S.p.x : inf), warp_box_min(active ? S.p.y : inf), warp_box_min(active ? S.p.z : inf));
-      whi = mk3(warp_box_max(active ? S.p.x : -inf), warp_box_max(active ? S.p.y : -inf), warp_box_max(active ? S.p.z : -inf));
-      reach = __uint_as_float(__reduce_max_sync(FULLMASK, active ? __float_as_uint(S.reach()) : 0u));
-    };
-    if (act) shrink();
-    for (uint32_t c0 = 0; c0 < nc && act; c0 += 32) {
-      const uint32_t c = c0 + lane;
-      float gap = 0.0f;
-      bool need = false;
-      if (c < nc && c != first) {
-        gap = box_gap(wlo, whi, B[2 * c], B[2 * c + 1]);
-        need = !(gap > reach);
+    // the nearest cluster, then those that the samples left may need: the
+    // nearest box of 32 boxes first
+    float reach = 0.0f, gap = 0.0f;
+    unsigned act = 0;
+    bool need = false;
+    for (uint32_t c = first, c0 = 0xffffffe0u; c != 0xffffffffu;) {
+      visit(c);
+      const unsigned left = __ballot_sync(FULLMASK, active);
+      if (left != act) {  // the box of the samples left
+        act = left;
+        if (act == 0) break;
+        const float inf = INFINITY;
+        wlo = mk3(warp_box_min(active ? S.p.x : inf), warp_box_min(active ? S.p.y : inf), warp_box_min(active ? S.p.z : inf));
+        whi = mk3(warp_box_max(active ? S.p.x : -inf), warp_box_max(active ? S.p.y : -inf), warp_box_max(active ? S.p.z : -inf));
       }
-      unsigned todo = __ballot_sync(FULLMASK, need);
-      while (todo) {
-        // nearest box first
+      reach = __uint_as_float(__reduce_max_sync(FULLMASK, active ? __float_as_uint(S.reach()) : 0u));
+      need = need && !(gap > reach);
+      for (c = 0xffffffffu; c == 0xffffffffu;) {
+        if (__ballot_sync(FULLMASK, need) == 0) {
+          c0 += 32;
+          if (c0 >= nc) break;
+          const uint32_t n = c0 + lane;
+          if (n < nc && n != first) {
+            gap = box_gap(wlo, whi, B[2 * n], B[2 * n + 1]);
+            need = !(gap > reach);
+          }
+          continue;
+        }
         const uint32_t key = need ? __float_as_uint(gap) : 0xffffffffu;
         const uint32_t k = __reduce_min_sync(FULLMASK, key);
         const uint32_t j = __ffs(__ballot_sync(FULLMASK, key == k && need)) - 1;
         if (lane == j) need = false;
         const float4 l = B[2 * (c0 + j)], h = B[2 * (c0 + j) + 1];
-        if (__any_sync(FULLMASK, active && !(box_gap(S.p, S.p, l, h) > S.reach()))) {
-          visit(c0 + j);
-          const unsigned a2 = __ballot_sync(FULLMASK, active);
-          if (a2 == 0) { act = 0; break; }
-          if (a2 != act) {
-            act = a2;
-            shrink();
-          } else {
-            reach = __uint_as_float(__reduce_max_sync(FULLMASK, active ? __float_as_uint(S.reach()) : 0u));
-          }
-          need = need && !(gap > reach);
-        }
-        todo = __ballot_sync(FULLMASK, need);
+        if (__any_sync(FULLMASK, active && !(box_gap(S.p, S.p, l, h) > S.reach()))) c = c0 + j;
       }
     }
-    // what is left against the target's slivers
-    const uint32_t nBad = act ? A.nBad[dst] : 0u;
-    if (nBad != 0 && ordered) {
-      const float p1 = l1(S.p);
-      // smallest distance before the current 32 triangles, slivers counted; a
-      // bound by the slivers' centroids
-      const float nearest = S.best;
-      float before = nearest, sub = 3.4e38f;
-      float prefix = 3.4e38f;  // the last answer to the question below: later ones are no larger
-      uint32_t group = 0xffffffffu;
-      active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
-      for (uint32_t k = 0; k < nBad; k++) {
-        if ((k & 31u) == 0 && __ballot_sync(FULLMASK, active) == 0) break;
-        const uint32_t i = A.bad[tb + k], t = order[i];
-        const float4* g = G + 3 * (size_t)i;
-        const float4 a = g[0], b = g[1], c = g[2];
-        if ((t >> 5) != group) {
-          group = t >> 5;
-          before = S.best;
-        }
-        const HdReach R(S.p, S.p2, p1, C[i]);
-        sub = fminf(sub, R.ub);
-        const float v = tri_sq(S.p, xyz(a), xyz(b), xyz(c));
-        nExact += active ? 1u : 0u;
-        const bool lower = active && v < S.best;
-        bool in = lower && R.within(fminf(before, sub));
-        // out of reach of the nearest triangle of all, but not of the slivers
-        // so far: in if it is within reach of the triangles before it
-        unsigned ask = __ballot_sync(FULLMASK, lower && !in && R.within(fminf(sub, prefix)) && S.at >= (t & ~31u));
-        while (ask) {
-          const uint32_t l = __ffs(ask) - 1;
-          ask &= ask - 1;
-          const f3 p = mk3(__shfl_sync(FULLMASK, S.p.x, l), __shfl_sync(FULLMASK, S.p.y, l), __shfl_sync(FULLMASK, S.p.z, l));
-          const float p2 = dot(p, p), pl = l1(p);
-          float low = 3.4e38f;
-          for (uint32_t j = lane; j < tnt; j += 32) {
-            const uint32_t s = order[j];
-            if (s > t) continue;
-            const float4 cj = C[j];
-            const HdReach Q(p, p2, pl, cj);
-            low = fminf(low, Q.ub);
-            if (s >= (t & ~31u) || cj.w < 0.0f || !Q.within(low)) continue;
-            const float4* h = G + 3 * (size_t)j;
-            low = fminf(low, tri_sq(p, xyz(h[0]), xyz(h[1]), xyz(h[2])));
+    if (ordered) {
+      // A dropped sample stays dropped unless a sliver's upper bound may be
+      // below the lower bound of the triangle u that dropped it, which then may
+      // not count. The sliver whose centroid is nearest is the one to ask: no
+      // upper bound of another sliver is below its lower bound, so either it
+      // counts, or something nearer than u does. The clusters that the search
+      // did not need are looked at for it.
+      settle(__uint_as_float(__ldcg(gmaxAt)));
+      const bool dropped = s0 + lane < ns && !active;
+      const float shown = dropped ? S.lower(C[why]) : 0.0f;
+      const float far = __uint_as_float(__reduce_max_sync(FULLMASK, dropped ? __float_as_uint(shown) : 0u));
+      if (far > 0.0f) {
+        const float inf = INFINITY;
+        const bool d = dropped;
+        wlo = mk3(warp_box_min(d ? S.p.x : inf), warp_box_min(d ? S.p.y : inf), warp_box_min(d ? S.p.z : inf));
+        whi = mk3(warp_box_max(d ? S.p.x : -inf), warp_box_max(d ? S.p.y : -inf), warp_box_max(d ? S.p.z : -inf));
+        for (uint32_t c0 = 0; c0 < nc; c0 += 32) {
+          const uint32_t c = c0 + lane;
+          bool need = false;
+          if (c < nc) {
+            const float4 l = B[2 * c], h = B[2 * c + 1];
+            need = h.w != 0.0f && !(box_gap(wlo, whi, l, h) >= far);
           }
-          low = f_unord(__reduce_min_sync(FULLMASK, f_ord(low)));
-          // a sliver counted before has made its distance the bound
-          if (lane == l) {
-            prefix = low;
-            in = R.within(before < nearest ? fminf(low, before) : low);
+          unsigned todo = __ballot_sync(FULLMASK, need);
+          while (todo) {
+            const uint32_t k = c0 + __ffs(todo) - 1;
+            todo &= todo - 1;
+            const bool open = dropped && !(box_gap(S.p, S.p, B[2 * k], B[2 * k + 1]) >= fminf(shown, S.sliver));
+            if (!__any_sync(FULLMASK, open)) continue;
+            const float4 m = 32 * k + lane < tnt ? C[32 * k + lane] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            unsigned of = __ballot_sync(FULLMASK, m.w < 0.0f);
+            while (of) {
+              const uint32_t j = __ffs(of) - 1;
+              of &= of - 1;
+              const f3 q = S.p - mk3(__shfl_sync(FULLMASK, m.x, j), __shfl_sync(FULLMASK, m.y, j),
+                                     __shfl_sync(FULLMASK, m.z, j));
+              S.meet(dot(q, q), 32 * k + j);
+            }
           }
-        }
-        if (in) {
-          S.best = v;
-          active = S.counts(__uint_as_float(__ldcg(gmaxAt)));
         }
       }
-    } else if (nBad != 0) {
+      bool open = dropped && shown > S.sliver;
+      if (open) {
+        open = !(tri_sq_at(S.p, G + 3 * (size_t)S.atSliver) <= __uint_as_float(__ldcg(gmaxAt)));
+        nExact++;
+      }
+      // the others in the triangles' order, the one that is farthest first
+      unsigned left = __ballot_sync(FULLMASK, active || open);
+      while (left) {
+        const uint32_t k = __reduce_max_sync(FULLMASK, ((left >> lane) & 1u) ? __float_as_uint(S.best) : 0u);
+        const uint32_t l = __ffs(__ballot_sync(FULLMASK, ((left >> lane) & 1u) && __float_as_uint(S.best) == k)) - 1;
+        left &= ~(1u << l);
+        const float gmax = __uint_as_float(__ldcg(gmaxAt));
+        if (__shfl_sync(FULLMASK, active && !S.counts(gmax) && !(S.lower(C[S.shows(gmax)]) > S.sliver), l)) continue;
+        const f3 p = mk3(__shfl_sync(FULLMASK, S.p.x, l), __shfl_sync(FULLMASK, S.p.y, l), __shfl_sync(FULLMASK, S.p.z, l));
+        uint32_t exact, met;
+        const float best = hd_ordered(A.triO + tb, A.boxO + 2 * (tb >> 5), G, A.cnt + tb, tnt, p, gmax, exact, met);
+        nExact += exact;
+        nScreen += met;
+        if (best > gmax && lane == 0) atomicMax(gmaxAt, __float_as_uint(best));
+      }
+      active = false;
+    } else if (slivers && act) {
+      // every sliver of a small target
       active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
-      for (uint32_t k = 0; k < nBad; k++) {
-        if ((k & 31u) == 0 && __ballot_sync(FULLMASK, active) == 0) break;
-        const float4* g = G + 3 * (size_t)A.bad[tb + k];
-        const float4 a = g[0], b = g[1], c = g[2];
-        if (active) {
-          S.best = fminf(S.best, tri_sq(S.p, xyz(a), xyz(b), xyz(c)));
-          nExact++;
+      for (uint32_t t0 = 0; t0 < tnt && __ballot_sync(FULLMASK, active) != 0; t0 += 32) {
+        const uint32_t w = t0 + lane < tnt ? A.cnt[tb + t0 + lane] : 0u;
+        unsigned of = __ballot_sync(FULLMASK, w >> 31);
+        while (of) {
+          const uint32_t j = __ffs(of) - 1;
+          of &= of - 1;
+          const uint32_t i = __shfl_sync(FULLMASK, w, j) & 0x7fffffffu;
+          if (active) {
+            S.best = fminf(S.best, tri_sq_at(S.p, G + 3 * (size_t)i));
+            nExact++;
+          }
         }
       }
     }
