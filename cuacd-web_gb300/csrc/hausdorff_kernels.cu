@@ -24,8 +24,10 @@
 // What bounds it: dependent loads and divergence in k_hd_near. Against a
 // tensor-core bound of every sample-triangle pair, whose epilogue was bound by
 // instruction issue: 24 cut halves of 1.5-30k triangles with their hulls
-// 11.4 -> 1.64 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.96 ms, 192
-// pairs of 160-6,000 triangles 5.8 + 0.71 -> 1.12 ms.
+// 11.4 -> 1.66 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.98 ms, 192
+// pairs of 160-6,000 triangles 5.8 + 0.71 -> 1.14 ms.
+#include <cuda_bf16.h>
+
 #include <algorithm>
 
 #include "cuacd_dev.cuh"
@@ -480,12 +482,23 @@ struct HdNear {
 // r)^2 is not above the smallest tri_sq of the 32s before and not above the
 // smallest |p - c|^2 + e up to its own. Of ordinary triangles alone, one that
 // is out of reach is not the nearest; but a sliver's tri_sq can lie on either
-// side of its bounds, so it decides what comes after it.
+// side of its bounds, so it decides what comes after it, and the rule is one
+// of values: |p - c|^2 is |p|^2 - 2 p.c + |c|^2 with p, -2c and |c|^2 taken to
+// two bfloat16 terms each, as a bfloat16 contraction forms it (up to 6.5e-5
+// |p|_1 |c|_1 from the plain one, which settled one in 60 of the parts of a
+// mesh cut 30 times differently).
+__device__ __forceinline__ float bf16_two(float x) {
+  const float hi = __bfloat162float(__float2bfloat16_rn(x));
+  return hi + __bfloat162float(__float2bfloat16_rn(x - hi));  // exact: within 24 bits
+}
+__device__ __forceinline__ f3 bf16_two(f3 v) { return mk3(bf16_two(v.x), bf16_two(v.y), bf16_two(v.z)); }
 struct HdReach {
   float lb, ub, slack;
-  __device__ __forceinline__ HdReach(f3 p, float p2, float p1, float4 c4) {
-    const f3 c = mk3(c4.x, c4.y, c4.z), d = p - c;
-    const float c2 = dot(c, c), q = dot(d, d), e = 1.220703125e-4f * (p2 + c2 + 2.0f * p1 * l1(c));
+  // pt: the point to two terms
+  __device__ __forceinline__ HdReach(f3 pt, float p2, float p1, float4 c4) {
+    const f3 c = mk3(c4.x, c4.y, c4.z);
+    const float c2 = dot(c, c), e = 1.220703125e-4f * (p2 + c2 + 2.0f * p1 * l1(c));
+    const float q = p2 + (dot(pt, bf16_two(-2.0f * c)) + bf16_two(c2));
     const float lo = sqrtf(fmaxf(q - e, 0.0f)) - fabsf(c4.w);
     lb = lo > 0.0f ? lo * lo : 0.0f;
     ub = q + e;
@@ -518,6 +531,7 @@ __device__ __noinline__ float hd_ordered(const float4* O, const float4* B, const
                                          uint32_t tnt, f3 p, float gmax, uint32_t& exact, uint32_t& met) {
   const uint32_t lane = threadIdx.x & 31;
   const float p2 = dot(p, p), p1 = l1(p);
+  const f3 pt = bf16_two(p);
   const uint32_t nb = (tnt + 31) / 32;
   float best = 3.4e38f, up = 3.4e38f;
   uint32_t nExact = 0, nMet = 0;
@@ -541,7 +555,7 @@ __device__ __noinline__ float hd_ordered(const float4* O, const float4* B, const
       uint32_t i = 0;
       if (t < tnt) {
         i = at[t] & 0x7fffffffu;
-        const HdReach R(p, p2, p1, O[t]);
+        const HdReach R(pt, p2, p1, O[t]);
         lbT = R.lb;
         ubT = fminf(ubT, R.ub);
         slackT = R.slack;
@@ -573,7 +587,7 @@ __device__ __noinline__ float hd_ordered(const float4* O, const float4* B, const
 // Warps take tiles of 32 samples from the work list. Targets below
 // A.screenMin triangles are searched exhaustively; for them the sort's boxes
 // save nothing that the extra steps do not cost. Seven blocks an SM: 192 halves
-// of 96 icosphere cuts 0.96 ms, with six 0.98, with five 1.03.
+// of 96 icosphere cuts 0.96 ms, with six 0.98 and with five 1.03.
 __global__ void __launch_bounds__(HD_NEAR, 7) k_hd_near(const HdArgs A, const Dev D) {
   __shared__ float4 sCent[HD_NEAR / 32][32];
   const uint32_t lane = threadIdx.x & 31;

@@ -246,3 +246,41 @@ def test_slivers_that_count_bound_what_follows(scenes):
         got = list(scenes.check(p, src, [(tri, val)]))
         assert len(got) == 1 and got[0][0] == corner
     assert n >= 3
+
+
+def tie(p, shell, needle, lb, width, rng):
+    """the sphere with the needle and, right before it in its 32 triangles, an
+    ordinary triangle whose upper bound is the needle's lower bound to a share
+    of `width`"""
+    d = rng.normal(size=3)
+    d /= np.linalg.norm(d)
+    shape = 0.01 * R * rng.normal(size=(3, 3))
+    lo, hi, goal = 0.0, 1.2 * R, lb * (1 + rng.uniform(-width, width)) / 1.001
+    for _ in range(60):
+        mid = (lo + hi) / 2
+        t = (p + mid * d + shape).astype(f32)
+        if bounds(p, t[None], False)[1][0] < goal:
+            lo = mid
+        else:
+            hi = mid
+    at = 2 * int(rng.integers(1, len(shell) // 2))
+    return np.concatenate([shell[:at], t[None], needle[None], shell[at:]]), at
+
+
+def test_reach_uses_split_coordinates(scenes):
+    """Where the two forms of |p - c|^2 decide differently, the split one does."""
+    n = 0
+    for seed, p, plain, needles, ns, rng, src, alone, base in scenes.all:
+        (lb, ub, _), other = bounds(p, needles, True), bounds(p, needles, False)
+        width = 2 * np.median(np.abs(lb - other[0]) / ub)
+        cases = []
+        for i in np.flatnonzero((alone < 0.9 * np.minimum(lb, base.min())) & (lb < 0.95 * R * R)
+                                & (lb > FLOOR ** 2)).tolist()[:16]:
+            for _ in range(24):
+                tri, at = tie(p, plain[:ns], needles[i], lb[i], width, rng)
+                val = np.insert(base[:ns], at, [direct_sq(p.astype(f64), tri[at]), alone[i]])
+                if not is_sliver(tri[at:at + 1])[0] and \
+                        differs(rule(bounds(p, tri, True), val), rule(bounds(p, tri, False), val)):
+                    cases.append((tri, val))
+        n += sum(1 for _ in scenes.check(p, src, cases)) if cases else 0
+    assert n >= 3, n
