@@ -820,9 +820,8 @@ __device__ __forceinline__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat
   const uint32_t x0 = P.cell_x(fbx0), x1 = P.cell_x(fbx1);
   const uint32_t y0 = P.cell_y(fby0), y1 = P.cell_y(fby1);
   // the nodes of one row of covered cells are contiguous in the grid's node
-  // list: up to 32 rows at once, their entries spread over the lanes (an ear
-  // covers a few rows of a few entries each), and the warp stops at the
-  // first 32 entries holding a node inside
+  // list: up to 32 rows at once (most ears cover a few rows of a few entries
+  // each), and the warp stops at the first 32 entries holding a node inside
   auto inside = [&](uint32_t q) -> bool {
     if (!(P.alive[q] & 1u) || q == a || q == b || q == c) return false;
     const float qxf = P.Xf[q], qyf = P.Yf[q];
@@ -874,15 +873,40 @@ __device__ __forceinline__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat
       if (lane >= d) inc += u;
     }
     const uint32_t total = __shfl_sync(CUT_FULL, inc, rows - 1), shift = e0 - (inc - len);
-    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+    // Rows of 16 entries and more on average one by one, shorter ones with
+    // their entries spread over the lanes, each lane searching for its row. (Every
+    // lane looked at every row for every 32 entries, 64 shuffles for an ear
+    // over 32 rows: batches of 5-8 cuts with caps of up to 12,000 edges
+    // 132, 158, 296, 992 and 2,830 ms; with the search 110, 136, 260, 971 and
+    // 2,402, with whole rows too 107, 126, 259, 782 and 2,447.)
+    const bool whole = total >= 16 * rows;
+    uint32_t row = 0, t0 = 0;  // the next entry: of the row, or of all
+    while (whole ? row < rows : t0 < total) {
       const uint32_t t = t0 + (uint32_t)lane;
-      uint32_t e = CUT_NONE;
-      for (uint32_t r = 0; r < rows; r++) {  // the row holding entry t: the first that ends behind it
-        const uint32_t end = __shfl_sync(CUT_FULL, inc, r), sh = __shfl_sync(CUT_FULL, shift, r);
-        if (t < end && e == CUT_NONE) e = t + sh;
+      uint32_t r = row;
+      bool in;
+      uint32_t e;
+      if (whole) {
+        const uint32_t n = __shfl_sync(CUT_FULL, len, row);
+        e = __shfl_sync(CUT_FULL, e0, row) + t;
+        in = t < n;
+        t0 += 32;
+        if (t0 >= n) {
+          t0 = 0;
+          row++;
+        }
+      } else {
+        for (uint32_t d = 16; d > 0; d >>= 1) {  // the first row that ends behind entry t
+          if (d >= rows) continue;               // the same for all lanes
+          const uint32_t end = __shfl_sync(CUT_FULL, inc, min(r + d, rows) - 1);
+          if (r + d < rows && t >= end) r += d;
+        }
+        e = t + __shfl_sync(CUT_FULL, shift, r);
+        in = t < total;
+        t0 += 32;
       }
-      const uint32_t q = e != CUT_NONE ? P.gNodes[e] : 0u;
-      const bool h = e != CUT_NONE && inside(q);
+      const uint32_t q = in ? P.gNodes[e] : 0u;
+      const bool h = in && inside(q);
       const uint32_t hb = __ballot_sync(CUT_FULL, h);
       if (hb) {
         hit = true;
