@@ -28,16 +28,16 @@ __device__ __forceinline__ void add_bytes(uint32_t* ctr, int slot, unsigned long
   atomicAdd(reinterpret_cast<unsigned long long*>(ctr + slot), b);
 }
 
-// PartDesc (shaders.ts:41-46), 16 words
-struct PartDesc {
+// PartDesc (shaders.ts:41-46), 16 words, read and written by 16-byte words
+struct alignas(16) PartDesc {
   uint32_t vOff, nv, tOff, nt;
   uint32_t eOff, ne;
   float meshVol, hullVol;
   uint32_t planeIds[4];
   uint32_t nPlanes, flags, pad0, pad1;
 };
-// ItemDesc (shaders.ts:48-53), 20 words
-struct ItemDesc {
+// ItemDesc (shaders.ts:48-53), 20 words, read and written by 16-byte words
+struct alignas(16) ItemDesc {
   uint32_t partIds[8];
   uint32_t np, srcPart, initialCut, nLevels;
   float levelCosts[4];

@@ -277,7 +277,7 @@ __device__ __forceinline__ void job_needs(const Level& P, const Dev& D, uint32_t
 // trees 0.39 and 0.21 ms.
 template <class T>
 __device__ __forceinline__ T load16(const T* p) {
-  static_assert(sizeof(T) % 16 == 0, "whole 16-byte words");
+  static_assert(sizeof(T) % 16 == 0 && alignof(T) >= 16, "whole 16-byte words, also of a local object");
   T t;
 #pragma unroll
   for (uint32_t k = 0; k < sizeof(T) / 16; k++) reinterpret_cast<uint4*>(&t)[k] = reinterpret_cast<const uint4*>(p)[k];
@@ -285,6 +285,7 @@ __device__ __forceinline__ T load16(const T* p) {
 }
 template <class T>
 __device__ __forceinline__ void store16(T* p, const T& t) {
+  static_assert(sizeof(T) % 16 == 0 && alignof(T) >= 16, "whole 16-byte words, also of a local object");
 #pragma unroll
   for (uint32_t k = 0; k < sizeof(T) / 16; k++) reinterpret_cast<uint4*>(p)[k] = reinterpret_cast<const uint4*>(&t)[k];
 }
