@@ -91,15 +91,21 @@ static const uint32_t HD_ORDERED_MIN = 256;
 // sample capacities follow from added on the device (k_hd_area, about 40 us
 // with its readback); smaller ones on the host, at 3.4 ns a triangle
 static const uint64_t HD_AREA_MIN = 16384;
-// parents with more points than this get a block per plan / emit job
+// Levels whose parents have more points than this add a part's flux over a
+// block's 256 lanes, the others over a warp's 32, in whichever form they run: a
+// float sum's lanes decide its rounding, so they follow from the size alone and
+// not from the schedule that the timing has picked. (The sums are compensated:
+// of 20,000 parts none differed between the two.)
 static const uint32_t BIG_JOB_NV = 2048;
 
 // Schedules the autotuner chooses between: the largest part a warp hulls
-// (larger ones go to blocks), the largest parent a warp plans and emits, and
-// the points from which warps hand parts beyond the register hull on to the
-// blocks, in a tree's levels and in hull batches.
-// The kernels' outputs do not depend on which group shape handles a part,
-// so every schedule gives the same results; they differ in speed with the
+// (larger ones go to blocks), the largest parent a warp may plan and emit (as
+// cuacd_tree_schedule states it; parents of WIDE_NV points and more take blocks
+// under each of them), and the points from which warps hand parts beyond the
+// register hull on to the blocks, in a tree's levels and in hull batches.
+// The hulls do not depend on which group shape handles a part, and the lanes of
+// plan's and emit's sums follow from the sizes (BIG_JOB_NV), so every schedule
+// gives the same results; they differ in speed with the
 // distribution of part sizes. The first is the fixed default. All but one hand
 // parts on: without it in the last two, 24 blobs of 8,000 triangles decomposed in
 // 96.9, 95.2, 99.6 and 126.5 ms a pass while trying schedule 0 to 3, with it in
@@ -578,7 +584,7 @@ struct Tree {
   }
 
   // parents shrink roughly by half per level
-  bool bigLevel(uint32_t l) const { return (maxSeedNv >> l) > bigJobNv(); }
+  bool bigLevel(uint32_t l) const { return (maxSeedNv >> l) > BIG_JOB_NV; }
   bool wideLevel(uint32_t l, uint32_t nJobs) const {
     return !bigLevel(l) && (nJobs <= WIDE_JOBS * (uint32_t)nSM || (maxSeedNv >> l) >= WIDE_NV);
   }

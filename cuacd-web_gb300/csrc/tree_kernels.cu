@@ -459,7 +459,9 @@ __global__ void __launch_bounds__(1024) k_scan(const Level P, const Dev D) {
 // (triangle t belongs to lane t mod LANES). A level of few jobs runs its
 // mid-sized parents on blocks with a warp's 32 lanes: the flux of each
 // triangle goes through shared memory and two warps add it in the warp
-// form's order, so a part's volume has the same bits whichever form it took.
+// form's order, so a part's volume has the same bits in both. Levels of large
+// parents (above 2,048 points) add over the block's own lanes, whose sums
+// round differently; which of the two a level takes follows from its size.
 template <int G, int LANES>
 __global__ void __launch_bounds__(256, 3) k_emit(const Level P, const Dev D) {
   constexpr bool STAGED = LANES < G;
