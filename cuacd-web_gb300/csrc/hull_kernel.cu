@@ -862,9 +862,7 @@ __device__ __noinline__ uint32_t hull_grow(const HullCtx& h, HullSm& hs, GrpSmem
 //     of a round's time.) The pool is the 2 nv words of the owner and
 //     distance arrays; when the bump pointer would pass its end the live
 //     segments are gathered to its front.
-#ifndef BIG_VIS
 #define BIG_VIS 128u
-#endif
 #define BIG_HASH 256u
 #define BIG_NREC 32u
 struct BigSm {
@@ -904,9 +902,7 @@ struct BigSm {
 #define BAT_FACES 32u   // faces of a batched patch, one per lane
 #define BAT_NEW 32u     // its new faces, one per lane
 #define BAT_HASH_BITS 6u
-#ifndef KMAX_CAP
 #define KMAX_CAP 16u
-#endif
 template <int NW>
 struct BatDims {
   // picks per round: one per warp, at most KMAX_CAP
@@ -2407,7 +2403,6 @@ __device__ bool hull_one(const Level& P, const Dev& D, uint32_t idx, uint32_t* s
   // hull that outgrows the warp is built again from the simplex in the
   // slot-array form (the same sequence, so the same result)
   bool tiny = G == 32 && nv <= QC_MAX;
-  if (G == 32 && P.handOn && !tiny) return false;
 restart:
   // initial simplex (shaders.ts:1227-1263). The reference scans the 80 seeds
   // serially with strict comparisons, so each choice is the first seed
