@@ -649,7 +649,9 @@ __global__ void __launch_bounds__(HD_NEAR, 7) k_hd_near(const HdArgs A, const De
       continue;
     }
     S.p2 = dot(S.p, S.p);
-    S.best = S.ub = S.sliver = 3.4e38f;
+    // a small target's search starts where the exhaustive one does
+    S.best = tnt < A.orderedMin ? 1e30f : 3.4e38f;
+    S.ub = S.sliver = 3.4e38f;
     S.atSliver = S.atBest = S.atUb = 0;
     const bool slivers = A.slivers[dst] != 0, ordered = slivers && tnt >= A.orderedMin;
     uint32_t why = 0;  // of a sample dropped: the triangle that shows why
