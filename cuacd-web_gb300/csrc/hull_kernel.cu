@@ -2664,7 +2664,7 @@ restart:
 // short loops stay rolled, the simplex's four faces are one piece of code, and
 // its points on the grid always lie in one array (a second way to read them
 // was part of every point access; a part whose points fit neither shared memory
-// nor the slab goes to a block): 218 to 167 KB of code, 50,400 staircase children
+// nor the slab goes to a block): 218 to 169 KB of code, 50,400 staircase children
 // 0.74 to 0.58 ms.
 template <int G>
 __global__ void __launch_bounds__(G >= 512 ? G : 256, G == 1024 ? 1 : (G == 512 ? 2 : 4))
