@@ -76,9 +76,10 @@ typedef struct {
                                < 0: never, every triangle is evaluated). The
                                results do not depend on it but for slivers (an
                                angle below 0.57 degrees), whose float distance
-                               can be noise: one out of reach does not count in
-                               targets of 256 triangles and more (or of this
-                               many, when set) */
+                               can be noise: in targets of 256 triangles and
+                               more (or of this many, when set) with slivers, a
+                               triangle out of reach of those before it does
+                               not count */
   int32_t autotune;         /* 1 (the default): when warpMaxNv is 0, the
                                warp/block thresholds of the hull, of handing on
                                and of plan/emit are chosen per distribution of part
