@@ -879,34 +879,37 @@ __device__ __forceinline__ bool is_ear(const Ring& P, uint32_t k, bool allowFlat
     // over 32 rows: batches of 5-8 cuts with caps of up to 12,000 edges
     // 132, 158, 296, 992 and 2,830 ms; with the search 110, 136, 260, 971 and
     // 2,402, with whole rows too 107, 126, 259, 782 and 2,447.)
-    const bool whole = total >= 16 * rows;
-    uint32_t row = 0, t0 = 0;  // the next entry: of the row, or of all
-    while (whole ? row < rows : t0 < total) {
-      const uint32_t t = t0 + (uint32_t)lane;
-      uint32_t r = row;
-      bool in;
-      uint32_t e;
-      if (whole) {
-        const uint32_t n = __shfl_sync(CUT_FULL, len, row);
-        e = __shfl_sync(CUT_FULL, e0, row) + t;
-        in = t < n;
-        t0 += 32;
-        if (t0 >= n) {
-          t0 = 0;
-          row++;
+    // Many rows of 16 entries and more on average: one by one. (Spread over the
+    // lanes they cost 2 shuffles a row for every 32 entries: batches of 5-8 cuts
+    // with caps of up to 12,000 edges 130, 158, 296, 992 and 2,837 ms, one by one
+    // 116, 127, 271, 749 and 2,474; a binary search for the row 107, 126, 259, 782
+    // and 2,457, but 96 icosphere cuts and 12 blob cuts 1-3 % slower than this.)
+    if (rows > 8 && total >= 16 * rows) {
+      for (uint32_t row = 0; row < rows && !hit; row++) {
+        const uint32_t b0 = __shfl_sync(CUT_FULL, e0, row), b1 = b0 + __shfl_sync(CUT_FULL, len, row);
+        for (uint32_t base = b0; base < b1; base += 32) {
+          const uint32_t e = base + (uint32_t)lane;
+          const uint32_t q = e < b1 ? P.gNodes[e] : 0u;
+          const bool h = e < b1 && inside(q);
+          const uint32_t hb = __ballot_sync(CUT_FULL, h);
+          if (hb) {
+            hit = true;
+            hitQ = __shfl_sync(CUT_FULL, q, __ffs(hb) - 1);
+            break;
+          }
         }
-      } else {
-        for (uint32_t d = 16; d > 0; d >>= 1) {  // the first row that ends behind entry t
-          if (d >= rows) continue;               // the same for all lanes
-          const uint32_t end = __shfl_sync(CUT_FULL, inc, min(r + d, rows) - 1);
-          if (r + d < rows && t >= end) r += d;
-        }
-        e = t + __shfl_sync(CUT_FULL, shift, r);
-        in = t < total;
-        t0 += 32;
       }
-      const uint32_t q = in ? P.gNodes[e] : 0u;
-      const bool h = in && inside(q);
+      continue;
+    }
+    for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+      const uint32_t t = t0 + (uint32_t)lane;
+      uint32_t e = CUT_NONE;
+      for (uint32_t r = 0; r < rows; r++) {  // the row holding entry t: the first that ends behind it
+        const uint32_t end = __shfl_sync(CUT_FULL, inc, r), sh = __shfl_sync(CUT_FULL, shift, r);
+        if (t < end && e == CUT_NONE) e = t + sh;
+      }
+      const uint32_t q = e != CUT_NONE ? P.gNodes[e] : 0u;
+      const bool h = e != CUT_NONE && inside(q);
       const uint32_t hb = __ballot_sync(CUT_FULL, h);
       if (hb) {
         hit = true;
