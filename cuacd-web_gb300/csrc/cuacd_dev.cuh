@@ -113,10 +113,11 @@ struct HdArgs {
   uint32_t screenMin;        // targets with at least this many triangles are searched by clusters
   uint32_t orderedMin;       // in targets with at least this many, with slivers, what is within reach counts
   const uint32_t* triOff;    // per mesh: first entry of its triangles below (a multiple of 32)
-  uint32_t* cnt;             // per triangle: its area, its samples, then its sorted number (bit 31: a sliver)
+  uint32_t* cnt;             // per triangle: its area, its samples, then its sorted number
   uint32_t* soff;            // per triangle: its cell, then (sorted) its first sample
   uint32_t* perm;            // sorted triangles' indices
-  uint32_t* slivers;         // per mesh: 1 when it has slivers
+  uint32_t* slivers;         // per mesh: how many slivers it has
+  uint32_t* bad;             // their sorted numbers, in any order
   float4* triC;              // sorted triangles: centroid, radius (negative: a sliver)
   float4* triG;              // sorted triangles: three corners
   float4* box;               // per cluster of 32 sorted triangles: low and high corner (w: has slivers)

@@ -928,7 +928,7 @@ struct Tree {
   // triCap: per mesh, an upper bound on its triangles
   int runHd(uint32_t nPairs, uint32_t partBase, const std::vector<uint32_t>& capN, const std::vector<uint32_t>& triCap) {
     const uint32_t nm = 2 * nPairs;
-    // sample capacities, triangle offsets (host) | sample counts, sliver flags, tile prefix, work counter (device)
+    // sample capacities, triangle offsets (host) | sample counts, sliver counts, tile prefix, work counter (device)
     std::vector<uint32_t> hm(2 * (size_t)nm);
     std::memcpy(hm.data(), capN.data(), 4ull * nm);
     uint64_t nTri = 0;
@@ -941,7 +941,8 @@ struct Tree {
     const size_t cOff = up((5 * (size_t)nm + 2) * 4), gOff = cOff + (size_t)nTri * 16, boxOff = gOff + (size_t)nTri * 48;
     const size_t cntOff = boxOff + (size_t)nTri, soffOff = cntOff + (size_t)nTri * 4, permOff = soffOff + (size_t)nTri * 4;
     const size_t oOff = permOff + (size_t)nTri * 4, boxOOff = oOff + (size_t)nTri * 16;
-    int rc = bHd.ensure(boxOOff + (size_t)nTri + 16);
+    const size_t badOff = boxOOff + (size_t)nTri;
+    int rc = bHd.ensure(badOff + (size_t)nTri * 4 + 16);
     if (rc) return rc;
     uint8_t* d = (uint8_t*)bHd.p;
     uint32_t* meta = (uint32_t*)bHd.p;
@@ -963,6 +964,7 @@ struct Tree {
     A.box = (float4*)(d + boxOff);
     A.triO = (float4*)(d + oOff);
     A.boxO = (float4*)(d + boxOOff);
+    A.bad = (uint32_t*)(d + badOff);
     A.cnt = (uint32_t*)(d + cntOff);
     A.soff = (uint32_t*)(d + soffOff);
     A.perm = (uint32_t*)(d + permOff);

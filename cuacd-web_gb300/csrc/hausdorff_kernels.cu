@@ -24,8 +24,8 @@
 // What bounds it: dependent loads and divergence in k_hd_near. Against a
 // tensor-core bound of every sample-triangle pair, whose epilogue was bound by
 // instruction issue: 24 cut halves of 1.5-30k triangles with their hulls
-// 11.4 -> 1.66 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.98 ms, 192
-// pairs of 160-6,000 triangles 5.8 + 0.71 -> 1.14 ms.
+// 11.4 -> 1.48 ms, the 192 halves of 96 icosphere cuts 8.5 -> 0.83 ms, 192
+// pairs of 160-6,000 triangles 5.8 + 0.71 -> 1.02 ms.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -328,9 +328,9 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
         if (!(n2 > 1e-4f * dot(ab, ab) * dot(ac, ac)) || n2 < 1.1e-20f) {
           r = -r;
           sliver = true;
-          sBad = 1;
+          A.bad[base + atomicAdd(&sBad, 1u)] = i;
         }
-        cnt[t] = i | (sliver ? 0x80000000u : 0u);  // its samples have been read
+        cnt[t] = i;  // its samples have been read
         float4* G = A.triG + 3 * (base + i);
         G[0] = make_float4(a.x, a.y, a.z, 0.0f);
         G[1] = make_float4(b.x, b.y, b.z, 0.0f);
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(HD_PREP) k_hd_prep(const HdArgs A, const Dev D
     const uint32_t t = t0 + lane;
     float4 c = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (t < nt) {
-      c = A.triC[base + (cnt[t] & 0x7fffffffu)];
+      c = A.triC[base + cnt[t]];
       A.triO[base + t] = c;
     }
     const int lo3 = f_ord(3.4e38f), hi3 = f_ord(-3.4e38f);
@@ -425,6 +425,11 @@ __global__ void __launch_bounds__(1024) k_hd_tiles(const HdArgs A, const Dev D) 
 // nearest triangles
 
 #define HD_NEAR 128u
+// slivers of a target that a sample asks one by one before it goes through the
+// target in order: 32 steps of a warp, about what the pass takes. With it 192
+// pairs take 1.02 ms, without 1.14; 24 cut halves 1.48 and 1.66; 192 icosphere
+// halves 0.83 and 0.98. Parts cut 30 times have more slivers than that.
+#define HD_FEW 1024u
 
 // A sample's state in the culled search. best is the smallest tri_sq so far;
 // ub bounds the tri_sq of some triangle from above by its centroid's distance
@@ -526,7 +531,7 @@ __device__ __forceinline__ float box_gap(f3 alo, f3 ahi, float4 blo, float4 bhi)
 // loads, 1,024 triangles a step where all are passed over. Every sliver
 // against every sample in turn, 1,200 cycles a sliver, took 740 ms for 96
 // unions of parts cut 30 times with their hulls (1.3 M triangles, two thirds
-// slivers); this takes 11 ms, and the tensor-core bound took 43.
+// slivers); this takes 12 ms, and the tensor-core bound took 43.
 __device__ __noinline__ float hd_ordered(const float4* O, const float4* B, const float4* G, const uint32_t* at,
                                          uint32_t tnt, f3 p, float gmax, uint32_t& exact, uint32_t& met) {
   const uint32_t lane = threadIdx.x & 31;
@@ -554,7 +559,7 @@ __device__ __noinline__ float hd_ordered(const float4* O, const float4* B, const
       float lbT = 3.4e38f, ubT = 3.4e38f, slackT = 0.0f;
       uint32_t i = 0;
       if (t < tnt) {
-        i = at[t] & 0x7fffffffu;
+        i = at[t];
         const HdReach R(pt, p2, p1, O[t]);
         lbT = R.lb;
         ubT = fminf(ubT, R.ub);
@@ -587,7 +592,7 @@ __device__ __noinline__ float hd_ordered(const float4* O, const float4* B, const
 // Warps take tiles of 32 samples from the work list. Targets below
 // A.screenMin triangles are searched exhaustively; for them the sort's boxes
 // save nothing that the extra steps do not cost. Seven blocks an SM: 192 halves
-// of 96 icosphere cuts 0.96 ms, with six 0.98 and with five 1.03.
+// of 96 icosphere cuts 0.83 ms and 24 cut halves 1.48, with six 0.86 and 1.45.
 __global__ void __launch_bounds__(HD_NEAR, 7) k_hd_near(const HdArgs A, const Dev D) {
   __shared__ float4 sCent[HD_NEAR / 32][32];
   const uint32_t lane = threadIdx.x & 31;
@@ -653,7 +658,8 @@ __global__ void __launch_bounds__(HD_NEAR, 7) k_hd_near(const HdArgs A, const De
     S.best = tnt < A.orderedMin ? 1e30f : 3.4e38f;
     S.ub = S.sliver = 3.4e38f;
     S.atSliver = S.atBest = S.atUb = 0;
-    const bool slivers = A.slivers[dst] != 0, ordered = slivers && tnt >= A.orderedMin;
+    const uint32_t slivers = A.slivers[dst];
+    const bool ordered = slivers != 0 && tnt >= A.orderedMin;
     uint32_t why = 0;  // of a sample dropped: the triangle that shows why
     auto settle = [&](float gmax) {
       if (active && !S.counts(gmax)) {
@@ -844,27 +850,36 @@ __global__ void __launch_bounds__(HD_NEAR, 7) k_hd_near(const HdArgs A, const De
         const float gmax = __uint_as_float(__ldcg(gmaxAt));
         if (__shfl_sync(FULLMASK, active && !S.counts(gmax) && !(S.lower(C[S.shows(gmax)]) > S.sliver), l)) continue;
         const f3 p = mk3(__shfl_sync(FULLMASK, S.p.x, l), __shfl_sync(FULLMASK, S.p.y, l), __shfl_sync(FULLMASK, S.p.z, l));
-        uint32_t exact, met;
-        const float best = hd_ordered(A.triO + tb, A.boxO + 2 * (tb >> 5), G, A.cnt + tb, tnt, p, gmax, exact, met);
+        // where no sliver is nearer than the nearest ordinary triangle, and none
+        // rules that one out, it decides: nothing that counts is below it, so
+        // neither a distance nor an ordinary triangle's upper bound puts it out
+        // of reach. A few slivers are asked at once, a lane each
+        float best = __shfl_sync(FULLMASK, S.best, l);
+        bool plain = slivers <= HD_FEW &&
+                     __shfl_sync(FULLMASK, active && !(S.lower(C[S.atBest]) > S.sliver), l);
+        if (plain) {
+          bool below = false;
+          for (uint32_t k = lane; k < slivers; k += 32) {
+            below = below || tri_sq_at(p, G + 3 * (size_t)A.bad[tb + k]) < best;
+            nExact++;
+          }
+          plain = !__any_sync(FULLMASK, below);
+        }
+        uint32_t exact = 0, met = 0;
+        if (!plain) best = hd_ordered(A.triO + tb, A.boxO + 2 * (tb >> 5), G, A.cnt + tb, tnt, p, gmax, exact, met);
         nExact += exact;
         nScreen += met;
         if (best > gmax && lane == 0) atomicMax(gmaxAt, __float_as_uint(best));
       }
       active = false;
-    } else if (slivers && act) {
+    } else if (slivers != 0 && act) {
       // every sliver of a small target
       active = active && S.counts(__uint_as_float(__ldcg(gmaxAt)));
-      for (uint32_t t0 = 0; t0 < tnt && __ballot_sync(FULLMASK, active) != 0; t0 += 32) {
-        const uint32_t w = t0 + lane < tnt ? A.cnt[tb + t0 + lane] : 0u;
-        unsigned of = __ballot_sync(FULLMASK, w >> 31);
-        while (of) {
-          const uint32_t j = __ffs(of) - 1;
-          of &= of - 1;
-          const uint32_t i = __shfl_sync(FULLMASK, w, j) & 0x7fffffffu;
-          if (active) {
-            S.best = fminf(S.best, tri_sq_at(S.p, G + 3 * (size_t)i));
-            nExact++;
-          }
+      for (uint32_t k = 0; k < slivers; k++) {
+        if ((k & 31u) == 0 && __ballot_sync(FULLMASK, active) == 0) break;
+        if (active) {
+          S.best = fminf(S.best, tri_sq_at(S.p, G + 3 * (size_t)A.bad[tb + k]));
+          nExact++;
         }
       }
     }
